@@ -240,7 +240,7 @@ def _with_state(solver, case, **kw):
     place[perm] = np.arange(perm.size, dtype=perm.dtype)
     holder = _DeviceState(solver)
     return {"case": case, "solver": solver, "holder": holder, "U": torch.as_tensor(holder, device="cuda"),
-            "place": torch.from_numpy(place.astype(np.int64)).cuda(), **kw}
+            "place": torch.from_numpy(place.astype(np.int64)).cuda()[:, None].expand(-1, 4), **kw}
 
 
 def _euler_solver(case, order=2, rk=3, local_dt=True, flux="hllc", limiter="venkat", fp32=False, cfl=1.2):
@@ -317,7 +317,7 @@ def run(state):
         lam, fsbar, history, _ = state["adjoint"].solve(g, max_iter=case["iterations"], tol=1e-300)
         return {"residual": residual, "J": J, "dJdU": g, "lambda": lam, "fsbar": fsbar, "history": history}
     history = s.run(case["steps"], history=True)
-    out = {"state": state["U"][state["place"]], "history": history}
+    out = {"state": state["U"].gather(0, state["place"]), "history": history}
     if kind == "rans":
         out["nut"] = s.nut_field()
     return out
