@@ -30,6 +30,7 @@
 #include <type_traits>
 
 #include "euler_o1.cuh"
+#include "fixed.cuh"
 #include "fpconv.cuh"
 
 namespace FV_KNS {
@@ -354,22 +355,35 @@ template <> struct OKey<float> {
 };
 
 // ---------------------------------------------------------------------------
-// Register caps: FP32 mode is latency bound (<= 64 registers, 32 warps per
-// SM); FP64 mode <= 128 (16 warps keep the FP64 pipe fed).
+// Batched solves: converged instances are frozen; each instance has its own
+// freestream (null otherwise: the patch's).
+__device__ __forceinline__ bool live_cell(const O2Args& a, int c, const double*& fs) {
+    fs = nullptr;
+    if (!a.cell_inst) return true;
+    const int inst = a.cell_inst[c];
+    if (a.active && !a.active[inst]) return false;
+    fs = a.inst_fs + 4 * inst;
+    return true;
+}
+
+// W + psi * increment at each of a cell's faces into its wf entry, with
+// recon's positivity fallback (x > 0 as sign bit clear and not +0).
+__device__ __forceinline__ void store_face_states(const O2Args& a, int e0, int e1, const V4<double>& w,
+                                                  const double gx[4], const double gy[4], const double* psi) {
+    for (int e = e0; e < e1; ++e) {
+        double rx, ry;
+        ld_pair<double>(a.erf, e, rx, ry);
+        St o = st_make(psi[0] * (gx[0] * rx + gy[0] * ry) + w.r, psi[1] * (gx[1] * rx + gy[1] * ry) + w.u,
+                       psi[2] * (gx[2] * rx + gy[2] * ry) + w.v, psi[3] * (gx[3] * rx + gy[3] * ry) + w.p);
+        if (OKey<double>::bits(o.r) <= 0 || OKey<double>::bits(o.E) <= 0) o = st_make(w.r, w.u, w.v, w.p);
+        st_state(a.wf, e, o);
+    }
+}
+
 template <typename T, int GRAD, int LIM>
-__global__ void __launch_bounds__(fvgb::kMaxBlock, sizeof(T) == 4 ? 2 : 1) k_grad(const O2Args a) {
+__device__ __forceinline__ void grad_cell(const O2Args& a, int c, const double* fs) {
     using WS = WStore<T>;
     using WT = typename WS::type;
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= a.m.n_cells) return;
-    // Batched solves: converged instances are frozen; each instance has
-    // its own freestream.
-    const double* fs = nullptr;
-    if (a.cell_inst) {
-        const int inst = a.cell_inst[c];
-        if (a.active && !a.active[inst]) return;
-        fs = a.inst_fs + 4 * inst;
-    }
     const WT* W = static_cast<const WT*>(a.W);
     const T g = pick<T>(a.gamma, a.gamma32);
     const V4<T> wc = WS::ld(W, c);
@@ -444,23 +458,16 @@ __global__ void __launch_bounds__(fvgb::kMaxBlock, sizeof(T) == 4 ? 2 : 1) k_gra
                 for (int k = 0; k < 4; ++k) a.lim_psi[4 * c + k] = 1.0;
         }
     }
-    // FP64 with a limiter: k_face reconstructs from the per-entry
-    // increments and the per-cell limiter values (O2Args::d2); the limited
-    // gradients are not stored.
+    // FP64 with a limiter: the reconstructed states of the cell's faces go
+    // to O2Args::wf, an entry each; the limited gradients are not stored.
     bool dpath = false;
-    if constexpr (sizeof(T) == 8) dpath = LIM != 0 && a.d2 != nullptr;
+    if constexpr (sizeof(T) == 8) dpath = LIM != 0 && a.wf != nullptr;
     if (LIM != 0 && a.psi_mode == 2) {
         // frozen limiter: the values captured earlier (psi = 1 scales exactly)
         const T* pb = static_cast<const T*>(a.psi_buf) + 4 * (size_t)c;
         if constexpr (sizeof(T) == 8) {
             if (dpath) {
-                for (int e = e0; e < e1; ++e) {
-                    T rx, ry;
-                    ld_pair<T>(a.erf, e, rx, ry);
-                    st_state(a.d2, e, st_make(gx[0] * rx + gy[0] * ry, gx[1] * rx + gy[1] * ry,
-                                              gx[2] * rx + gy[2] * ry, gx[3] * rx + gy[3] * ry));
-                }
-                st_state(a.psi4, c, st_make(pb[0], pb[1], pb[2], pb[3]));
+                store_face_states(a, e0, e1, wc, gx, gy, pb);
                 return;
             }
         }
@@ -497,9 +504,6 @@ __global__ void __launch_bounds__(fvgb::kMaxBlock, sizeof(T) == 4 ? 2 : 1) k_gra
                 pmax[k] = pmax[k] < b ? b : pmax[k];
                 const I bn = b ^ sign;
                 nmax[k] = nmax[k] < bn ? bn : nmax[k];
-            }
-            if constexpr (sizeof(T) == 8) {
-                if (dpath) st_state(a.d2, e, st_make(d2v[0], d2v[1], d2v[2], d2v[3]));
             }
         }
         T psiv[4];
@@ -557,7 +561,7 @@ __global__ void __launch_bounds__(fvgb::kMaxBlock, sizeof(T) == 4 ? 2 : 1) k_gra
         }
         if constexpr (sizeof(T) == 8) {
             if (dpath) {
-                st_state(a.psi4, c, st_make(psiv[0], psiv[1], psiv[2], psiv[3]));
+                store_face_states(a, e0, e1, wc, gx, gy, psiv);
                 return;
             }
         }
@@ -566,6 +570,16 @@ __global__ void __launch_bounds__(fvgb::kMaxBlock, sizeof(T) == 4 ? 2 : 1) k_gra
 #pragma unroll
     for (int k = 0; k < 4; ++k) { out.gx[k] = gx[k]; out.gy[k] = gy[k]; }
     GStore<T>::st(static_cast<typename GStore<T>::type*>(a.G), c, out);
+}
+
+// Register caps: FP32 mode is latency bound (<= 64 registers, 32 warps per
+// SM); FP64 mode <= 128 (16 warps keep the FP64 pipe fed).
+template <typename T, int GRAD, int LIM>
+__global__ void __launch_bounds__(fvgb::kMaxBlock, sizeof(T) == 4 ? 2 : 1) k_grad(const O2Args a) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= a.m.n_cells) return;
+    const double* fs;
+    if (live_cell(a, c, fs)) grad_cell<T, GRAD, LIM>(a, c, fs);
 }
 
 template <typename T>
@@ -579,14 +593,6 @@ __device__ __forceinline__ V4<T> recon(const V4<T>& w, const G8<T>& g, T rx, T r
     return o;
 }
 
-// w + psi * inc (the limited increment to the face, one multiply-add per
-// variable), with recon's positivity fallback.
-__device__ __forceinline__ V4<double> recon_inc(const V4<double>& w, const St& psi, const St& inc) {
-    const V4<double> o = {psi.r * inc.r + w.r, psi.ru * inc.ru + w.u, psi.rv * inc.rv + w.v, psi.E * inc.E + w.p};
-    if (OKey<double>::bits(o.r) <= 0 || OKey<double>::bits(o.p) <= 0) return w;
-    return o;
-}
-
 template <typename T, int FLUX>
 __device__ __forceinline__ V4<T> num_flux_p(const V4<T>& L, const V4<T>& R, T nx, T ny, T g, T igm1, double tol,
                                             int maxit) {
@@ -597,6 +603,19 @@ __device__ __forceinline__ V4<T> num_flux_p(const V4<T>& L, const V4<T>& R, T nx
         St F = exact_riemann(UL, UR, (double)nx, (double)ny, (double)g, tol, maxit);
         return {(T)F.r, (T)F.ru, (T)F.rv, (T)F.E};
     } else return rusanov_p<T>(L, R, nx, ny, g, igm1);
+}
+
+// The block's smallest candidate into the step's global-dt minimum.
+__device__ __forceinline__ void block_min_dt(double cand, StepCtl* ctl) {
+    __shared__ double smin[fvgb::kMaxBlock / 32];
+    cand = warp_min(cand);
+    if ((threadIdx.x & 31) == 0) smin[threadIdx.x >> 5] = cand;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double v = smin[0];
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) v = fmin(v, smin[w]);
+        atomicMin(&ctl->dt_bits, (unsigned long long)__double_as_longlong(v));
+    }
 }
 
 // DT: 0 = no time step this stage, 1 = global (atomicMin), 2 = local (per face).
@@ -619,12 +638,12 @@ __global__ void __launch_bounds__(fvgb::kMaxBlock) k_face(const O2Args a) {
         V4<T> wl = WS::ld(W, L), wr;
         const V4<T> wlc = wl;
         bool dpath = false;
-        if constexpr (sizeof(T) == 8) dpath = ORDER == 2 && a.d2 != nullptr;
+        if constexpr (sizeof(T) == 8) dpath = ORDER == 2 && a.wf != nullptr;
         if (dpath) {
             if constexpr (sizeof(T) == 8) {
                 const int2 ee = __ldg(a.fe + f);
-                wl = recon_inc(wl, ld_state(a.psi4, L), ld_state(a.d2, ee.x));
-                if (R >= 0) wr = recon_inc(WS::ld(W, R), ld_state(a.psi4, R), ld_state(a.d2, ee.y));
+                wl = WS::ld(a.wf, ee.x);
+                if (R >= 0) wr = WS::ld(a.wf, ee.y);
             }
         } else if (ORDER == 2) {
             T rxl, ryl, rxr, ryr;
@@ -662,17 +681,7 @@ __global__ void __launch_bounds__(fvgb::kMaxBlock) k_face(const O2Args a) {
             }
         }
     }
-    if (DT == 1) {
-        __shared__ double smin[fvgb::kMaxBlock / 32];
-        cand = warp_min(cand);
-        if ((threadIdx.x & 31) == 0) smin[threadIdx.x >> 5] = cand;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double v = smin[0];
-            for (int w = 1; w < (int)(blockDim.x >> 5); ++w) v = fmin(v, smin[w]);
-            atomicMin(&a.ctl->dt_bits, (unsigned long long)__double_as_longlong(v));
-        }
-    }
+    if (DT == 1) block_min_dt(cand, a.ctl);
 }
 
 // FP32-flux mode: the primitive copy and the sound speed only feed FP32

@@ -296,6 +296,7 @@ extern "C" int fv_solver_update_nodes(fv_solver_t solver, fv_mesh_t mesh, const 
                 geo::k_o2_face_offsets<double><<<(s.F + B - 1) / B, B, 0, s.stream>>>(a);
             }
             FV_CUDA(cudaGetLastError());
+            s.refresh_fixed_geometry();
         }
         FV_CUDA(cudaStreamSynchronize(s.stream));
         // host copies of the wall faces (force integration)

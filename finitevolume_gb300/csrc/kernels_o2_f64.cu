@@ -1,6 +1,6 @@
 // Second-order kernels instantiated for double flux/gradient arithmetic.
 #define FV_KNS fast
-#include "euler_o2.cuh"
+#include "euler_o2_fixed.cuh"
 
 namespace {
 using R = double;
@@ -11,12 +11,27 @@ using fvgb::O2Config;
 template <int GRAD, int LIM>
 void grad(const O2Args& a, int bs, cudaStream_t s) {
     const int cb = (a.m.n_cells + bs - 1) / bs;
+    // The adjoint's linearisation (wf null) takes its gradients from the FP64 pass.
+    if constexpr (GRAD == 0 && LIM != 0) {
+        if (a.fxs && a.wf) {
+            k_grad_fx<LIM><<<(4LL * a.m.n_cells + bs - 1) / bs, bs, 0, s>>>(a);  // four lanes per cell
+            return;
+        }
+    }
     k_grad<R, GRAD, LIM><<<cb, bs, 0, s>>>(a);
 }
 
 template <int FLUX, int ORDER>
 void face(const O2Args& a, int dt, int bs, cudaStream_t s) {
     const int fb = (a.m.n_faces + bs - 1) / bs;
+    if constexpr (FLUX != 2) {
+        if (a.fixed) {
+            if (dt == 1) k_face_fx<FLUX, ORDER, 1><<<fb, bs, 0, s>>>(a);
+            else if (dt == 2) k_face_fx<FLUX, ORDER, 2><<<fb, bs, 0, s>>>(a);
+            else k_face_fx<FLUX, ORDER, 0><<<fb, bs, 0, s>>>(a);
+            return;
+        }
+    }
     if (dt == 1) k_face<R, FLUX, ORDER, 1><<<fb, bs, 0, s>>>(a);
     else if (dt == 2) k_face<R, FLUX, ORDER, 2><<<fb, bs, 0, s>>>(a);
     else k_face<R, FLUX, ORDER, 0><<<fb, bs, 0, s>>>(a);
@@ -36,6 +51,10 @@ namespace o2 {
 void launch_batch_norms(const O2Args& a, int n_inst, const int* inst_off, double* inst_norms, int* inst_iter,
                         int* active, double tol, cudaStream_t s) {
     ::fast::k_batch_norms<<<n_inst, 256, 0, s>>>(a, inst_off, inst_norms, inst_iter, active, tol);
+}
+
+void launch_fix_geom(const O2Args& a, int4* fxa, int4* fxr, int* fxs, cudaStream_t s) {
+    ::fast::k_fix_geom<<<(a.m.n_cells + 255) / 256, 256, 0, s>>>(a, fxa, fxr, fxs);
 }
 
 void launch_prim_f64(const O2Args& a, cudaStream_t s) {

@@ -245,9 +245,29 @@ void Solver::init(const HostMesh& hm, const fv_bc_t* bcs, int n_bcs, double g, d
                 if (ent & 1) fev[ent >> 1].x = (int)e;
                 else fev[ent >> 1].y = (int)e;
             }
-            d2 = dalloc<St>(E, owned);
-            psi4 = dalloc<St>(N, owned);
+            wf = dalloc<St>(E, owned);
             fe = dupload(fev, owned);
+        }
+        // The fixed-point passes cover the Rusanov and HLLC fluxes, and with a
+        // limiter the least-squares gradients.
+        fixed = !cfg.fp32 && cfg.flux != FV_FLUX_EXACT && fixed_gamma() && (cfg.order == 1 || cfg.limiter != 0);
+        if (fixed) {
+            const double* st = batch ? batch_freestream : &bc.st[0][0];
+            std::vector<double> q;
+            for (int i = 0; i < (batch ? n_inst : kMaxPatches); ++i, st += 4) {
+                const bool has = st[0] != 0.0;  // patches without a farfield state stay zero
+                const double r = st[0], u = has ? st[1] / r : 0.0, v = has ? st[2] / r : 0.0;
+                const double p = (gamma - 1.0) * (st[3] - 0.5 * r * (u * u + v * v));
+                const double c = has ? std::sqrt(gamma * p / r) : 0.0;
+                for (double x : {r, u, v, p, c, has ? 1.0 / c : 0.0, 1.0 / gamma, 0.0}) q.push_back(x);
+            }
+            fsp = dupload(q, owned);
+        }
+        if (fixed && cfg.order == 2 && cfg.gradient == 0) {
+            fxa = dalloc<int4>(h2.d_cf.size(), owned);
+            fxr = dalloc<int4>(h2.d_cf.size(), owned);
+            fxs = dalloc<int>(N, owned);
+            refresh_fixed_geometry();
         }
     }
 
@@ -483,12 +503,32 @@ O2Args Solver::o2_args() const {
     a.lim_psi = nullptr;
     a.psi_buf = psi_buf;
     a.psi_mode = psi_mode;
-    a.d2 = d2;
-    a.psi4 = psi4;
+    a.wf = wf;
     a.fe = fe;
     a.forcing = forcing;
     a.resid = nullptr;
+    a.fixed = fixed;
+    a.fxa = fxa;
+    a.fxr = fxr;
+    a.fxs = fxs;
+    a.fxc = flux_const();
+    a.fsp = fsp;
     return a;
+}
+
+fvfix::FluxConst Solver::flux_const() const {
+    fvfix::FluxConst k{};
+    if (!fixed_gamma()) return k;
+    k.gamma = std::llrint(std::ldexp(gamma, 60));
+    k.igm1_4 = std::llrint(std::ldexp(0.25 / (gamma - 1.0), 60));
+    k.gammaf = (float)gamma;
+    return k;
+}
+
+void Solver::refresh_fixed_geometry() {
+    if (!fxs) return;
+    o2::launch_fix_geom(o2_args(), fxa, fxr, fxs, stream);
+    FV_CUDA(cudaGetLastError());
 }
 
 void Solver::refresh_primitives() {

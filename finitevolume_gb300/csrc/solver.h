@@ -117,9 +117,13 @@ struct Solver {
     const float4* fgeom32 = nullptr;
     const St* forcing = nullptr;    // multigrid coarse levels: FAS forcing term
     void* psi_buf = nullptr;        // frozen limiter values [4N], flux precision
-    St* d2 = nullptr;               // FP64 live limiter: per-entry increments [E] (O2Args::d2)
-    St* psi4 = nullptr;             //   and per-cell limiter values [N]
+    St* wf = nullptr;               // FP64 with a limiter: per-entry face states [E] (O2Args::wf)
     int2* fe = nullptr;             //   owner / neighbour entry per face [F]
+    int fixed = 0;                  // fixed-point passes (O2Args::fixed) and their geometry
+    int4* fxa = nullptr;
+    int4* fxr = nullptr;
+    int* fxs = nullptr;
+    double* fsp = nullptr;          // farfield primitives (O2Args::fsp)
     int psi_mode = 0;               // 0 evaluated, 2 frozen (see O2Args)
 
     // Persistent first-order path (order 1, forward Euler, FP64 Euler): one
@@ -151,6 +155,10 @@ struct Solver {
     RansArgs rans_args() const;
     O2Args o2_args() const;
     void refresh_primitives();
+    // gammas whose energies stay within the fixed-point fluxes' units
+    bool fixed_gamma() const { return gamma >= 1.2 && gamma <= 3.0; }
+    fvfix::FluxConst flux_const() const;
+    void refresh_fixed_geometry();  // after the reconstruction geometry changed
     void launch_step(std::vector<int>* classes, std::vector<cudaEvent_t>* events, size_t* ev_pos);
     // k steps: one persistent launch, or k x launch_step
     void launch_steps(int k, std::vector<int>* classes, std::vector<cudaEvent_t>* events, size_t* ev_pos);

@@ -5,6 +5,8 @@
 
 #include <cuda_runtime.h>
 
+#include "fixed_types.h"
+
 namespace fvgb {
 
 // Conserved state of one cell, AoS, one 32-byte sector: {rho, rho_u, rho_v, E}.
@@ -156,21 +158,29 @@ struct O2Args {
     // instead of evaluating the limiter; 0 neither.
     void* psi_buf;
     int psi_mode;
-    // FP64 live-limiter reconstruction (null otherwise): per cell-face
-    // entry the unlimited increment g . (x_f - x_c) of the four primitives,
-    // per cell the four limiter values, and per face the entries of its
-    // owner and neighbour (-1 on a boundary face).  With psi_mode != 2
-    // k_grad writes the first two instead of the limited gradients, and
-    // k_face reconstructs W + psi * increment: the increments k_grad forms
-    // for the limiter anyway are not formed a second time.
-    St* d2;
-    St* psi4;
+    // FP64 reconstruction with a limiter (null otherwise): per cell-face
+    // entry the reconstructed state of the cell at that face, written by
+    // k_grad and read by k_face, and per face the entries of its owner and
+    // neighbour (-1 on a boundary face).
+    St* wf;
     const int2* fe;
     // Multigrid (null otherwise): a forcing term added to every cell's
     // residual (coarse levels of the full-approximation scheme), and the
     // output of the residual-only pass.
     const St* forcing;
     St* resid;
+    // Fixed-point form of the FP64 gradient and face passes
+    // (euler_o2_fixed.cuh): `fixed` where the scheme has one; per entry the
+    // scaled weights and offsets, per cell their common exponent (null
+    // without them: the FP64 gradient pass); flux constants.
+    int fixed;
+    const int4* fxa;
+    const int4* fxr;
+    const int* fxs;
+    fvfix::FluxConst fxc;
+    // Farfield states for those passes: r, u, v, p, c, 1/c, 1/gamma, 0 per
+    // patch (batched solves: per instance).
+    const double* fsp;
 };
 
 // Second-order path configuration (validated by the solver).
@@ -202,6 +212,8 @@ void launch_part_f32(const O2Args& a, const O2Config& c, int stage, int part, cu
 // the last face pass; no update
 void launch_residual_f64(const O2Args& a, cudaStream_t s);
 void launch_residual_f32(const O2Args& a, cudaStream_t s);
+// the fixed-point gradient geometry (O2Args::fxa, fxr, fxs) from a.lsq, a.erf
+void launch_fix_geom(const O2Args& a, int4* fxa, int4* fxr, int* fxs, cudaStream_t s);
 void launch_batch_norms(const O2Args& a, int n_inst, const int* inst_off, double* inst_norms, int* inst_iter,
                         int* active, double tol, cudaStream_t s);
 }  // namespace o2
