@@ -697,6 +697,47 @@ __device__ __forceinline__ V4<float> prim32(const St& un, float gf, float& cs) {
     return {rf, uf, vf, pf};
 }
 
+// FP64 mode: the same from the state in FP64, and the sound speed on the
+// integer pipe.
+__device__ __forceinline__ V4<double> prim64(const St& un, double g) {
+    const double ir = fvconv::rcp_nr3(un.r);
+    const double uu = un.ru * ir, vv = un.rv * ir;
+    return {un.r, uu, vv, (g - 1.0) * (un.E - 0.5 * (un.ru * uu + un.rv * vv))};
+}
+__device__ __forceinline__ double sound64(const V4<double>& w, double g) {
+    double c;
+    if (!fvfix::sound_speed(w.r, w.p, g, c)) c = sqrt(g * w.p / w.r);
+    return c;
+}
+
+// The signed sum of a cell's N face fluxes, component by component on the
+// integer pipe (the FP64 pipe bounds the update: N - 1 additions a component
+// there).
+template <int N>
+__device__ __forceinline__ St gather_fixed(const St* ff, const int* cf) {
+    double x[4][N];
+    int neg[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const int ent = __ldg(cf + i);
+        const St F = ld_state(ff, ent >> 1);
+        x[0][i] = F.r; x[1][i] = F.ru; x[2][i] = F.rv; x[3][i] = F.E;
+        neg[i] = ent;
+    }
+    return st_make(fvfix::signed_sum<N>(x[0], neg), fvfix::signed_sum<N>(x[1], neg), fvfix::signed_sum<N>(x[2], neg),
+                   fvfix::signed_sum<N>(x[3], neg));
+}
+template <int N>
+__device__ __forceinline__ St gather_fixed(const float4*, const int*) { return {}; }  // FP32 flux: gather32
+
+// x / 4 by the exponent field where that is exact
+__device__ __forceinline__ double quarter(double x) {
+    return fvfix::biased(fvfix::hi_word(x)) - 3u < 2040u ? fvfix::scale2(x, -2) : 0.25 * x;
+}
+__device__ __forceinline__ St quarter(const St& s) {
+    return st_make(quarter(s.r), quarter(s.ru), quarter(s.rv), quarter(s.E));
+}
+
 // STAGE: 0..NST-1; NST: 1 (forward Euler) or 3 (SSP-RK3); DT: 1 global, 2 local.
 template <typename T, int STAGE, int NST, int DT>
 __global__ void __launch_bounds__(fvgb::kMaxBlock) k_update(const O2Args a) {
@@ -712,17 +753,23 @@ __global__ void __launch_bounds__(fvgb::kMaxBlock) k_update(const O2Args a) {
         if constexpr (std::is_same<T, float>::value) {
             R = gather32<STAGE == 0 && DT == 2>(ff, reinterpret_cast<const float*>(a.dtf), a.m.cf, e0, e1, lamf);
         } else {
-            // Every cell has faces: the sum starts from the first signed flux
-            // instead of 0 + flux (one FP64 add per component less; only the
-            // sign of an exactly-zero sum can differ, and u + dt * (+-0) = u).
-            const int ent0 = a.m.cf[e0];
-            R = flip_if(ld_flux(ff, ent0 >> 1), ent0);
-            if (STAGE == 0 && DT == 2) lam = a.dtf[ent0 >> 1];
-            for (int e = e0 + 1; e < e1; ++e) {
-                const int ent = a.m.cf[e];
-                const int f = ent >> 1;
-                R += flip_if(ld_flux(ff, f), ent);
-                if (STAGE == 0 && DT == 2) lam += a.dtf[f];
+            const int n = e1 - e0;
+            if (n == 4) R = gather_fixed<4>(ff, a.m.cf + e0);
+            else if (n == 3) R = gather_fixed<3>(ff, a.m.cf + e0);
+            else {
+                // Every cell has faces: the sum starts from the first signed flux
+                // instead of 0 + flux (one FP64 add per component less; only the
+                // sign of an exactly-zero sum can differ, and u + dt * (+-0) = u).
+                const int ent0 = a.m.cf[e0];
+                R = flip_if(ld_flux(ff, ent0 >> 1), ent0);
+                for (int e = e0 + 1; e < e1; ++e) {
+                    const int ent = a.m.cf[e];
+                    R += flip_if(ld_flux(ff, ent >> 1), ent);
+                }
+            }
+            if (STAGE == 0 && DT == 2) {
+                lam = a.dtf[a.m.cf[e0] >> 1];
+                for (int e = e0 + 1; e < e1; ++e) lam += a.dtf[a.m.cf[e] >> 1];
             }
         }
         if (a.forcing) R += ld_state(a.forcing, c);
@@ -752,7 +799,7 @@ __global__ void __launch_bounds__(fvgb::kMaxBlock) k_update(const O2Args a) {
         St un;
         if (NST == 1) un = e;
         else if (STAGE == 0) { st_state(a.U0, c, u); un = e; }
-        else if (STAGE == 1) un = 0.75 * ld_state(a.U0, c) + 0.25 * e;
+        else if (STAGE == 1) un = 0.75 * ld_state(a.U0, c) + quarter(e);
         else un = (1.0 / 3.0) * ld_state(a.U0, c) + (2.0 / 3.0) * e;
         st_state(a.U, c, un);
         const double g = a.gamma;
@@ -761,11 +808,9 @@ __global__ void __launch_bounds__(fvgb::kMaxBlock) k_update(const O2Args a) {
             WStore<T>::st(static_cast<typename WStore<T>::type*>(a.W), c, prim32(un, a.gamma32, cs));
             if (STAGE == NST - 1) static_cast<float*>(a.cs)[c] = cs;
         } else {
-            const double ir = fvconv::rcp_nr3(un.r);  // same as k_prim / k_update
-            const double uu = un.ru * ir, vv = un.rv * ir;
-            const double p = (g - 1.0) * (un.E - 0.5 * un.r * (uu * uu + vv * vv));
-            WStore<T>::st(static_cast<typename WStore<T>::type*>(a.W), c, V4<T>{un.r, uu, vv, p});
-            if (STAGE == NST - 1) static_cast<double*>(a.cs)[c] = sqrt(g * p * ir);
+            const V4<double> w = prim64(un, g);
+            WStore<T>::st(static_cast<typename WStore<T>::type*>(a.W), c, w);
+            if (STAGE == NST - 1) static_cast<double*>(a.cs)[c] = sound64(w, g);
         }
     }
     // Batched solves reduce per instance instead (k_batch_norms); a.r2 is
@@ -838,16 +883,14 @@ __global__ void __launch_bounds__(fvgb::kCellBlock) k_prim(const O2Args a) {
     if (c >= a.m.n_cells) return;
     const St un = ld_state(a.U, c);
     const double g = a.gamma;
-    const double ir = fvconv::rcp_nr3(un.r);  // same as k_prim / k_update
-    const double uu = un.ru * ir, vv = un.rv * ir;
-    const double p = (g - 1.0) * (un.E - 0.5 * un.r * (uu * uu + vv * vv));
     if constexpr (std::is_same<T, float>::value) {
         float cs;
         WStore<T>::st(static_cast<typename WStore<T>::type*>(a.W), c, prim32(un, a.gamma32, cs));
         static_cast<float*>(a.cs)[c] = cs;
     } else {
-        WStore<T>::st(static_cast<typename WStore<T>::type*>(a.W), c, V4<T>{(T)un.r, (T)uu, (T)vv, (T)p});
-        static_cast<double*>(a.cs)[c] = sqrt(g * p * ir);
+        const V4<double> w = prim64(un, g);
+        WStore<T>::st(static_cast<typename WStore<T>::type*>(a.W), c, w);
+        static_cast<double*>(a.cs)[c] = sound64(w, g);
     }
 }
 

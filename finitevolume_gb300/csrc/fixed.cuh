@@ -310,6 +310,42 @@ __device__ __forceinline__ bool flux(const W& L, const W& R, double cLd, double 
     return true;
 }
 
+// Sound speed sqrt(g p / r) within an ulp, with one FP64 instruction (the
+// FP64 form takes ten); false outside the ranges.
+__device__ __forceinline__ bool sound_speed(double r, double p, double g, double& c) {
+    const int er = (int)((unsigned)hi_word(r) >> 20), ep = (int)((unsigned)hi_word(p) >> 20);
+    const int eg = (int)((unsigned)hi_word(g) >> 20) - 1023;  // 0 or 1: gamma in [1, 4)
+    if ((unsigned)(er - 723) > 600u || (unsigned)(ep - 723) > 600u || (unsigned)eg > 1u) return false;
+    // r = m 2^er, p = q 2^(er + 2 kc) with q in [1, 4): c = sqrt(g q / m) 2^kc
+    const int kc = (ep - er) >> 1, odd = (ep - er) & 1;
+    const float y = rsqrt_f((float)g * mant_float(p, odd) * mant_float(r, 0));
+    const i64 m4 = shr_short(top_bits(r), 5), g2 = shr_short(top_bits(g), 4 - eg), q8 = shr_short(top_bits(p), 6 - odd);
+    const i64 gq = mul<4>(g2, q8);    // g q / 16
+    const i64 x = mul<4>(gq, m4);     // g q m / 64
+    c = scale2(__ll2double_rn(sound(gq, x, (unsigned)__float2int_rn(y * 134217728.0f))), kc + 1 - 60);  // Q24 of 8 y
+    return true;
+}
+
+// The signed sum of N FP64 values (bit 0 of neg[i] flips the sign of x[i]) in
+// fixed point: exact but for bits below 2^-59 of the largest, one FP64
+// instruction instead of N - 1.
+template <int N>
+__device__ __forceinline__ double signed_sum(const double (&x)[N], const int (&neg)[N]) {
+    int E = 0;
+#pragma unroll
+    for (int i = 0; i < N; ++i) E = max(E, biased(hi_word(x[i])));
+    if ((unsigned)(E - 150) > 1750u) {  // all zero, tiny, huge or not finite
+        double s = 0.0;
+#pragma unroll
+        for (int i = 0; i < N; ++i) s += neg[i] & 1 ? -x[i] : x[i];
+        return s;
+    }
+    i64 s = 0;
+#pragma unroll
+    for (int i = 0; i < N; ++i) s += to_fixed<59>(x[i], E, -(neg[i] & 1));
+    return to_double(s, E - 1023 - 59);
+}
+
 // num / den * 2^52, rounded, for 0 < num <= den, den in [2^56, 2^62): three
 // quotient digits of 20, 20 and 12 bits, each from the float quotient of
 // the exact remainder (within 3/4 of a unit).
