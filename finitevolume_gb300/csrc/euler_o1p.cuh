@@ -49,6 +49,7 @@
 #pragma once
 
 #include "euler_o1.cuh"
+#include "fixed.cuh"
 #include "fpconv.cuh"
 
 namespace FV_KNS {
@@ -72,7 +73,7 @@ __device__ __forceinline__ Prim prim_of(const St& s, double g) {
     q.u = s.ru * ir;
     q.v = s.rv * ir;
     q.p = (g - 1.0) * (s.E - 0.5 * (s.ru * q.u + s.rv * q.v));
-    q.c = sqrt(g * q.p * ir);
+    if (!fvfix::sound_speed(s.r, q.p, g, q.c)) q.c = sqrt(g * q.p * ir);
 #endif
     return q;
 }
@@ -266,6 +267,23 @@ __device__ __forceinline__ double face_phase_face(const O1Args& a, const double4
         PR = prim_of(UR, g);
 #endif
     }
+#ifndef FV_STRICT_ORDER
+    // Fixed point (fixed.cuh): the FP64 form below takes what it refuses.
+    if (FLUX != FLUX_EXACT && a.fixed) {
+        const fvfix::State L4 = {UL.r, PL.u, PL.v, PL.p}, R4 = {UR.r, PR.u, PR.v, PR.p};
+        fvfix::State F;
+        double lam;
+        if (fvfix::flux<FLUX == FLUX_HLLC ? 1 : 0, true, true>(L4, R4, PL.c, PR.c, geo.x, geo.y, geo.z, a.fxc, F,
+                                                               R >= 0, lam)) {
+            st_state(a.ff, f, st_make(F.r, F.u, F.v, F.p));
+            if (LOCAL) {
+                a.dtf[f] = lam * geo.z;
+                return DBL_MAX;
+            }
+            return cfl * geo.w * fvconv::rcp_nr3(lam);
+        }
+    }
+#endif
     const St Fl = num_flux_p<FLUX>(UL, PL, UR, PR, geo.x, geo.y, g, a.exact_tol, a.exact_max_iter);
     st_state(a.ff, f, geo.z * Fl);
     const double Smax = face_smax_p(PL, PR, R >= 0, geo.x, geo.y);
@@ -276,6 +294,28 @@ __device__ __forceinline__ double face_phase_face(const O1Args& a, const double4
     return cfl * geo.w / Smax;
 }
 
+#ifndef FV_STRICT_ORDER
+// The signed sum of a cell's N face fluxes and, with LOCAL, the sum of its
+// faces' lambda * length, on the integer pipe (fvfix::signed_sum).
+template <int N, bool LOCAL>
+__device__ __forceinline__ St gather_cell(const O1Args& a, int e0, double& lam) {
+    double x[4][N], l[N];
+    int neg[N], none[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const int ent = a.m.cf[e0 + i];
+        const St F = ld_state_cg(a.ff, ent >> 1);
+        x[0][i] = F.r; x[1][i] = F.ru; x[2][i] = F.rv; x[3][i] = F.E;
+        if (LOCAL) l[i] = __ldcg(a.dtf + (ent >> 1));
+        neg[i] = ent;
+        none[i] = 0;
+    }
+    if (LOCAL) lam = fvfix::signed_sum<N>(l, none);
+    return st_make(fvfix::signed_sum<N>(x[0], neg), fvfix::signed_sum<N>(x[1], neg), fvfix::signed_sum<N>(x[2], neg),
+                   fvfix::signed_sum<N>(x[3], neg));
+}
+#endif
+
 // One cell of the cell phase: the signed gather of its face fluxes,
 // U += dt/V R, the new primitives, and the squares of R for the norms.
 template <bool LOCAL>
@@ -285,6 +325,12 @@ __device__ __forceinline__ void cell_phase_cell(const O1Args& a, double4_32a* P,
     St Rs = st_make(0.0, 0.0, 0.0, 0.0);
     const int e0 = a.m.cf_off[c], e1 = a.m.cf_off[c + 1];
     double lam = 0.0;
+#ifndef FV_STRICT_ORDER
+    const int n = e1 - e0;
+    if (n == 4) Rs = gather_cell<4, LOCAL>(a, e0, lam);
+    else if (n == 3) Rs = gather_cell<3, LOCAL>(a, e0, lam);
+    else
+#endif
     for (int e = e0; e < e1; ++e) {
         const int ent = a.m.cf[e];
         const int f = ent >> 1;
@@ -296,7 +342,7 @@ __device__ __forceinline__ void cell_phase_cell(const O1Args& a, double4_32a* P,
     if (LOCAL) dt = cfl * a.m.vol[c] / lam;
     coef = dt / a.m.vol[c];
 #else
-    coef = LOCAL ? cfl * fvconv::rcp_nr3(lam) : dt / a.m.vol[c];
+    coef = LOCAL ? cfl * fvconv::rcp_nr3(lam) : dt * fvconv::rcp_nr3(a.m.vol[c]);
 #endif
     s0 = Rs.r * Rs.r; s1 = Rs.ru * Rs.ru; s2 = Rs.rv * Rs.rv; s3 = Rs.E * Rs.E;
     const St u = ld_state_cg(a.U, c);

@@ -461,6 +461,8 @@ O1Args Solver::o1_args() const {
     a.exact_max_iter = opt.exact_max_iter;
     a.flux = opt.flux;
     a.local_dt = opt.dt_mode == FV_DT_LOCAL;
+    a.fixed = !opt.strict && fixed_gamma();
+    a.fxc = flux_const();
     return a;
 }
 

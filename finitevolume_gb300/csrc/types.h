@@ -111,6 +111,8 @@ struct O1Args {
     int exact_max_iter;
     int flux;          // 0 Rusanov, 1 HLLC, 2 exact
     int local_dt;
+    int fixed;         // the persistent kernel's default build takes its fluxes in fixed point
+    fvfix::FluxConst fxc;
 };
 
 struct O2Args {
