@@ -10,6 +10,12 @@
 //              squared-residual sum and phi += dt / V * r.
 // Expressions keep the reference's evaluation order; built without FMA
 // contraction (strict) the field is bit-identical to the reference.
+//
+// Bound: FP64 issue in the face pass (8 instructions a face: the difference,
+// the quotient as five multiply-adds with the prepared reciprocal, two
+// products), launches below about 100k cells.  260k cells: face pass 16 ->
+// 14 us (division -> quotient), cell pass 66 -> 11 us (its last block folded
+// the block partials with one thread, and every cell divided dt by V).
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
@@ -19,11 +25,14 @@
 
 #include "../../include/fv_gb300.h"
 #include "errors.h"
+#include "fpconv.cuh"
 #include "mesh_host.h"
 #include "types.h"
 
 namespace fvgb {
 namespace {
+
+constexpr int kGroup = 16;  // steps per graph and per fold of the norms
 
 struct DiffArgs {
     int n_cells, n_faces;
@@ -31,17 +40,17 @@ struct DiffArgs {
     const int* fr;
     const int* fpatch;
     const double* farea;
-    const double* fdist;   // internal: centroid-centroid; boundary: centroid-midpoint
+    const double2* fdist;  // internal: centroid-centroid; boundary: centroid-midpoint; and 1 / that (0: use the division)
     const int* cf_off;
     const int* cf;
-    const double* vol;
+    const double* coef;    // dt / V
     double* phi;
     double* ff;
     double* partials;
     double* hist;
     int hist_cap;
     StepCtl* ctl;
-    double alpha, dt;
+    double alpha;
     int ptype[kMaxPatches];
     double pval[kMaxPatches];
 };
@@ -57,14 +66,14 @@ __global__ void __launch_bounds__(kFaceBlock) k_diff_face(const DiffArgs a) {
     const int R = a.fr[f];
     double flux;
     if (R >= 0) {
-        const double gn = (a.phi[R] - phiL) / a.fdist[f];
+        const double gn = fvconv::quotient(a.phi[R] - phiL, a.fdist[f]);
         flux = -a.alpha * gn * a.farea[f];
     } else {
         const int p = a.fpatch[f];
         if (a.ptype[p] == 1) {
             flux = a.pval[p] * a.farea[f];
         } else {
-            const double gn = (a.pval[p] - phiL) / a.fdist[f];
+            const double gn = fvconv::quotient(a.pval[p] - phiL, a.fdist[f]);
             flux = -a.alpha * gn * a.farea[f];
         }
     }
@@ -77,7 +86,8 @@ __device__ __forceinline__ double wsum(double v) {
     return v;
 }
 
-__global__ void __launch_bounds__(kCellBlock) k_diff_cell(const DiffArgs a) {
+// slot: which of a group's kGroup partial rows this step leaves.
+__global__ void __launch_bounds__(kCellBlock) k_diff_cell(const DiffArgs a, int slot) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     double s = 0.0;
     if (c < a.n_cells) {
@@ -87,31 +97,38 @@ __global__ void __launch_bounds__(kCellBlock) k_diff_cell(const DiffArgs a) {
             r += flip1(a.ff[ent >> 1], ent);
         }
         s = r * r;
-        a.phi[c] += (a.dt / a.vol[c]) * r;
+        a.phi[c] += a.coef[c] * r;
     }
     __shared__ double red[kCellBlock / 32];
-    __shared__ bool last;
     s = wsum(s);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
     __syncthreads();
     if (threadIdx.x == 0) {
         double v = 0.0;
         for (int i = 0; i < kCellBlock / 32; ++i) v += red[i];
-        a.partials[blockIdx.x] = v;
-        __threadfence();
-        last = (atomicAdd(&a.ctl->done_blocks, 1u) == gridDim.x - 1);
+        a.partials[(size_t)slot * gridDim.x + blockIdx.x] = v;
+    }
+}
+
+// Norms of a group of n <= kGroup steps, one warp a step: after the group
+// instead of in each step's last block, which would hold up the next step.
+__global__ void __launch_bounds__(32 * kGroup) k_diff_norms(const DiffArgs a, int n, int nblk) {
+    __shared__ double norm[kGroup];
+    const int w = threadIdx.x >> 5;
+    if (w < n) {
+        double t = 0.0;
+        for (int b = threadIdx.x & 31; b < nblk; b += 32) t += a.partials[(size_t)w * nblk + b];
+        t = wsum(t);
+        if ((threadIdx.x & 31) == 0) norm[w] = sqrt(t);
     }
     __syncthreads();
-    if (!last || threadIdx.x != 0) return;
-    __threadfence();
-    double t = 0.0;
-    for (int b = 0; b < (int)gridDim.x; ++b) t += ((volatile double*)a.partials)[b];
-    const double n = sqrt(t);
-    a.ctl->norms[0] = n;
-    a.hist[a.ctl->step % a.hist_cap] = n;
-    if (!isfinite(n)) a.ctl->nonfinite = 1;
-    a.ctl->step += 1;
-    a.ctl->done_blocks = 0u;
+    if (threadIdx.x != 0) return;
+    for (int i = 0; i < n; ++i) {
+        a.hist[(a.ctl->step + i) % a.hist_cap] = norm[i];
+        if (!isfinite(norm[i])) a.ctl->nonfinite = 1;
+    }
+    a.ctl->norms[0] = norm[n - 1];
+    a.ctl->step += n;
 }
 
 __global__ void k_diff_scatter(const double* __restrict__ phi, double* __restrict__ out, const int* __restrict__ perm,
@@ -134,7 +151,7 @@ struct DiffSolver {
     double* staging = nullptr;
     cudaStream_t stream = nullptr;
     std::vector<void*> owned;
-    std::vector<cudaGraphExec_t> graph;  // one 16-step graph
+    std::vector<cudaGraphExec_t> graph;  // one graph of kGroup steps
 
     template <typename T>
     T* up(const std::vector<T>& v) {
@@ -157,9 +174,12 @@ struct DiffSolver {
         if (stream) cudaStreamDestroy(stream);
     }
 
-    void launch() {
-        k_diff_face<<<(F + kFaceBlock - 1) / kFaceBlock, kFaceBlock, 0, stream>>>(a);
-        k_diff_cell<<<nblk, kCellBlock, 0, stream>>>(a);
+    void launch(int n) {
+        for (int i = 0; i < n; ++i) {
+            k_diff_face<<<(F + kFaceBlock - 1) / kFaceBlock, kFaceBlock, 0, stream>>>(a);
+            k_diff_cell<<<nblk, kCellBlock, 0, stream>>>(a, i);
+        }
+        if (n > 0) k_diff_norms<<<1, 32 * kGroup, 0, stream>>>(a, n, nblk);
     }
 };
 
@@ -208,7 +228,8 @@ int fv_diffusion_create(fv_mesh_t mesh, double alpha, double dt, double initial_
         FV_CUDA(cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking));
         // Face distances with the reference's own formula
         // (src/UnstructuredFVMSolver.cpp:58-62, :122-125), device face order.
-        std::vector<double> area(s.F), dist(s.F);
+        std::vector<double> area(s.F), coef(s.N);
+        std::vector<double2> dist(s.F);
         for (int i = 0; i < s.F; ++i) {
             int f = h.fperm[i];
             area[i] = h.farea[f];
@@ -220,8 +241,10 @@ int fv_diffusion_create(fv_mesh_t mesh, double alpha, double dt, double initial_
                 dx = h.fxm[f] - h.cx[h.fl[f]];
                 dy = h.fym[f] - h.cy[h.fl[f]];
             }
-            dist[i] = std::sqrt(dx * dx + dy * dy);
+            const double d = std::sqrt(dx * dx + dy * dy);
+            dist[i] = make_double2(d, d > 1e-100 && d < 1e100 ? 1.0 / d : 0.0);
         }
+        for (int i = 0; i < s.N; ++i) coef[i] = dt / h.d_vol[i];
         fvgb::DiffArgs& a = s.a;
         a.n_cells = s.N;
         a.n_faces = s.F;
@@ -232,16 +255,15 @@ int fv_diffusion_create(fv_mesh_t mesh, double alpha, double dt, double initial_
         a.fdist = s.up(dist);
         a.cf_off = s.up(h.d_cf_off);
         a.cf = s.up(h.d_cf);
-        a.vol = s.up(h.d_vol);
+        a.coef = s.up(coef);
         a.phi = s.alloc<double>(s.N);
         a.ff = s.alloc<double>(s.F);
-        a.partials = s.alloc<double>(s.nblk);
+        a.partials = s.alloc<double>((size_t)fvgb::kGroup * s.nblk);
         a.hist_cap = 1 << 16;
         a.hist = s.alloc<double>(a.hist_cap);
         a.ctl = s.alloc<fvgb::StepCtl>(1);
         FV_CUDA(cudaMemsetAsync(a.ctl, 0, sizeof(fvgb::StepCtl), s.stream));
         a.alpha = alpha;
-        a.dt = dt;
         for (int p = 0; p < h.n_patches; ++p) {
             if (patch_type[p] != 0 && patch_type[p] != 1) raise(FV_ERR_BAD_ARG, "patch type must be 0 or 1");
             a.ptype[p] = patch_type[p];
@@ -273,23 +295,26 @@ int fv_diffusion_step(fv_diffusion_t d, int32_t n, double* history) {
         if (s.graph.empty()) {
             cudaGraph_t g;
             FV_CUDA(cudaStreamBeginCapture(s.stream, cudaStreamCaptureModeThreadLocal));
-            for (int i = 0; i < 16; ++i) s.launch();
+            s.launch(fvgb::kGroup);
             FV_CUDA(cudaStreamEndCapture(s.stream, &g));
             cudaGraphExec_t ge;
             FV_CUDA(cudaGraphInstantiate(&ge, g, 0));
             cudaGraphDestroy(g);
             s.graph.push_back(ge);
         }
-        for (int i = 0; i < n / 16; ++i) FV_CUDA(cudaGraphLaunch(s.graph[0], s.stream));
-        for (int i = 0; i < n % 16; ++i) s.launch();
+        for (int i = 0; i < n / fvgb::kGroup; ++i) FV_CUDA(cudaGraphLaunch(s.graph[0], s.stream));
+        s.launch(n % fvgb::kGroup);
         FV_CUDA(cudaGetLastError());
         fvgb::StepCtl c;
         FV_CUDA(cudaMemcpyAsync(&c, s.a.ctl, sizeof(c), cudaMemcpyDeviceToHost, s.stream));
         FV_CUDA(cudaStreamSynchronize(s.stream));
         if (history && n > 0) {
-            std::vector<double> all(s.a.hist_cap);
-            FV_CUDA(cudaMemcpy(all.data(), s.a.hist, sizeof(double) * all.size(), cudaMemcpyDeviceToHost));
-            for (int i = 0; i < n; ++i) history[i] = all[(c.step - n + i) % s.a.hist_cap];
+            // rows (step mod capacity), in one or two pieces of the ring
+            const int cap = s.a.hist_cap, r0 = (c.step - n) % cap, k = std::min(n, cap - r0);
+            FV_CUDA(cudaMemcpyAsync(history, s.a.hist + r0, sizeof(double) * k, cudaMemcpyDeviceToHost, s.stream));
+            if (n > k)
+                FV_CUDA(cudaMemcpyAsync(history + k, s.a.hist, sizeof(double) * (n - k), cudaMemcpyDeviceToHost, s.stream));
+            FV_CUDA(cudaStreamSynchronize(s.stream));
         }
         if (c.nonfinite) raise(FV_ERR_NONFINITE, "non-finite residual norm");
     });

@@ -98,6 +98,19 @@ __device__ __forceinline__ double rcp_nr3(double x) {
     return fma(y, fma(r, r, r), y);
 }
 
+// x / d.x, correctly rounded, from y = d.y = 1 / d.x correctly rounded: x y is
+// within two ulps, its first correction within one, and a correction with an
+// exact remainder of such a quotient is the rounded quotient (Markstein, IBM
+// J. Res. Dev. 34(1), 1990).  Exponents that could over- or underflow in
+// between take the division.
+__device__ __forceinline__ double quotient(double x, double2 d) {
+    const unsigned e = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
+    if (d.y == 0.0 || e - 300u > 1400u) return x / d.x;
+    double q = x * d.y;
+    q = fma(fma(-d.x, q, x), d.y, q);
+    return fma(fma(-d.x, q, x), d.y, q);
+}
+
 // x^k for x near 1 with a short chain of dependent FP64 operations (for
 // boundary states on a critical path; the library pow is a much longer
 // chain).  ln x = 2 atanh z with z = (x - 1) / (x + 1) (x - 1 is exact for
