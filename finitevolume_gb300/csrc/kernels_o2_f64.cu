@@ -48,9 +48,18 @@ void update(const O2Args& a, int local, int bs, cudaStream_t s) {
 namespace fvgb {
 namespace o2 {
 
-void launch_batch_norms(const O2Args& a, int n_inst, const int* inst_off, double* inst_norms, int* inst_iter,
-                        int* active, double tol, cudaStream_t s) {
-    ::fast::k_batch_norms<<<n_inst, 256, 0, s>>>(a, inst_off, inst_norms, inst_iter, active, tol);
+void launch_batch_norms(const O2Args& a, int n_inst, const BatchNorms& b, double tol, cudaStream_t s) {
+    // 65,535 instances a launch (grid limit)
+    for (int i0 = 0; i0 < n_inst; i0 += 65535) {
+        BatchNorms q = b;
+        q.inst_off += i0;
+        q.active += i0;
+        q.iter += i0;
+        q.norms += 4 * (size_t)i0;
+        q.part += 4 * (size_t)i0 * b.chunks;
+        q.done += i0;
+        ::fast::k_batch_norms<<<dim3(b.chunks, n_inst - i0 < 65535 ? n_inst - i0 : 65535), 256, 0, s>>>(a, q, tol);
+    }
 }
 
 void launch_fix_geom(const O2Args& a, int4* fxa, int4* fxr, int* fxs, cudaStream_t s) {

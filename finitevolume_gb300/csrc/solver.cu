@@ -285,6 +285,15 @@ void Solver::init(const HostMesh& hm, const fv_bc_t* bcs, int n_bcs, double g, d
         inst_fs = dupload(inst_fs_host, owned);
         inst_norms = dupload(std::vector<double>(4 * (size_t)n_inst, 0.0), owned);
         r2 = dalloc<double4_32a>(N, owned);
+        int most = 1;
+        for (int i = 0; i < n_inst; ++i) most = std::max(most, group_off[i + 1] - group_off[i]);
+        bn.inst_off = inst_off;
+        bn.active = active;
+        bn.iter = inst_iter;
+        bn.norms = inst_norms;
+        bn.chunks = (most + kNormChunk - 1) / kNormChunk;
+        bn.part = dalloc<double>(4 * (size_t)n_inst * bn.chunks, owned);
+        bn.done = dupload(std::vector<unsigned int>(n_inst, 0u), owned);
     }
 
     if (viscous) {
@@ -579,7 +588,7 @@ void Solver::launch_step(std::vector<int>* classes, std::vector<cudaEvent_t>* ev
         }
     }
     if (batch) {
-        o2::launch_batch_norms(a, n_inst, inst_off, inst_norms, inst_iter, active, tol, stream);
+        o2::launch_batch_norms(a, n_inst, bn, tol, stream);
         mark(2);
     }
 }

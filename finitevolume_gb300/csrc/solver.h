@@ -87,6 +87,7 @@ struct Solver {
     std::vector<double> inst_fs_host;   // the same, host copy (coarse multigrid levels)
     double* inst_norms = nullptr;
     double4_32a* r2 = nullptr;
+    BatchNorms bn{};
     double tol = -1.0;                // density-norm tolerance; < 0 never freezes
 
     // Navier-Stokes path (and RANS-SA on top of it)

@@ -199,6 +199,19 @@ struct O2Config {
     int blk_grad, blk_face, blk_cell;
 };
 
+// Per-instance norms of a batched solve: outputs, and per instance the
+// partial sums of its chunks of kNormChunk cells and the count of those done.
+struct BatchNorms {
+    const int* inst_off;  // [n_inst + 1]
+    int* active;
+    int* iter;
+    double* norms;        // [4 n_inst]
+    double* part;         // [4 n_inst * chunks]
+    unsigned int* done;   // [n_inst], zero between launches
+    int chunks;           // of the largest instance
+};
+constexpr int kNormChunk = 1024;
+
 constexpr int kCellBlock = 256;
 constexpr int kFaceBlock = 256;
 constexpr int kMaxBlock = 512;  // largest tunable block of the second-order kernels
@@ -216,8 +229,7 @@ void launch_residual_f64(const O2Args& a, cudaStream_t s);
 void launch_residual_f32(const O2Args& a, cudaStream_t s);
 // the fixed-point gradient geometry (O2Args::fxa, fxr, fxs) from a.lsq, a.erf
 void launch_fix_geom(const O2Args& a, int4* fxa, int4* fxr, int* fxs, cudaStream_t s);
-void launch_batch_norms(const O2Args& a, int n_inst, const int* inst_off, double* inst_norms, int* inst_iter,
-                        int* active, double tol, cudaStream_t s);
+void launch_batch_norms(const O2Args& a, int n_inst, const BatchNorms& b, double tol, cudaStream_t s);
 }  // namespace o2
 
 // part 0: face pass, 1: cell pass.
