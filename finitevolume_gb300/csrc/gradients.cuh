@@ -75,6 +75,11 @@ __device__ __forceinline__ void cell_gradient(const GradDev& g, int c, const Phi
     }
 }
 
+// The viscous solvers' default build keeps these arrays in layouts of its own
+// (viscous_fast.cuh): lsq_w folded with lsq_inv, gg = (outward nx * length / V,
+// outward ny * length / V, owner weight, 0), fgrad = 1/nd, length, kx, ky,
+// w_L, nd, nx, ny.
+
 struct FaceGrad {
     double dphidn, gx, gy;  // corrected normal derivative, corrected full gradient
 };
@@ -102,6 +107,13 @@ __device__ __forceinline__ FaceGrad face_gradient(const double* fg, bool boundar
     r.gx = gfx + delta * nx;
     r.gy = gfy + delta * ny;
     return r;
+}
+
+// The same from the default build's fgrad row.
+__device__ __forceinline__ FaceGrad face_gradient_fast(const double* fg, bool boundary, double phiL, double phiR,
+                                                       double gLx, double gLy, double gRx, double gRy) {
+    const double q[8] = {1.0, 1.0, fg[2], fg[3], fg[4], fg[5], fg[6], fg[7]};
+    return face_gradient(q, boundary, 0.0, (phiR - phiL) * fg[0], gLx, gLy, gRx, gRy);
 }
 
 }  // namespace fvgb

@@ -17,29 +17,22 @@
 #ifdef FV_NS_FAST
 #define FV_KNS nsk_fast
 #define FV_NS_FN(name) name##_fast
+#define FV_NS_FACE_GRADIENT fvgb::face_gradient_fast
 #else
 #define FV_KNS nsk
 #define FV_NS_FN(name) name
+#define FV_NS_FACE_GRADIENT fvgb::face_gradient
 #endif
 #include "euler_o1.cuh"
 #include "gradients.cuh"
 #include "ns.h"
+#ifdef FV_NS_FAST
+#include "viscous_fast.cuh"
+#endif
 
 namespace FV_KNS {
 
 using fvgb::NSArgs;
-
-__global__ void __launch_bounds__(fvgb::kCellBlock) k_ns_prim(const NSArgs a) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= a.g.n_cells) return;
-    const St s = ld_state(a.U, c);
-    double4_32a w;
-    w.x = s.ru / s.r;
-    w.y = s.rv / s.r;
-    w.z = pressure(s, a.gamma) / (s.r * a.gas_constant);
-    w.w = 0.0;
-    a.prim[c] = w;
-}
 
 // build_boundary_fields (src/NavierStokesFVMSolver.cpp:55-84) for one
 // boundary face owned by cell cl, variable k (0 u, 1 v, 2 T).
@@ -52,6 +45,103 @@ __device__ __forceinline__ double boundary_field(const NSArgs& a, int face, int 
     }
     const double4_32a w = a.prim[cl];
     return k == 0 ? w.x : (k == 1 ? w.y : w.z);
+}
+
+#ifdef FV_NS_FAST
+// Default build (viscous_fast.cuh).  Bound: FP64 issue, about 75 instructions
+// a face (370 in the strict order), 55 a cell for the gradients (155).
+__global__ void __launch_bounds__(fvgb::kCellBlock) k_ns_prim(const NSArgs a) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c < a.g.n_cells) a.prim[c] = prim_visc(ld_state(a.U, c), a.gamma, a.inv_R);
+}
+
+__global__ void __launch_bounds__(fvgb::kCellBlock) k_ns_grad(const NSArgs a) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= a.g.n_cells) return;
+    double gx[3], gy[3];
+    cell_gradient_fast<3>(
+        a.g, a.prim, c,
+        [&](int f, const double4_32a&) {
+            double4_32a w;
+            w.x = boundary_field(a, f, c, 0);
+            w.y = boundary_field(a, f, c, 1);
+            w.z = boundary_field(a, f, c, 2);
+            w.w = 0.0;
+            return w;
+        },
+        gx, gy);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) a.grad[3 * c + k] = make_double2(gx[k], gy[k]);
+}
+
+template <int FLUX>
+__global__ void __launch_bounds__(fvgb::kFaceBlock) k_ns_face(const NSArgs a) {
+    // from the last face down: the boundary faces start first
+    const int f = (gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x;
+    double cand = DBL_MAX;
+    if (f < a.g.n_faces) {
+        const int cl = a.fl[f], cr = a.g.fr[f];
+        const bool bnd = cr < 0;
+        const double* fg = a.g.fgrad + 8 * (size_t)f;
+        const double4_32a wl = a.prim[cl];
+        double4_32a wr = bnd ? wl : a.prim[cr];
+        const double rL = a.U[cl].r, rR = bnd ? rL : a.U[cr].r;
+        St F;
+        double uR, vR;
+        const double smax = inviscid<FLUX>(a, f, cl, cr, fg, rL, wl, rR, wr, F, uR, vR);
+        // compute_dt: Smax + 2 nu / nd with the larger of the cells' mu / rho
+        const double nu = (a.mu > 0.0) ? a.mu * rmax(wl.w, wr.w) : 0.0;
+        cand = (a.ctl->cfl * fg[5]) * fvconv::rcp_nr3(smax + 2.0 * nu * fg[0]);
+        const int p = bnd ? a.fpatch[f] : 0;
+        if (!bnd || a.bc.type[p] == BC_NOSLIP) {
+            if (bnd) {
+                wr.x = boundary_field(a, f, cl, 0);
+                wr.y = boundary_field(a, f, cl, 1);
+                wr.z = boundary_field(a, f, cl, 2);
+            }
+            const int q = bnd ? cl : cr;
+            double ux, uy, du, vx, vy, dv, tx, ty, unused0, unused1, dT = 0.0;
+            face_normal_gradient(fg, bnd, wr.x - wl.x, a.grad[3 * cl], a.grad[3 * q], ux, uy, du);
+            face_normal_gradient(fg, bnd, wr.y - wl.y, a.grad[3 * cl + 1], a.grad[3 * q + 1], vx, vy, dv);
+            if (!bnd || a.bc.isothermal[p])
+                face_normal_gradient(fg, bnd, wr.z - wl.z, a.grad[3 * cl + 2], a.grad[3 * q + 2], unused0, unused1, dT);
+            traction(fg, ux, uy, du, vx, vy, dv, tx, ty);
+            const double am = fg[1] * a.mu;
+            tx *= am;
+            ty *= am;
+            const double us = bnd ? wr.x : 0.5 * (wl.x + wr.x), vs = bnd ? wr.y : 0.5 * (wl.y + wr.y);
+            F.ru -= tx;
+            F.rv -= ty;
+            F.E -= us * tx + vs * ty + (fg[1] * a.kcond) * dT;
+        }
+        st_state(a.ff, f, F);
+    }
+    min_candidate(cand, a.ctl);
+}
+
+// The Euler cell pass with the fluxes summed on the integer pipe.
+__global__ void __launch_bounds__(fvgb::kCellBlock) k_ns_cell(const O1Args a) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+    if (c < a.m.n_cells) {
+        const double dt = __longlong_as_double((long long)a.ctl->dt_bits);
+        const St R = gather_any(a.ff, a.m.cf, a.m.cf_off[c], a.m.cf_off[c + 1]);
+        s0 = R.r * R.r; s1 = R.ru * R.ru; s2 = R.rv * R.rv; s3 = R.E * R.E;
+        st_state(a.U, c, ld_state(a.U, c) + (dt * fvconv::rcp_nr3(a.m.vol[c])) * R);
+    }
+    finish_norms(s0, s1, s2, s3, a.ctl, a.partials, a.hist, a.hist_cap);
+}
+#else
+__global__ void __launch_bounds__(fvgb::kCellBlock) k_ns_prim(const NSArgs a) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= a.g.n_cells) return;
+    const St s = ld_state(a.U, c);
+    double4_32a w;
+    w.x = s.ru / s.r;
+    w.y = s.rv / s.r;
+    w.z = pressure(s, a.gamma) / (s.r * a.gas_constant);
+    w.w = 0.0;
+    a.prim[c] = w;
 }
 
 __global__ void __launch_bounds__(fvgb::kCellBlock) k_ns_grad(const NSArgs a) {
@@ -154,6 +244,8 @@ __global__ void __launch_bounds__(fvgb::kFaceBlock) k_ns_face(const NSArgs a) {
     }
 }
 
+#endif
+
 // compute_wall_traction for one wall face (src/WallTraction.cpp:110-139):
 // out = (tau_wall, p of the owner cell).
 __global__ void k_ns_wall(const NSArgs a, const int* __restrict__ faces, int n, double2* __restrict__ out) {
@@ -164,8 +256,8 @@ __global__ void k_ns_wall(const NSArgs a, const int* __restrict__ faces, int n, 
     const double* fg = a.g.fgrad + 8 * (size_t)f;
     const double4_32a wl = a.prim[cl];
     const double2 gu0 = a.grad[3 * cl], gv0 = a.grad[3 * cl + 1];
-    const fvgb::FaceGrad fu = fvgb::face_gradient(fg, true, wl.x, boundary_field(a, f, cl, 0), gu0.x, gu0.y, 0.0, 0.0);
-    const fvgb::FaceGrad fv = fvgb::face_gradient(fg, true, wl.y, boundary_field(a, f, cl, 1), gv0.x, gv0.y, 0.0, 0.0);
+    const fvgb::FaceGrad fu = FV_NS_FACE_GRADIENT(fg, true, wl.x, boundary_field(a, f, cl, 0), gu0.x, gu0.y, 0.0, 0.0);
+    const fvgb::FaceGrad fv = FV_NS_FACE_GRADIENT(fg, true, wl.y, boundary_field(a, f, cl, 1), gv0.x, gv0.y, 0.0, 0.0);
     const double mu = a.mu;
     const double div_v = fu.gx + fv.gy;
     const double tau_xx = mu * (2.0 * fu.gx - (2.0 / 3.0) * div_v);
@@ -193,7 +285,11 @@ void FV_NS_FN(ns_launch_step)(const NSArgs& a, const O1Args& cell, cudaStream_t 
         case 2: FV_KNS::k_ns_face<2><<<fb, kFaceBlock, 0, s>>>(a); break;
         default: FV_KNS::k_ns_face<0><<<fb, kFaceBlock, 0, s>>>(a); break;
     }
+#ifdef FV_NS_FAST
+    FV_KNS::k_ns_cell<<<cb, kCellBlock, 0, s>>>(cell);
+#else
     FV_KNS::k_cell_o1<false><<<cb, kCellBlock, 0, s>>>(cell);
+#endif
 }
 
 void FV_NS_FN(ns_launch_wall)(const NSArgs& a, const int* faces, int n, double2* out, cudaStream_t s) {

@@ -13,12 +13,15 @@ struct NSArgs {
     const double4_32a* fgeom;  // nx, ny, length, CFL length
     St* U;
     St* ff;
-    double4_32a* prim;         // u, v, T, unused
+    double4_32a* prim;         // u, v, T, and 1/rho (default build) or unused
     double2* grad;             // 3 per cell: grad u, grad v, grad T
     StepCtl* ctl;
     BCTable bc;
     double gamma, gas_constant, mu, kcond, exact_tol;
     int exact_max_iter, flux;
+    int fixed;                 // default build: inviscid fluxes in fixed point (fixed.cuh)
+    fvfix::FluxConst fxc;
+    double inv_R;              // 1 / gas_constant
 };
 
 // Strict (no FMA contraction, reference evaluation order) and _fast

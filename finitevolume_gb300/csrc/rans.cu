@@ -22,13 +22,18 @@
 #ifdef FV_NS_FAST
 #define FV_KNS ransk_fast
 #define FV_NS_FN(name) name##_fast
+#define FV_NS_FACE_GRADIENT fvgb::face_gradient_fast
 #else
 #define FV_KNS ransk
 #define FV_NS_FN(name) name
+#define FV_NS_FACE_GRADIENT fvgb::face_gradient
 #endif
 #include "euler_o1.cuh"
 #include "gradients.cuh"
 #include "rans.h"
+#ifdef FV_NS_FAST
+#include "viscous_fast.cuh"
+#endif
 
 namespace FV_KNS {
 
@@ -43,6 +48,71 @@ __device__ __forceinline__ double sa_fv1(double nut, double nu, const double* c)
 }
 __device__ __forceinline__ double sa_nut(double nut, double nu, const double* c) { return nut * sa_fv1(nut, nu, c); }
 
+#ifdef FV_NS_FAST
+// Default build (viscous_fast.cuh).  Bound: FP64 issue, about 105
+// instructions a face (430 in the strict order), 65 a cell for the gradients
+// (155), 90 for the cell pass (245), 27 for the primitives (67).
+
+// nu_t = nut fv1(chi) with chi = nut / nu
+__device__ __forceinline__ double sa_fv1_chi(double chi, double cv1_3) {
+    const double chi3 = chi * chi * chi;
+    return chi3 * fvconv::rcp_nr3(chi3 + cv1_3);
+}
+__device__ __forceinline__ double sa_nut_fast(double nut, double chi, double cv1_3) {
+    return nut <= 0.0 ? 0.0 : nut * sa_fv1_chi(chi, cv1_3);
+}
+
+// z^(-1/6): a float estimate y (within 2^-20), then y (1 - e)^(-1/6) with e =
+// 1 - z y^6 as a series to e^3 (e below 2^-17, the next term below 2^-70).
+__device__ __forceinline__ double inv_root6(double z) {
+    const int e = fvfix::biased(fvfix::hi_word(z));
+    if ((unsigned)(e - 963) > 160u) return 1.0 / cbrt(sqrt(z));  // outside [2^-60, 2^100]
+    float l, s;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(fvconv::d2f(z)));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(l * (-1.0f / 6.0f)));
+    const double y = fvconv::f2d(s);
+    const double y2 = y * y, y6 = y2 * y2 * y2;
+    const double r = fma(-z, y6, 1.0);
+    return fma(y * r, fma(r, fma(r, 91.0 / 1296.0, 7.0 / 72.0), 1.0 / 6.0), y);
+}
+
+// sa_source of the strict build with its divisions as reciprocals shared
+// between terms; chi = nut / nu.
+__device__ __forceinline__ double sa_source(const RansArgs& a, double nut, double chi, double omega, double d,
+                                            double gx, double gy) {
+    const double cb1 = a.sa[0], cw2 = a.sa[4], cv2 = a.sa[7], cv3 = a.sa[8];
+    const bool pos = nut > 0.0;
+    chi = pos ? chi : 0.0;
+    const double fv1 = pos ? sa_fv1_chi(chi, a.cv1_3) : 0.0;
+    const double fv2 = 1.0 - chi * fvconv::rcp_nr3(1.0 + chi * fv1);
+    const double id = fvconv::rcp_nr3(d);
+    const double q = nut * ((id * id) * a.inv_kappa2), s_bar = q * fv2;
+    double s_tilde;
+    if (s_bar >= -cv2 * omega) s_tilde = omega + s_bar;
+    else s_tilde = omega + omega * (cv2 * cv2 * omega + cv3 * s_bar) / ((cv3 - 2.0 * cv2) * omega - s_bar);
+    double source = cb1 * s_tilde * nut;
+    if (pos) {
+        const double r = rmin(q * fvconv::rcp_nr3(rmax(s_tilde, 1e-10)), 10.0);
+        const double r2 = r * r, g = r + cw2 * (r2 * r2 * r2 - r), g2 = g * g;
+        // ((1 + cw3^6) / (g^6 + cw3^6))^(1/6)
+        const double fw = g * inv_root6((g2 * g2 * g2 + a.cw3_6) * a.inv_1_cw3_6);
+        const double nd = nut * id;
+        source -= a.cw1 * fw * nd * nd;
+    }
+    return source + a.cb2_sigma * (gx * gx + gy * gy);
+}
+
+__global__ void __launch_bounds__(fvgb::kCellBlock) k_sa_prim(const RansArgs a) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= a.ns.g.n_cells) return;
+    const St s = ld_state(a.ns.U, c);
+    double4_32a w = prim_visc(s, a.ns.gamma, a.ns.inv_R);
+    const double nu = a.ns.mu * w.w;
+    w.w = a.nut[c];
+    a.ns.prim[c] = w;
+    a.nu[c] = make_double2(nu, sa_nut_fast(w.w, w.w * (s.r * a.inv_mu), a.cv1_3));
+}
+#else
 // constants c[]: cb1, cb2, sigma, kappa, cw2, cw3, cv1, cv2, cv3; cw3_6 = cw3^6.
 // The model's integer powers r^6, g^6 are formed by three multiplies and
 // its sixth root as cbrt(sqrt(.)): within a few ulp of pow(), at a small
@@ -108,6 +178,8 @@ __global__ void __launch_bounds__(fvgb::kCellBlock) k_sa_prim(const RansArgs a) 
     a.nu[c] = make_double2(nu, sa_nut(w.w, nu, a.sa));
 }
 
+#endif
+
 // build_boundary_fields / build_boundary_nut for one boundary face owned by
 // cell cl, variable k (0 u, 1 v, 2 T, 3 nu-tilde).
 __device__ __forceinline__ double boundary_field(const RansArgs& a, int face, int cl, int k) {
@@ -127,6 +199,91 @@ __device__ __forceinline__ double boundary_field(const RansArgs& a, int face, in
     return k == 0 ? w.x : (k == 1 ? w.y : w.z);
 }
 
+#ifdef FV_NS_FAST
+__device__ __forceinline__ double4_32a boundary_values(const RansArgs& a, int f, int cl) {
+    double4_32a w;
+    w.x = boundary_field(a, f, cl, 0);
+    w.y = boundary_field(a, f, cl, 1);
+    w.z = boundary_field(a, f, cl, 2);
+    w.w = boundary_field(a, f, cl, 3);
+    return w;
+}
+
+__global__ void __launch_bounds__(fvgb::kCellBlock) k_sa_grad(const RansArgs a) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= a.ns.g.n_cells) return;
+    double gx[4], gy[4];
+    cell_gradient_fast<4>(a.ns.g, a.ns.prim, c, [&](int f, const double4_32a&) { return boundary_values(a, f, c); },
+                          gx, gy);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) a.grad[4 * c + k] = make_double2(gx[k], gy[k]);
+}
+
+template <int FLUX>
+__global__ void __launch_bounds__(fvgb::kFaceBlock) k_sa_face(const RansArgs a) {
+    // from the last face down: the boundary faces start first
+    const int f = (gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x;
+    double cand = DBL_MAX;
+    if (f < a.ns.g.n_faces) {
+        const fvgb::NSArgs& n = a.ns;
+        const int cl = n.fl[f], cr = n.g.fr[f];
+        const bool bnd = cr < 0;
+        const double* fg = n.g.fgrad + 8 * (size_t)f;
+        const double area = fg[1];
+        const double4_32a wl = n.prim[cl];
+        double4_32a wr = bnd ? wl : n.prim[cr];
+        const double2 nuL = a.nu[cl], nuR = bnd ? nuL : a.nu[cr];
+        const double rL = n.U[cl].r, rR = bnd ? rL : n.U[cr].r;
+        St F;
+        double uR, vR;
+        const double smax = inviscid<FLUX>(n, f, cl, cr, fg, rL, wl, rR, wr, F, uR, vR);
+        const double nu_eff = ((n.mu > 0.0) ? rmax(nuL.x, nuR.x) : 0.0) + rmax(nuL.y, nuR.y);
+        cand = (n.ctl->cfl * fg[5]) * fvconv::rcp_nr3(smax + 2.0 * nu_eff * fg[0]);
+
+        // nu-tilde upwinded by the mean velocity of the inviscid state pair
+        const double Vn = 0.5 * ((wl.x + uR) * fg[6] + (wl.y + vR) * fg[7]);
+        if (bnd) wr = boundary_values(a, f, cl);
+        double nut_flux = Vn * ((Vn >= 0.0) ? wl.w : wr.w) * area;
+
+        const int p = bnd ? n.fpatch[f] : 0;
+        if (!bnd || n.bc.type[p] == BC_NOSLIP) {
+            const int q = bnd ? cl : cr;
+            double ux, uy, du, vx, vy, dv, tx, ty, unused0, unused1, dT = 0.0, dnt;
+            face_normal_gradient(fg, bnd, wr.x - wl.x, a.grad[4 * cl], a.grad[4 * q], ux, uy, du);
+            face_normal_gradient(fg, bnd, wr.y - wl.y, a.grad[4 * cl + 1], a.grad[4 * q + 1], vx, vy, dv);
+            if (!bnd || n.bc.isothermal[p])
+                face_normal_gradient(fg, bnd, wr.z - wl.z, a.grad[4 * cl + 2], a.grad[4 * q + 2], unused0, unused1, dT);
+            face_normal_gradient(fg, bnd, wr.w - wl.w, a.grad[4 * cl + 3], a.grad[4 * q + 3], unused0, unused1, dnt);
+            traction(fg, ux, uy, du, vx, vy, dv, tx, ty);
+            const double nt_R = bnd ? sa_nut_fast(wr.w, wr.w * (rL * a.inv_mu), a.cv1_3) : nuR.y;
+            const double turb = 0.5 * (rL * nuL.y + rR * nt_R);
+            const double am = area * (n.mu + turb);
+            tx *= am;
+            ty *= am;
+            const double us = bnd ? wr.x : 0.5 * (wl.x + wr.x), vs = bnd ? wr.y : 0.5 * (wl.y + wr.y);
+            F.ru -= tx;
+            F.rv -= ty;
+            F.E -= us * tx + vs * ty + (area * (a.k_lam + a.cp_prt * turb)) * dT;
+            nut_flux -= a.half_inv_sigma * ((nuL.x + nuR.x) + (nuL.y + nt_R)) * (dnt * area);
+        }
+        st_state(n.ff, f, F);
+        a.nut_ff[f] = nut_flux;
+    }
+    min_candidate(cand, a.ns.ctl);
+}
+
+template <int N> __device__ __forceinline__ double gather_nut(const double* ff, const int* cf) {
+    double x[N];
+    int neg[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const int ent = __ldg(cf + i);
+        x[i] = __ldg(ff + (ent >> 1));
+        neg[i] = ent;
+    }
+    return fvfix::signed_sum<N>(x, neg);
+}
+#else
 __global__ void __launch_bounds__(fvgb::kCellBlock) k_sa_grad(const RansArgs a) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= a.ns.g.n_cells) return;
@@ -255,6 +412,8 @@ __global__ void __launch_bounds__(fvgb::kFaceBlock) k_sa_face(const RansArgs a) 
     }
 }
 
+#endif
+
 // Cell pass: gathers, SA sources, five norms (deterministic last-block
 // fold, as the Euler cell pass), U and nu-tilde updates with the global dt.
 __global__ void __launch_bounds__(fvgb::kCellBlock) k_sa_cell(const RansArgs a) {
@@ -262,6 +421,24 @@ __global__ void __launch_bounds__(fvgb::kCellBlock) k_sa_cell(const RansArgs a) 
     double s[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     fvgb::StepCtl* ctl = a.ns.ctl;
     if (c < a.ns.g.n_cells) {
+#ifdef FV_NS_FAST
+        const int e0 = a.cf_off[c], e1 = a.cf_off[c + 1];
+        const St R = gather_any(a.ns.ff, a.cf, e0, e1);
+        double Rn = 0.0;
+        if (e1 - e0 == 4) Rn = gather_nut<4>(a.nut_ff, a.cf + e0);
+        else if (e1 - e0 == 3) Rn = gather_nut<3>(a.nut_ff, a.cf + e0);
+        else
+            for (int e = e0; e < e1; ++e) Rn += (a.cf[e] & 1) ? -a.nut_ff[a.cf[e] >> 1] : a.nut_ff[a.cf[e] >> 1];
+        const double2 gu = a.grad[4 * c], gv = a.grad[4 * c + 1], gn = a.grad[4 * c + 3];
+        const double vol = a.vol[c], nut = a.nut[c];
+        const St u = ld_state(a.ns.U, c);
+        Rn += vol * sa_source(a, nut, nut * (u.r * a.inv_mu), fabs(gv.x - gu.y), a.walld[c], gn.x, gn.y);
+        s[0] = R.r * R.r; s[1] = R.ru * R.ru; s[2] = R.rv * R.rv; s[3] = R.E * R.E; s[4] = Rn * Rn;
+        const double k = __longlong_as_double((long long)ctl->dt_bits) * fvconv::rcp_nr3(vol);
+        st_state(a.ns.U, c, u + k * R);
+        a.nut[c] = nut + k * Rn;
+    }
+#else
         St R = st_make(0.0, 0.0, 0.0, 0.0);
         double Rn = 0.0;
         for (int e = a.cf_off[c]; e < a.cf_off[c + 1]; ++e) {
@@ -282,13 +459,22 @@ __global__ void __launch_bounds__(fvgb::kCellBlock) k_sa_cell(const RansArgs a) 
         st_state(a.ns.U, c, u + k * R);
         a.nut[c] = a.nut[c] + k * Rn;
     }
+#endif
     __shared__ double red[fvgb::kCellBlock / 32][5];
     __shared__ bool last;
     const int w = threadIdx.x >> 5;
+#ifdef FV_NS_FAST
+    const double s4 = warp_sum4(s[0], s[1], s[2], s[3]);
+    s[4] = warp_sum(s[4]);
+    const int lane = threadIdx.x & 31;
+    if ((lane & 7) == 0) red[w][lane >> 3] = s4;
+    if (lane == 0) red[w][4] = s[4];
+#else
 #pragma unroll
     for (int q = 0; q < 5; ++q) s[q] = warp_sum(s[q]);
     if ((threadIdx.x & 31) == 0)
         for (int q = 0; q < 5; ++q) red[w][q] = s[q];
+#endif
     __syncthreads();
     if (threadIdx.x < 5) {
         double v = 0.0;
@@ -343,8 +529,8 @@ __global__ void k_sa_wall(const RansArgs a, const int* __restrict__ faces, int n
     const double* fg = a.ns.g.fgrad + 8 * (size_t)f;
     const double4_32a wl = a.ns.prim[cl];
     const double2 gu0 = a.grad[4 * cl], gv0 = a.grad[4 * cl + 1];
-    const fvgb::FaceGrad fu = fvgb::face_gradient(fg, true, wl.x, boundary_field(a, f, cl, 0), gu0.x, gu0.y, 0.0, 0.0);
-    const fvgb::FaceGrad fv = fvgb::face_gradient(fg, true, wl.y, boundary_field(a, f, cl, 1), gv0.x, gv0.y, 0.0, 0.0);
+    const fvgb::FaceGrad fu = FV_NS_FACE_GRADIENT(fg, true, wl.x, boundary_field(a, f, cl, 0), gu0.x, gu0.y, 0.0, 0.0);
+    const fvgb::FaceGrad fv = FV_NS_FACE_GRADIENT(fg, true, wl.y, boundary_field(a, f, cl, 1), gv0.x, gv0.y, 0.0, 0.0);
     const St s = ld_state(a.ns.U, cl);
     const double mu = a.ns.mu + s.r * a.nu[cl].y;
     const double div_v = fu.gx + fv.gy;

@@ -26,6 +26,9 @@ struct RansArgs {
     double cw3_6;          // cw3^6, formed on the host by std::pow
     double cp, prandtl, prandtl_t;
     double k_lam;          // cp * mu / Pr, formed on the host in that order
+    // quotients of the constants for the default build: 1/mu, cv1^3,
+    // 1/kappa^2, cw1, cb2/sigma, 1/(1 + cw3^6), 1/(2 sigma), cp/Pr_t
+    double inv_mu, cv1_3, inv_kappa2, cw1, cb2_sigma, inv_1_cw3_6, half_inv_sigma, cp_prt;
 };
 
 void rans_wall_distance(const RansArgs& a, const double4_32a* seg, int n_seg, cudaStream_t s);

@@ -309,7 +309,31 @@ void Solver::init(const HostMesh& hm, const fv_bc_t* bcs, int n_bcs, double g, d
             if (!(hg.fgrad[8 * (size_t)i + 5] > 0.0))
                 raise(FV_ERR_BAD_MESH, "face " + std::to_string(hm.fperm[i]) +
                                            ": neighbouring centroids on one side (overlapping cells)");
+        if (!opt.strict) {
+            // the default build's layouts (gradients.cuh), divisions prepared
+            for (int c = 0; c < N; ++c)
+                for (int e = hm.d_cf_off[c]; e < hm.d_cf_off[c + 1]; ++e) {
+                    double* q = &hg.gg[4 * (size_t)e];
+                    const double k = q[2] / hm.d_vol[c], w = q[3];
+                    q[0] *= k;
+                    q[1] *= k;
+                    q[2] = w;
+                    q[3] = 0.0;
+                    const double* m3 = &hg.lsq_inv[3 * (size_t)c];
+                    const double x = hg.lsq_w[2 * (size_t)e], y = hg.lsq_w[2 * (size_t)e + 1];
+                    hg.lsq_w[2 * (size_t)e] = m3[0] * x + m3[1] * y;
+                    hg.lsq_w[2 * (size_t)e + 1] = m3[1] * x + m3[2] * y;
+                }
+            for (int f = 0; f < F; ++f) {
+                double* q = &hg.fgrad[8 * (size_t)f];
+                q[0] = 1.0 / (q[0] * q[1]);
+                q[1] = hm.d_fgeom[4 * (size_t)f + 2];
+            }
+        }
         NSArgs& a = ns;
+        a.fixed = !opt.strict && fixed_gamma();
+        a.fxc = flux_const();
+        a.inv_R = 1.0 / opt.gas_constant;
         a.g.n_cells = N;
         a.g.n_faces = F;
         a.g.scheme = opt.gradient;
@@ -367,6 +391,14 @@ void Solver::init(const HostMesh& hm, const fv_bc_t* bcs, int n_bcs, double g, d
         r.prandtl = opt.prandtl;
         r.prandtl_t = opt.prandtl_t;
         r.k_lam = r.cp * opt.mu / opt.prandtl;
+        r.inv_mu = 1.0 / opt.mu;
+        r.cv1_3 = opt.sa[6] * opt.sa[6] * opt.sa[6];
+        r.inv_kappa2 = 1.0 / (opt.sa[3] * opt.sa[3]);
+        r.cb2_sigma = opt.sa[1] / opt.sa[2];
+        r.cw1 = opt.sa[0] / (opt.sa[3] * opt.sa[3]) + (1.0 + opt.sa[1]) / opt.sa[2];
+        r.inv_1_cw3_6 = 1.0 / (1.0 + r.cw3_6);
+        r.half_inv_sigma = 0.5 / opt.sa[2];
+        r.cp_prt = r.cp / opt.prandtl_t;
         std::vector<double4_32a> seg;
         for (int f = 0; f < F; ++f) {
             if (hm.fr[f] >= 0 || bc.type[hm.fpatch[f]] != FV_BC_NOSLIP) continue;
