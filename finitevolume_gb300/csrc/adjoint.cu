@@ -144,6 +144,19 @@ __device__ __forceinline__ V4<double> ldW(const St* W, int i) {
     const St s = ld_state(W, i);
     return {s.r, s.ru, s.rv, s.E};
 }
+// Four doubles of a 32-byte-aligned row, one 256-bit access.
+__device__ __forceinline__ double4_32a ld4(const double* p) { return *reinterpret_cast<const double4_32a*>(p); }
+__device__ __forceinline__ void st4(double* p, double a, double b, double c, double d) {
+    double4_32a q;
+    q.x = a; q.y = b; q.z = c; q.w = d;
+    *reinterpret_cast<double4_32a*>(p) = q;
+}
+__device__ __forceinline__ void ld_grad(const double2* G, int c, double2 g[4]) {
+    const double* p = reinterpret_cast<const double*>(G + 4 * (size_t)c);
+    const double4_32a a = ld4(p), b = ld4(p + 4);
+    g[0] = make_double2(a.x, a.y); g[1] = make_double2(a.z, a.w);
+    g[2] = make_double2(b.x, b.y); g[3] = make_double2(b.z, b.w);
+}
 __device__ __forceinline__ double vget(const V4<double>& w, int k) { return (&w.r)[k]; }
 // Conserved freestream of boundary face f's farfield: the patch's, or (batched
 // solvers) the owner cell's instance's.
@@ -207,10 +220,180 @@ __device__ __forceinline__ unsigned char recon_face(const AdjArgs& a, int f, int
     return flags;
 }
 
+// Flux (F), times the length, and its Jacobians with respect to both
+// primitive states, in closed form: hllc_p / rusanov_p differentiated, branch
+// by branch as the dual numbers of the boundary faces take them.  The other
+// side of an HLLC star state enters only through S* and S_K, so each Jacobian
+// is a 4 x 4 part of its own side plus two outer products.
+struct FluxLin {
+    double F[4], J[2][16];
+};
+// (r, Vn, p, E) partials of one side's flux vector with its own normal velocity
+__device__ __forceinline__ void add_side(double J[16], const double gr[4], const double gn[4], const double gp[4],
+                                         double M, double gE, const V4<double>& w, double nx, double ny, double igm1) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        J[4 * i] += gr[i];
+        J[4 * i + 1] += gn[i] * nx;
+        J[4 * i + 2] += gn[i] * ny;
+        J[4 * i + 3] += gp[i];
+    }
+    J[5] += M;
+    J[10] += M;
+    J[12] += gE * (0.5 * (w.u * w.u + w.v * w.v));
+    J[13] += gE * (w.r * w.u);
+    J[14] += gE * (w.r * w.v);
+    J[15] += gE * igm1;
+}
+__device__ __forceinline__ void add_outer(double J[16], const double g[4], const double d[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) J[4 * i + k] += g[i] * d[k];
+}
+// the physical flux (times s) of one side and its Jacobian
+__device__ __forceinline__ void lin_phys(double s, const V4<double>& w, double Vn, double E, double nx, double ny,
+                                         double igm1, double F[4], double J[16]) {
+    const double rV = s * (w.r * Vn), sV = s * Vn;
+    F[0] += rV;
+    F[1] += rV * w.u + s * (w.p * nx);
+    F[2] += rV * w.v + s * (w.p * ny);
+    F[3] += sV * (E + w.p);
+    const double gr[4] = {sV, sV * w.u, sV * w.v, 0.0};
+    const double gn[4] = {s * w.r, s * (w.r * w.u), s * (w.r * w.v), s * (E + w.p)};
+    const double gp[4] = {0.0, s * nx, s * ny, sV};
+    add_side(J, gr, gn, gp, rV, sV, w, nx, ny, igm1);
+}
+__device__ void lin_flux(int flux, const V4<double>& L, const V4<double>& R, double nx, double ny, double ar, double g,
+                         double igm1, FluxLin& o) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o.F[i] = 0.0;
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+#pragma unroll
+        for (int i = 0; i < 16; ++i) o.J[s][i] = 0.0;
+    const double VL = L.u * nx + L.v * ny, VR = R.u * nx + R.v * ny;
+    const double EL = L.p * igm1 + 0.5 * L.r * (L.u * L.u + L.v * L.v);
+    const double ER = R.p * igm1 + 0.5 * R.r * (R.u * R.u + R.v * R.v);
+    const double gpL = g * L.p, gpR = g * R.p;
+    const double cL = gpL * rsqrt(gpL * L.r), cR = gpR * rsqrt(gpR * R.r);
+    // dc = -c/(2r) dr + c/(2p) dp
+    const double crL = 0.5 * cL / L.r, cpL = 0.5 * cL / L.p, crR = 0.5 * cR / R.r, cpR = 0.5 * cR / R.p;
+    if (flux != FLUX_HLLC) {
+        const double sl = fabs(VL) + cL, sr = fabs(VR) + cR;
+        const bool right = sr > sl;
+        const double h = 0.5 * ar, S = right ? sr : sl;
+        lin_phys(h, L, VL, EL, nx, ny, igm1, o.F, o.J[0]);
+        lin_phys(h, R, VR, ER, nx, ny, igm1, o.F, o.J[1]);
+        const double d[4] = {R.r - L.r, R.r * R.u - L.r * L.u, R.r * R.v - L.r * L.v, ER - EL};
+        const double hs = h * S;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o.F[i] -= hs * d[i];
+        // -h S dU(R) + h S dU(L)
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            const V4<double>& w = s ? R : L;
+            const double k = s ? -hs : hs;
+            double* J = o.J[s];
+            J[0] += k;
+            J[4] += k * w.u; J[5] += k * w.r;
+            J[8] += k * w.v; J[10] += k * w.r;
+            J[12] += k * (0.5 * (w.u * w.u + w.v * w.v)); J[13] += k * (w.r * w.u); J[14] += k * (w.r * w.v);
+            J[15] += k * igm1;
+        }
+        const double V = right ? VR : VL, sg = V < 0.0 ? -1.0 : 1.0;
+        const double ds[4] = {right ? -crR : -crL, sg * nx, sg * ny, right ? cpR : cpL};
+        const double gs[4] = {-h * d[0], -h * d[1], -h * d[2], -h * d[3]};
+        if (right) add_outer(o.J[1], gs, ds);
+        else add_outer(o.J[0], gs, ds);
+        return;
+    }
+    const bool minR = VR - cR < VL - cL, maxR = VR + cR > VL + cL;  // which side sets S_L, S_R
+    const double SL = minR ? VR - cR : VL - cL, SR = maxR ? VR + cR : VL + cL;
+    if (SL >= 0.0) {
+        lin_phys(ar, L, VL, EL, nx, ny, igm1, o.F, o.J[0]);
+        return;
+    }
+    if (SR <= 0.0) {
+        lin_phys(ar, R, VR, ER, nx, ny, igm1, o.F, o.J[1]);
+        return;
+    }
+    const double mL = L.r * (SL - VL), mR = R.r * (SR - VR);
+    const double num = R.p - L.p + mL * VL - mR * VR, den = mL - mR;
+    const bool left = num <= 0.0;
+    const double SK = left ? SL : SR, V = left ? VL : VR, m = left ? mL : mR, E = left ? EL : ER;
+    const V4<double> K = left ? L : R;
+    const double t = SK * den - num, rr = 1.0 / (den * t);
+    const double Ss = num * (t * rr), q = den * (den * rr), id = t * rr;  // id = 1 / den
+    const double d = SK - V, w = Ss - V, ps = K.p + m * w, fac = m * q, M = fac * Ss, T = ps + M * w;
+    const double A = d * E - K.p * V + ps * Ss, Es = q * A;
+    o.F[0] = ar * M;
+    o.F[1] = ar * (M * K.u + T * nx);
+    o.F[2] = ar * (M * K.v + T * ny);
+    o.F[3] = ar * (Ss * (Es + ps));
+    // partials of (M, T, F_E) with respect to r, Vn, p, S_K and S*, as flux vectors
+    auto vec = [&](double dM, double dT, double dE, double out[4]) {
+        out[0] = ar * dM;
+        out[1] = ar * (dM * K.u + dT * nx);
+        out[2] = ar * (dM * K.v + dT * ny);
+        out[3] = ar * dE;
+    };
+    double gr[4], gn[4], gp[4], gK[4], gS[4];
+    {
+        const double dps = w * d, dM = Ss * q * d;
+        vec(dM, dps + w * dM, Ss * (q * (Ss * dps) + dps), gr);
+    }
+    {
+        const double dps = -w * K.r - m, dM = -Ss * q * K.r;
+        vec(dM, dps + w * dM - M, Ss * (q * (Ss * dps - E - K.p) + dps), gn);
+    }
+    vec(0.0, 1.0, Ss * (q * (Ss - V) + 1.0), gp);
+    {
+        const double dps = w * K.r, dM = Ss * (q * K.r - fac * q);
+        vec(dM, dps + w * dM, Ss * (q * (E + Ss * dps) - Es * q + dps), gK);
+    }
+    {
+        const double dM = Ss * (fac * q) + fac;
+        vec(dM, m + w * dM + M, (Es + ps) + Ss * (q * (Ss * m + ps) + Es * q + m), gS);
+    }
+    double JK[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) JK[i] = 0.0;
+    add_side(JK, gr, gn, gp, ar * M, ar * (Ss * q * d), K, nx, ny, igm1);
+    // dS* on both sides: directly, and through S_L and S_R
+    const double wL = VL - Ss, wR = VR - Ss;
+    const double nL = (mL - wL * L.r) * id, nR = (wR * R.r - mR) * id;
+    double sL[4] = {wL * (SL - VL) * id, nL * nx, nL * ny, -id}, sR[4] = {-wR * (SR - VR) * id, nR * nx, nR * ny, id};
+    const double aL = wL * L.r * id, aR = -wR * R.r * id;
+    const double dSL[4] = {minR ? crR : crL, nx, ny, minR ? -cpR : -cpL};
+    const double dSR[4] = {maxR ? -crR : -crL, nx, ny, maxR ? cpR : cpL};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const double x = aL * dSL[k], y = aR * dSR[k];
+        sL[k] += (minR ? 0.0 : x) + (maxR ? 0.0 : y);
+        sR[k] += (minR ? x : 0.0) + (maxR ? y : 0.0);
+    }
+    add_outer(o.J[0], gS, sL);
+    add_outer(o.J[1], gS, sR);
+    const bool onR = left ? minR : maxR;  // the side that sets S_K
+    double dK[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) dK[k] = left ? dSL[k] : dSR[k];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const double x = gK[i] * dK[k];
+            o.J[0][4 * i + k] += (onR ? 0.0 : x) + (left ? JK[4 * i + k] : 0.0);
+            o.J[1][4 * i + k] += (onR ? x : 0.0) + (left ? 0.0 : JK[4 * i + k]);
+        }
+}
+
 // Per face: reconstruction (with its positivity decisions), flux value and
 // the flux Jacobians.
 __global__ void k_lin_face(const AdjArgs a) {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    // from the last face down: the boundary faces' long dual-number chains start first
+    const int f = (gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x;
     if (f >= a.n_faces) return;
     const int L = a.fl[f], R = a.fr[f];
     const double4_32a geo = a.fgeom[f];
@@ -225,10 +408,17 @@ __global__ void k_lin_face(const AdjArgs a) {
     double* JR = a.JR + 16 * (size_t)f;
     V4<D4> F1;
     if (R >= 0) {
-        F1 = flux_of<D4>(a.flux, seed(wl), cst(wr), nxD, nyD, gD, iD);
-        store_jac(JL, F1, ar);
-        const V4<D4> F2 = flux_of<D4>(a.flux, cst(wl), seed(wr), nxD, nyD, gD, iD);
-        store_jac(JR, F2, ar);
+        // closed form: about 330 FP64 instructions (two passes of dual numbers
+        // took 1,600 and 789 us at 250k faces)
+        FluxLin o;
+        lin_flux(a.flux, wl, wr, nx, ny, ar, g, a.igm1, o);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            st4(JL + 4 * i, o.J[0][4 * i], o.J[0][4 * i + 1], o.J[0][4 * i + 2], o.J[0][4 * i + 3]);
+            st4(JR + 4 * i, o.J[1][4 * i], o.J[1][4 * i + 1], o.J[1][4 * i + 2], o.J[1][4 * i + 3]);
+        }
+        st_state(a.F, f, st_make(o.F[0], o.F[1], o.F[2], o.F[3]));
+        return;
     } else {
         const int patch = a.fpatch[f];
         const int t = a.bc.type[patch];
@@ -518,6 +708,9 @@ __global__ void k_fwd_cell3(const AdjArgs a, St* __restrict__ dR) {
 
 // ---------------------------------------------------------------------------
 // Cotangent map: Ubar = (dR/dU)^T lam, fsbar = (dR/dfs)^T lam.
+// Bound: the flux Jacobians (256 B a face) where they do not fit in L2, else
+// FP64 issue; they are read a row of four per 256-bit load (as scalars, 32
+// lanes each on a line of its own, the pass took 43 us at 250k faces).
 __global__ void k_bwd_face(const AdjArgs a, const St* __restrict__ lam) {
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= a.n_faces) return;
@@ -531,16 +724,16 @@ __global__ void k_bwd_face(const AdjArgs a, const St* __restrict__ lam) {
     }
     const double* JL = a.JL + 16 * (size_t)f;
     const double* JR = a.JR + 16 * (size_t)f;
-    double* wb = a.wbar + 8 * (size_t)f;
+    double tl[4] = {0.0, 0.0, 0.0, 0.0}, tr[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        double tl = 0.0, tr = 0.0;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) { tl += JL[4 * i + k] * fbar[i]; tr += JR[4 * i + k] * fbar[i]; }
-        wb[k] = tl;
-        if (R >= 0) wb[4 + k] = tr;
-        else a.fsb[4 * (size_t)(f - a.n_int_faces) + k] = tr;
+    for (int i = 0; i < 4; ++i) {
+        const double4_32a l = ld4(JL + 4 * i), q = ld4(JR + 4 * i);
+        tl[0] += l.x * fbar[i]; tl[1] += l.y * fbar[i]; tl[2] += l.z * fbar[i]; tl[3] += l.w * fbar[i];
+        tr[0] += q.x * fbar[i]; tr[1] += q.y * fbar[i]; tr[2] += q.z * fbar[i]; tr[3] += q.w * fbar[i];
     }
+    double* wb = a.wbar + 8 * (size_t)f;
+    st4(wb, tl[0], tl[1], tl[2], tl[3]);
+    st4(R >= 0 ? wb + 4 : a.fsb + 4 * (size_t)(f - a.n_int_faces), tr[0], tr[1], tr[2], tr[3]);
 }
 
 // Gather of the face-state cotangents: W-bar and the gradient cotangent.
@@ -548,11 +741,11 @@ __global__ void k_bwd_face(const AdjArgs a, const St* __restrict__ lam) {
 __device__ __forceinline__ void finish_cell(const AdjArgs& a, int c, const double wbar[4], int mode,
                                             St* __restrict__ out, St* __restrict__ lam, St* __restrict__ lam0,
                                             const St* __restrict__ rhs, double* __restrict__ r2) {
-    double J[16];
-    prim_jac(ldW(a.W, c), a.gamma, J);
-    double u[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) u[k] = J[k] * wbar[0] + J[4 + k] * wbar[1] + J[8 + k] * wbar[2] + J[12 + k] * wbar[3];
+    // (dW/dU)^T wbar (prim_jac), with one reciprocal
+    const V4<double> w = ldW(a.W, c);
+    const double ir = fvconv::rcp_nr3(w.r), m1 = wbar[1] * ir, m2 = wbar[2] * ir, g3 = (a.gamma - 1.0) * wbar[3];
+    const double u[4] = {wbar[0] - (w.u * m1 + w.v * m2) + (0.5 * g3) * (w.u * w.u + w.v * w.v), m1 - w.u * g3,
+                         m2 - w.v * g3, g3};
     if (mode == 0) {
         st_state(out, c, st_make(u[0], u[1], u[2], u[3]));
         return;
@@ -602,7 +795,8 @@ __global__ void __launch_bounds__(256) k_bwd_cell1(const AdjArgs a, int mode, St
             const int ent = a.cf[e];
             const int f = ent >> 1;
             const bool owner = ent & 1;
-            const double* w = a.wbar + 8 * (size_t)f + (owner ? 0 : 4);
+            const double4_32a wq = ld4(a.wbar + 8 * (size_t)f + (owner ? 0 : 4));
+            const double w[4] = {wq.x, wq.y, wq.z, wq.w};
 #pragma unroll
             for (int k = 0; k < 4; ++k) wb[k] += w[k];
             if (a.order == 2 && !(a.fb[f] & (owner ? 1 : 2))) {
@@ -614,11 +808,12 @@ __global__ void __launch_bounds__(256) k_bwd_cell1(const AdjArgs a, int mode, St
         }
         if (a.order == 2) {
             double gux[4], guy[4];
+            const double4_32a pq = ld4(a.psi + 4 * (size_t)c);
+            const double pv[4] = {pq.x, pq.y, pq.z, pq.w};
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const double p = a.psi[4 * c + k];
-                gux[k] = p * gx[k];
-                guy[k] = p * gy[k];
+                gux[k] = pv[k] * gx[k];
+                guy[k] = pv[k] * gy[k];
             }
             if (a.full) {
                 // psi-bar = Gbar . Gu; then through psi = phi(d1, y):
@@ -655,8 +850,9 @@ __global__ void __launch_bounds__(256) k_bwd_cell1(const AdjArgs a, int mode, St
             }
             St q = st_make(wb[0], wb[1], wb[2], wb[3]);
             st_state(a.Wbar, c, q);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) a.Gub[4 * c + k] = make_double2(gux[k], guy[k]);
+            double* gub = reinterpret_cast<double*>(a.Gub + 4 * (size_t)c);
+            st4(gub, gux[0], guy[0], gux[1], guy[1]);
+            st4(gub + 4, gux[2], guy[2], gux[3], guy[3]);
         } else {
             finish_cell(a, c, wb, mode, out, lam, lam0, rhs, r2);
         }
@@ -673,8 +869,7 @@ __global__ void __launch_bounds__(256) k_bwd_cell2(const AdjArgs a, int mode, St
         const St w0 = ld_state(a.Wbar, c);
         double wb[4] = {w0.r, w0.ru, w0.rv, w0.E};
         double2 gc[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) gc[k] = a.Gub[4 * c + k];
+        ld_grad(a.Gub, c, gc);
         const double2 s = a.lsq_sum[c];
 #pragma unroll
         for (int k = 0; k < 4; ++k) wb[k] -= s.x * gc[k].x + s.y * gc[k].y;
@@ -683,10 +878,11 @@ __global__ void __launch_bounds__(256) k_bwd_cell2(const AdjArgs a, int mode, St
             if (nb >= 0) {
                 const int tw = a.twin[e];
                 const double2 w = a.lsq[tw];
+                double2 gn[4];
+                ld_grad(a.Gub, nb, gn);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    const double2 q = a.Gub[4 * nb + k];
-                    wb[k] += w.x * q.x + w.y * q.y;
+                    wb[k] += w.x * gn[k].x + w.y * gn[k].y;
                     if (a.full && a.led[4 * nb + k] == tw) wb[k] += a.ldb[4 * nb + k];
                 }
             } else {
@@ -1086,7 +1282,7 @@ void linearise(fv_adjoint_s* A) {
         fvgb::o2::launch_prim_f64(o, s.stream);
         check_launch();
     }
-    adjk::k_lin_face<<<blocks(A->F), kB, 0, s.stream>>>(a);
+    adjk::k_lin_face<<<(A->F + 127) / 128, 128, 0, s.stream>>>(a);
     check_launch();
     if (a.full) {
         adjk::k_lin_lim<<<blocks(A->N), kB, 0, s.stream>>>(a);
@@ -1100,7 +1296,6 @@ void linearise(fv_adjoint_s* A) {
 void backward(fv_adjoint_s* A, const St* lam, int mode, St* out) {
     fvgb::Solver& s = A->solver->s;
     AdjArgs& a = A->a;
-    if (A->Fb) FV_CUDA(cudaMemsetAsync(a.fsb, 0, sizeof(double) * 4 * (size_t)A->Fb, s.stream));
     adjk::k_bwd_face<<<blocks(A->F), kB, 0, s.stream>>>(a, lam);
     check_launch();
     adjk::k_bwd_cell1<<<blocks(A->N), kB, 0, s.stream>>>(a, mode, out, A->lam, A->lam0, A->rhs, A->partials);
