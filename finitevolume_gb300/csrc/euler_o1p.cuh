@@ -243,23 +243,14 @@ __device__ __forceinline__ void ghost_p(const BCTable& bc, int patch, const St& 
 }
 #endif
 
-// One face of the face phase: the flux times the face length into ff[f]
-// and, with local dt, lambda * length into dtf[f].  Returns the face's
-// global-dt candidate cfl * (CFL length) / max(|Vn| + c) (DBL_MAX with
-// local dt).
+// One face of the face phase: its flux times the face length and, in dt, with
+// local dt lambda * length, else the face's global-dt candidate cfl * (CFL
+// length) / max(|Vn| + c).  UR, PR: the right cell of an internal face (a
+// boundary face's ghost is formed here).
 template <int FLUX, bool LOCAL>
-__device__ __forceinline__ double face_phase_face(const O1Args& a, const double4_32a* P, int f, double g,
-                                                  double cfl) {
-    const int L = a.m.fl[f], R = a.m.fr[f];
-    const double4_32a geo = a.m.fgeom[f];
-    const St UL = ld_state_cg(a.U, L);
-    const Prim PL = ld_prim(P, L);
-    St UR;
-    Prim PR;
-    if (R >= 0) {
-        UR = ld_state_cg(a.U, R);
-        PR = ld_prim(P, R);
-    } else {
+__device__ __forceinline__ St face_compute(const O1Args& a, int f, bool interior, const double4_32a& geo, const St& UL,
+                                           const Prim& PL, St UR, Prim PR, double g, double cfl, double& dt) {
+    if (!interior) {
 #ifndef FV_STRICT_ORDER
         ghost_p(a.bc, a.m.fpatch[f], UL, PL, geo.x, geo.y, g, UR, PR);
 #else
@@ -273,41 +264,49 @@ __device__ __forceinline__ double face_phase_face(const O1Args& a, const double4
         const fvfix::State L4 = {UL.r, PL.u, PL.v, PL.p}, R4 = {UR.r, PR.u, PR.v, PR.p};
         fvfix::State F;
         double lam;
-        if (fvfix::flux<FLUX == FLUX_HLLC ? 1 : 0, true, true>(L4, R4, PL.c, PR.c, geo.x, geo.y, geo.z, a.fxc, F,
-                                                               R >= 0, lam)) {
-            st_state(a.ff, f, st_make(F.r, F.u, F.v, F.p));
-            if (LOCAL) {
-                a.dtf[f] = lam * geo.z;
-                return DBL_MAX;
-            }
-            return cfl * geo.w * fvconv::rcp_nr3(lam);
+        if (fvfix::flux<FLUX == FLUX_HLLC ? 1 : 0, true, true>(L4, R4, PL.c, PR.c, UL, UR, geo.x, geo.y, geo.z, a.fxc,
+                                                               F, interior, lam)) {
+            dt = LOCAL ? lam * geo.z : cfl * geo.w * fvconv::rcp_nr3(lam);
+            return st_make(F.r, F.u, F.v, F.p);
         }
     }
 #endif
     const St Fl = num_flux_p<FLUX>(UL, PL, UR, PR, geo.x, geo.y, g, a.exact_tol, a.exact_max_iter);
-    st_state(a.ff, f, geo.z * Fl);
-    const double Smax = face_smax_p(PL, PR, R >= 0, geo.x, geo.y);
-    if (LOCAL) {
-        a.dtf[f] = Smax * geo.z;
-        return DBL_MAX;
-    }
-    return cfl * geo.w / Smax;
+    const double Smax = face_smax_p(PL, PR, interior, geo.x, geo.y);
+    dt = LOCAL ? Smax * geo.z : cfl * geo.w / Smax;
+    return geo.z * Fl;
+}
+
+// The same with the states read from and the results left in global memory;
+// returns the global-dt candidate (DBL_MAX with local dt).
+template <int FLUX, bool LOCAL>
+__device__ __forceinline__ double face_phase_face(const O1Args& a, const double4_32a* P, int f, double g,
+                                                  double cfl) {
+    const int L = a.m.fl[f], R = a.m.fr[f];
+    const St UL = ld_state_cg(a.U, L);
+    const Prim PL = ld_prim(P, L);
+    const int Rs = R >= 0 ? R : L;
+    double dt;
+    st_state(a.ff, f, face_compute<FLUX, LOCAL>(a, f, R >= 0, a.m.fgeom[f], UL, PL, ld_state_cg(a.U, Rs),
+                                                ld_prim(P, Rs), g, cfl, dt));
+    if (!LOCAL) return dt;
+    a.dtf[f] = dt;
+    return DBL_MAX;
 }
 
 #ifndef FV_STRICT_ORDER
 // The signed sum of a cell's N face fluxes and, with LOCAL, the sum of its
 // faces' lambda * length, on the integer pipe (fvfix::signed_sum).
-template <int N, bool LOCAL>
-__device__ __forceinline__ St gather_cell(const O1Args& a, int e0, double& lam) {
+// face(i, lam): the flux and lambda * length of the cell's i-th face.
+template <int N, bool LOCAL, class Face>
+__device__ __forceinline__ St gather_cell(const int* cf, const Face& face, double& lam) {
     double x[4][N], l[N];
     int neg[N], none[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) {
-        const int ent = a.m.cf[e0 + i];
-        const St F = ld_state_cg(a.ff, ent >> 1);
+        const St F = face(i, l[i]);
         x[0][i] = F.r; x[1][i] = F.ru; x[2][i] = F.rv; x[3][i] = F.E;
-        if (LOCAL) l[i] = __ldcg(a.dtf + (ent >> 1));
-        neg[i] = ent;
+        neg[i] = cf[i];
         none[i] = 0;
     }
     if (LOCAL) lam = fvfix::signed_sum<N>(l, none);
@@ -316,26 +315,26 @@ __device__ __forceinline__ St gather_cell(const O1Args& a, int e0, double& lam) 
 }
 #endif
 
-// One cell of the cell phase: the signed gather of its face fluxes,
-// U += dt/V R, the new primitives, and the squares of R for the norms.
-template <bool LOCAL>
-__device__ __forceinline__ void cell_phase_cell(const O1Args& a, double4_32a* P, int c, double g, double cfl,
-                                                double dt_g, double& s0, double& s1, double& s2, double& s3) {
+// One cell of the cell phase: the signed gather of its face fluxes, U + dt/V R
+// (returned) from its state u, the new primitives q, and the squares of R for
+// the norms.
+template <bool LOCAL, class Face>
+__device__ __forceinline__ St cell_compute(const O1Args& a, int c, const Face& face, const St& u, double g, double cfl,
+                                           double dt_g, Prim& q, double& s0, double& s1, double& s2, double& s3) {
     double dt = dt_g;
     St Rs = st_make(0.0, 0.0, 0.0, 0.0);
-    const int e0 = a.m.cf_off[c], e1 = a.m.cf_off[c + 1];
+    const int e0 = a.m.cf_off[c], n = a.m.cf_off[c + 1] - e0;
+    const int* cf = a.m.cf + e0;
     double lam = 0.0;
 #ifndef FV_STRICT_ORDER
-    const int n = e1 - e0;
-    if (n == 4) Rs = gather_cell<4, LOCAL>(a, e0, lam);
-    else if (n == 3) Rs = gather_cell<3, LOCAL>(a, e0, lam);
+    if (n == 4) Rs = gather_cell<4, LOCAL>(cf, face, lam);
+    else if (n == 3) Rs = gather_cell<3, LOCAL>(cf, face, lam);
     else
 #endif
-    for (int e = e0; e < e1; ++e) {
-        const int ent = a.m.cf[e];
-        const int f = ent >> 1;
-        Rs += flip_if(ld_state_cg(a.ff, f), ent);
-        if (LOCAL) lam += __ldcg(a.dtf + f);
+    for (int i = 0; i < n; ++i) {
+        double l;
+        Rs += flip_if(face(i, l), cf[i]);
+        if (LOCAL) lam += l;
     }
     double coef;  // dt / V
 #ifdef FV_STRICT_ORDER
@@ -345,10 +344,26 @@ __device__ __forceinline__ void cell_phase_cell(const O1Args& a, double4_32a* P,
     coef = LOCAL ? cfl * fvconv::rcp_nr3(lam) : dt * fvconv::rcp_nr3(a.m.vol[c]);
 #endif
     s0 = Rs.r * Rs.r; s1 = Rs.ru * Rs.ru; s2 = Rs.rv * Rs.rv; s3 = Rs.E * Rs.E;
-    const St u = ld_state_cg(a.U, c);
     const St un = u + coef * Rs;
+    q = prim_of(un, g);
+    return un;
+}
+
+template <bool LOCAL>
+__device__ __forceinline__ void cell_phase_cell(const O1Args& a, double4_32a* P, int c, double g, double cfl,
+                                                double dt_g, double& s0, double& s1, double& s2, double& s3) {
+    const int* cf = a.m.cf + a.m.cf_off[c];
+    Prim q;
+    const St un = cell_compute<LOCAL>(
+        a, c,
+        [&](int i, double& l) {
+            const int f = cf[i] >> 1;
+            if (LOCAL) l = __ldcg(a.dtf + f);
+            return ld_state_cg(a.ff, f);
+        },
+        ld_state_cg(a.U, c), g, cfl, dt_g, q, s0, s1, s2, s3);
     st_state(a.U, c, un);
-    st_prim(P, c, prim_of(un, g));
+    st_prim(P, c, q);
 }
 
 // Grid barrier with a bounded wait.  Returns false (in every thread of the
@@ -665,6 +680,213 @@ __global__ void __launch_bounds__(fvgb::kDfBlock, 1) k_o1_dataflow(const O1Args 
     if (b == 0 && threadIdx.x == 0) a.ctl->step = step0 + nsteps;
 }
 
+// The same with the block's own cells and the fluxes of all their faces in
+// shared memory, for blocks that fit (DfPlan::smem).  A face between two
+// blocks is computed by both, from the same states by the same operations, so
+// cells' states are all that blocks exchange, once a step, and a step has two
+// block barriers and no other wait than the outer faces' for their states.
+//
+// Exchange: a cell that another block reads has a mailbox of two slots
+// (DfPlan::mail; the state of step s in slot s & 1), eight 16-byte words each
+// of one value and the tag s + 1, written and read as single 128-bit relaxed
+// accesses.  A reader polls the words themselves, so no fence, flag or second
+// round trip is needed.  A slot is free when it is written again: the state of
+// step s + 2 follows the reading of the neighbour's state s + 1 across the
+// same face, which followed the neighbour's reading of state s.
+//
+// Bound: the dependent chain of one step (mailbox round trip, a face's flux, a
+// cell's update) below about 20k cells, FP64 issue above.  32k cells,
+// Rusanov: see the launch rule.
+__device__ __forceinline__ void mail_store(double2* w, double v, unsigned long long tag) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    asm volatile("{.reg .b128 q; mov.b128 q, {%1, %2}; st.relaxed.gpu.global.b128 [%0], q;}" ::"l"(w), "l"(b), "l"(tag)
+                 : "memory");
+}
+__device__ __forceinline__ double mail_load(const double2* w, unsigned long long& tag) {
+    unsigned long long b;
+    asm volatile("{.reg .b128 q; ld.relaxed.gpu.global.b128 q, [%2]; mov.b128 {%0, %1}, q;}"
+                 : "=l"(b), "=l"(tag)
+                 : "l"(w)
+                 : "memory");
+    return __longlong_as_double((long long)b);
+}
+// One slot: conserved state and primitives.
+__device__ __forceinline__ void mail_put(double2* w, const St& u, const Prim& q, unsigned long long tag) {
+    mail_store(w, u.r, tag);
+    mail_store(w + 1, u.ru, tag);
+    mail_store(w + 2, u.rv, tag);
+    mail_store(w + 3, u.E, tag);
+    mail_store(w + 4, q.u, tag);
+    mail_store(w + 5, q.v, tag);
+    mail_store(w + 6, q.p, tag);
+    mail_store(w + 7, q.c, tag);
+}
+// Waits for the slot's tag, bounded by pc->limit cycles like the grid barrier
+// (false, with pc->err set, when it runs out or another block has given up).
+__device__ __forceinline__ bool mail_get(PersistCtl* pc, const double2* w, unsigned long long tag, St& u, Prim& q) {
+    const volatile int* verr = &pc->err;
+    const long long t0 = clock64(), lim = pc->limit;
+    for (unsigned int it = 0;; ++it) {
+        unsigned long long t[8];
+        u.r = mail_load(w, t[0]);
+        u.ru = mail_load(w + 1, t[1]);
+        u.rv = mail_load(w + 2, t[2]);
+        u.E = mail_load(w + 3, t[3]);
+        q.u = mail_load(w + 4, t[4]);
+        q.v = mail_load(w + 5, t[5]);
+        q.p = mail_load(w + 6, t[6]);
+        q.c = mail_load(w + 7, t[7]);
+        unsigned long long d = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) d |= t[i] ^ tag;
+        if (d == 0) return true;
+        if ((it & 15u) == 15u && (*verr || clock64() - t0 > lim)) {
+            atomicExch(&pc->err, 1);
+            return false;
+        }
+    }
+}
+
+__device__ __forceinline__ St ld_shared(const double2* s, int i) {
+    const double2 x = s[2 * i], y = s[2 * i + 1];
+    return st_make(x.x, x.y, y.x, y.y);
+}
+__device__ __forceinline__ void st_shared(double2* s, int i, double a, double b, double c, double d) {
+    s[2 * i] = make_double2(a, b);
+    s[2 * i + 1] = make_double2(c, d);
+}
+
+template <int FLUX>
+__global__ void __launch_bounds__(fvgb::kDfBlock, 1) k_o1_dataflow_sm(const O1Args a, PersistCtl* __restrict__ pc,
+                                                                     const DfPlan d, int nsteps) {
+    extern __shared__ double2 sm[];
+    const double g = a.gamma;
+    const int b = blockIdx.x, nb = gridDim.x;
+    const unsigned int expected = (unsigned int)nb + (unsigned int)pc->phantom;
+    const int c0 = d.cell_off[b], nc = d.cell_off[b + 1] - c0;
+    const int f0 = d.xface_off[b], nf = d.xface_off[b + 1] - f0;
+    const int nf_in = d.face_in[b];    // faces that need no other block's cell, first
+    double2* sU = sm;                  // own states
+    double2* sP = sU + 2 * nc;         // their primitives
+    double2* sN = sP + 2 * nc;         // squared residuals
+    double2* sF = sN + 2 * nc;         // fluxes of the own cells' faces
+    double* sL = reinterpret_cast<double*>(sF + 2 * nf);  // their lambda * length
+    const int step0 = a.ctl->step;
+    const double cfl = a.ctl->cfl;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int nwarps = fvgb::kDfBlock / 32;
+
+    // prologue: own states and primitives; the mailboxes' first slots hold
+    // them as step 0, their second slots nothing of this launch
+    for (int i = threadIdx.x; i < nc; i += blockDim.x) {
+        const St u = ld_state_cg(a.U, c0 + i);
+        const Prim q = prim_of(u, g);
+        st_shared(sU, i, u.r, u.ru, u.rv, u.E);
+        st_shared(sP, i, q.u, q.v, q.p, q.c);
+        const int m = d.mail_of[c0 + i];
+        if (m >= 0) {
+            mail_put(d.mail + 16 * (size_t)m, u, q, 1ull);
+            mail_put(d.mail + 16 * (size_t)m + 8, u, q, 0ull);
+        }
+    }
+    __shared__ int failed;
+    if (threadIdx.x == 0) failed = 0;
+    if (!grid_barrier(pc, expected)) return;
+
+    // padded positions: the outer faces start at a warp boundary
+    const int fpad = (nf_in + 31) & ~31, fend = fpad + nf - nf_in;
+    for (int s = 0; s < nsteps; ++s) {
+        for (int j = threadIdx.x; j < fend; j += fvgb::kDfBlock) {
+            const bool outer = j >= fpad;
+            if (!outer && j >= nf_in) continue;
+            const int k = outer ? j - fpad + nf_in : j;  // slot of the face
+            const int f = d.xfaces[f0 + k];
+            // cells: own (>= 0), another block's (-1 - mailbox), none (boundary)
+            const int2 lr = d.xcells[f0 + k];
+            St UL, UR;
+            Prim PL, PR;
+            auto own = [&](int i, St& u, Prim& q) {
+                u = ld_shared(sU, i);
+                const St p = ld_shared(sP, i);
+                q.u = p.r; q.v = p.ru; q.p = p.rv; q.c = p.E;
+            };
+            bool interior = true;
+            if (outer) {
+                const bool left = lr.x < 0;  // the left cell is the other block's
+                St u;
+                Prim q;
+                if (!mail_get(pc, d.mail + 16 * (size_t)(-1 - (left ? lr.x : lr.y)) + 8 * (s & 1), s + 1ull, u, q)) {
+                    failed = 1;
+                    continue;
+                }
+                own(left ? lr.y : lr.x, UL, PL);
+                UR = u;
+                PR = q;
+                if (left) {
+                    UR = UL; PR = PL;
+                    UL = u; PL = q;
+                }
+            } else {
+                own(lr.x, UL, PL);
+                interior = lr.y >= 0;
+                own(interior ? lr.y : lr.x, UR, PR);
+            }
+            double lam;
+            const St F = face_compute<FLUX, true>(a, f, interior, a.m.fgeom[f], UL, PL, UR, PR, g, cfl, lam);
+            st_shared(sF, k, F.r, F.ru, F.rv, F.E);
+            sL[k] = lam;
+        }
+        __syncthreads();
+        if (failed) return;
+
+        const bool last = s == nsteps - 1;
+        for (int i = threadIdx.x; i < nc; i += fvgb::kDfBlock) {
+            const int c = c0 + i, e0 = a.m.cf_off[c];
+            Prim q;
+            double s0, s1, s2, s3;
+            const St un = cell_compute<true>(
+                a, c,
+                [&](int m, double& l) {
+                    const int k = d.slot[e0 + m];
+                    l = sL[k];
+                    return ld_shared(sF, k);
+                },
+                ld_shared(sU, i), g, cfl, 0.0, q, s0, s1, s2, s3);
+            const int m = d.mail_of[c];
+            if (last) st_state(a.U, c, un);
+            else if (m >= 0) mail_put(d.mail + 16 * (size_t)m + 8 * ((s + 1) & 1), un, q, s + 2ull);
+            st_shared(sU, i, un.r, un.ru, un.rv, un.E);
+            st_shared(sP, i, q.u, q.v, q.p, q.c);
+            st_shared(sN, i, s0, s1, s2, s3);
+        }
+        __syncthreads();
+
+        // the step's norm partials, one per 32-cell warp in cell order, by the
+        // last warps (the first ones have the next step's faces with the
+        // longest chains)
+        double* wp = d.wpart + (size_t)s * d.n_warps * 4;
+        for (int cw = nwarps - 1 - warp; cw * 32 < nc; cw += nwarps) {
+            St n = st_make(0.0, 0.0, 0.0, 0.0);
+            if (cw * 32 + lane < nc) n = ld_shared(sN, cw * 32 + lane);
+            const double ws = warp_sum4(n.r, n.ru, n.rv, n.E);
+            if ((lane & 7) == 0) wp[(size_t)(c0 / 32 + cw) * 4 + (lane >> 3)] = ws;
+        }
+    }
+    if (!grid_barrier(pc, expected)) return;
+    for (int s = b; s < nsteps; s += nb) df_fold(a, d, s, (step0 + s) % a.hist_cap, s == nsteps - 1);
+    if (b == 0 && threadIdx.x == 0) a.ctl->step = step0 + nsteps;
+}
+
+template <int FLUX>
+static int o1df_sm_blocks_per_sm(size_t smem) {
+    int nb = 0;
+    if (cudaFuncSetAttribute(k_o1_dataflow_sm<FLUX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)fvgb::kDfMaxSmem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_o1_dataflow_sm<FLUX>, fvgb::kDfBlock, smem) != cudaSuccess)
+        return 0;
+    return nb;
+}
+
 template <int FLUX>
 static int o1df_blocks_per_sm() {
     int nb = 0;
@@ -679,13 +901,14 @@ static cudaError_t launch_o1df(const O1Args& a, double4_32a* P, PersistCtl* pc, 
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(fvgb::kDfBlock);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = d.smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    if (d.smem) return cudaLaunchKernelEx(&cfg, k_o1_dataflow_sm<FLUX>, a, pc, d, nsteps);
     return cudaLaunchKernelEx(&cfg, k_o1_dataflow<FLUX>, a, P, pc, d, nsteps);
 }
 
@@ -738,6 +961,13 @@ int o1df_max_blocks_per_sm(int flux) {
         case 0: return ::FV_KNS::o1df_blocks_per_sm<0>();
         case 1: return ::FV_KNS::o1df_blocks_per_sm<1>();
         default: return ::FV_KNS::o1df_blocks_per_sm<2>();
+    }
+}
+int o1df_sm_max_blocks_per_sm(int flux, size_t smem) {
+    switch (flux) {
+        case 0: return ::FV_KNS::o1df_sm_blocks_per_sm<0>(smem);
+        case 1: return ::FV_KNS::o1df_sm_blocks_per_sm<1>(smem);
+        default: return ::FV_KNS::o1df_sm_blocks_per_sm<2>(smem);
     }
 }
 cudaError_t launch_o1_dataflow(const O1Args& a, double4_32a* P, PersistCtl* pc, const DfPlan& d, int nsteps,

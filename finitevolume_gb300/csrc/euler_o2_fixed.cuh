@@ -312,7 +312,8 @@ __global__ void __launch_bounds__(fvgb::kMaxBlock, 1) k_face_fx(const O2Args a) 
         if (R < 0) wr = ghost_fast(a, f, a.m.fl[f], wl, nx, ny);
         V4<double> F;
         double unused;
-        if (!fvfix::flux<FLUX == FLUX_HLLC ? 1 : 0, false, false>(wl, wr, 0.0, 0.0, nx, ny, ar, a.fxc, F, true, unused))
+        if (!fvfix::flux<FLUX == FLUX_HLLC ? 1 : 0, false, false>(wl, wr, 0.0, 0.0, fvfix::NoCons{}, fvfix::NoCons{}, nx,
+                                                                         ny, ar, a.fxc, F, true, unused))
             F = face_flux_f64<FLUX>(wl, wr, nx, ny, ar, a.gamma, a.igm1);
         st_flux(static_cast<St*>(a.ff), f, F);
         if (DT != 0) {

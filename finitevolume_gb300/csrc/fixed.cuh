@@ -121,6 +121,7 @@ __device__ __forceinline__ double scale2(double x, int k) {
 // and sound speeds are below 1, pressures below 1/gamma, everything else
 // below 8, the range of Q60.
 struct State { double r, u, v, p; };
+struct NoCons {};  // no conserved states given
 
 __device__ __forceinline__ float mant_float(double x, int k) {
     // mantissa of x (in [1, 2)) times 2^k, truncated to 24 bits
@@ -165,16 +166,18 @@ __device__ __forceinline__ i64 recip(i64 D) {
 __device__ __forceinline__ i64 iabs(i64 x) { return x < 0 ? -x : x; }
 
 // Flux times the face length: FLUX 0 Rusanov, 1 HLLC, on primitive inputs
-// (r, u, v, p) and, with C, the sound speeds.  False where the ranges do not
-// hold (F is not set then).  With LAM, lam is the face's largest wave speed
+// (r, u, v, p) and, with C, the sound speeds and the conserved states, whose
+// energies (and momenta, for Rusanov's dissipation) are taken instead of
+// formed.  False where the ranges do not hold (F is not set then).  With LAM, lam is the face's largest wave speed
 // max(|Vn| + c) over both sides, or the left one's (`both` false).
 //
 // Bound: the integer pipes (about 620 32-bit and 120 wide multiply-add
 // instructions for HLLC, next to the 8 FP64 ones that convert and scale the
 // result; the FP64 form takes 94 FP64 instructions a face).
-template <int FLUX, bool C, bool LAM, typename W>
-__device__ __forceinline__ bool flux(const W& L, const W& R, double cLd, double cRd, double nx, double ny, double ar,
-                                     const FluxConst& k, W& F, bool both, double& lam) {
+template <int FLUX, bool C, bool LAM, typename W, typename Cons>
+__device__ __forceinline__ bool flux(const W& L, const W& R, double cLd, double cRd, const Cons& UL, const Cons& UR,
+                                     double nx, double ny, double ar, const FluxConst& k, W& F, bool both,
+                                     double& lam) {
     const int rLh = hi_word(L.r), rRh = hi_word(R.r), pLh = hi_word(L.p), pRh = hi_word(R.p);
     const int erL = (int)((unsigned)rLh >> 20), erR = (int)((unsigned)rRh >> 20);  // sign included: must be clear
     const int epL = (int)((unsigned)pLh >> 20), epR = (int)((unsigned)pRh >> 20);
@@ -213,6 +216,10 @@ __device__ __forceinline__ bool flux(const W& L, const W& R, double cLd, double 
     const i64 pLq = shr_short(top_bits(L.p), ep1 + 3 - epL), pRq = shr_short(top_bits(R.p), ep1 + 3 - epR);
     const Sp pL = split(pLq), pR = split(pRq);
     const int evb = ev + 1023;  // above 1023 - 105
+    const int emb = er + 1 + ev, eeb = er + 3 + 2 * ev;  // units of momentum and of energy / 4
+    if constexpr (C) {
+        if (max(biased(hi_word(UL.E)), biased(hi_word(UR.E))) > eeb) return false;
+    }
     const Sp uL = split(to_fixed<60>(L.u, evb)), vL = split(to_fixed<60>(L.v, evb));
     const Sp uR = split(to_fixed<60>(R.u, evb)), vR = split(to_fixed<60>(R.v, evb));
     const Sp nX = split(to_fixed<60>(nx, 1023)), nY = split(to_fixed<60>(ny, 1023));
@@ -234,13 +241,23 @@ __device__ __forceinline__ bool flux(const W& L, const W& R, double cLd, double 
         const i64 S = max(iabs(VL) + cL, iabs(VR) + cR);
         const Sp S2 = split(S >> 1), vnL = split(VL), vnR = split(VR);
         const Sp mL = split(mul<4>(rL, vnL) >> 1), mR = split(mul<4>(rR, vnR) >> 1);  // half the mass fluxes
-        const Sp ig = split(k.igm1_4);
-        const i64 qL = mul<4>(uL, uL) + mul<4>(vL, vL), qR = mul<4>(uR, uR) + mul<4>(vR, vR);
-        const i64 EL = mul<4>(pL, ig) + (mul<4>(rL, split(qL)) >> 3), ER = mul<4>(pR, ig) + (mul<4>(rR, split(qR)) >> 3);
+        i64 EL, ER, du, dv;
+        if constexpr (C) {
+            EL = to_fixed<60>(UL.E, eeb);
+            ER = to_fixed<60>(UR.E, eeb);
+            du = to_fixed<60>(UR.ru, emb) - to_fixed<60>(UL.ru, emb);
+            dv = to_fixed<60>(UR.rv, emb) - to_fixed<60>(UL.rv, emb);
+        } else {
+            const Sp ig = split(k.igm1_4);
+            const i64 qL = mul<4>(uL, uL) + mul<4>(vL, vL), qR = mul<4>(uR, uR) + mul<4>(vR, vR);
+            EL = mul<4>(pL, ig) + (mul<4>(rL, split(qL)) >> 3);
+            ER = mul<4>(pR, ig) + (mul<4>(rR, split(qR)) >> 3);
+            du = mul<4>(rR, uR) - mul<4>(rL, uL);
+            dv = mul<4>(rR, vR) - mul<4>(rL, vL);
+        }
         const Sp ps = split((pLq >> 1) + (pRq >> 1));
         const i64 rLq = ((i64)rL.h << 32) + rL.l, rRq = ((i64)rR.h << 32) + rR.l;
         f0 = (mul<4>(rL, vnL) >> 1) + (mul<4>(rR, vnR) >> 1) - mul<4>(S2, split(rRq - rLq));
-        const i64 du = mul<4>(rR, uR) - mul<4>(rL, uL), dv = mul<4>(rR, vR) - mul<4>(rL, vL);
         f1 = mul<4>(mL, uL) + mul<4>(mR, uR) + mul<4>(ps, nX) - mul<4>(S2, split(du));
         f2 = mul<4>(mL, vL) + mul<4>(mR, vR) + mul<4>(ps, nY) - mul<4>(S2, split(dv));
         f3 = (mul<4>(split(EL + (pLq >> 2)), vnL) >> 1) + (mul<4>(split(ER + (pRq >> 2)), vnR) >> 1) -
@@ -258,8 +275,9 @@ __device__ __forceinline__ bool flux(const W& L, const W& R, double cLd, double 
         const Sp rK = left ? rL : rR, uK = left ? uL : uR, vK = left ? vL : vR, pK = left ? pL : pR;
         const i64 VK = left ? VL : VR, pKq = left ? pLq : pRq, SK = left ? SL : SR, mK = left ? mL : mR;
         const i64 dK = left ? dL : dR;
-        const i64 q2 = mul<4>(uK, uK) + mul<4>(vK, vK);
-        const i64 EK = mul<4>(pK, split(k.igm1_4)) + (mul<4>(rK, split(q2)) >> 3);  // E / 4
+        i64 EK;  // E / 4
+        if constexpr (C) EK = to_fixed<60>(left ? UL.E : UR.E, eeb);
+        else EK = mul<4>(pK, split(k.igm1_4)) + (mul<4>(rK, split(mul<4>(uK, uK) + mul<4>(vK, vK))) >> 3);
         i64 Ss, fac, Es, ps, w = 0;
         if (sup) {
             Ss = VK;

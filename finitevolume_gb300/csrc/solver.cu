@@ -7,6 +7,7 @@
 // host may change (CFL number, step counter) lives in device memory.
 #include <algorithm>
 #include <cfloat>
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -719,6 +720,60 @@ void Solver::build_dataflow(const HostMesh& hm, int sms) {
     dfp.prog = dalloc<unsigned int>((size_t)nb * kDfProgStride, owned);
     dfp.wpart = dalloc<double>((size_t)dfp.max_steps * Wn * 4, owned);
     dfp.n_warps = Wn;
+    // The shared-memory form where every block's cells (96 bytes each) and
+    // their faces (40) fit: up to about 1,100 cells a block, 170k a mesh.
+    // Larger meshes keep their states in L2 and are bound by the work itself.
+    dfp.smem = 0;
+    size_t own = 0;
+    for (int b = 0; b < nb; ++b)
+        own = std::max(own, 96 * (size_t)(p.cell_off[b + 1] - p.cell_off[b]) +
+                                40 * (size_t)(p.face_off[b + 1] - p.face_off[b]));
+    if (own <= kDfMaxSmem) {
+        std::vector<int> block_of(N), mail_of(N, -1), off(nb + 1, 0), xf, fin(nb, 0), slot(hm.d_cf.size(), -1), place(F);
+        std::vector<int2> xc;
+        for (int b = 0; b < nb; ++b)
+            for (int c = p.cell_off[b]; c < p.cell_off[b + 1]; ++c) block_of[c] = b;
+        int n_mail = 0;
+        auto between = [&](int f) { return hm.d_fr[f] >= 0 && block_of[hm.d_fl[f]] != block_of[hm.d_fr[f]]; };
+        for (int f = 0; f < F; ++f)
+            if (between(f))
+                for (int c : {hm.d_fl[f], hm.d_fr[f]})
+                    if (mail_of[c] < 0) mail_of[c] = n_mail++;
+        size_t smem = 0;
+        for (int b = 0; b < nb; ++b) {
+            const int c0 = p.cell_off[b], c1 = p.cell_off[b + 1];
+            // the plan's own faces in its order (boundary faces first), then
+            // those between blocks, owned or not, as this block's cells list them
+            auto add = [&](int f) {
+                place[f] = (int)xf.size() - off[b];
+                xf.push_back(f);
+                auto code = [&](int c) {
+                    return c < 0 ? INT_MIN : (block_of[c] == b ? c - c0 : -1 - mail_of[c]);
+                };
+                xc.push_back(make_int2(code(hm.d_fl[f]), code(hm.d_fr[f])));
+            };
+            for (int j = p.face_off[b]; j < p.face_off[b + 1]; ++j)
+                if (!between(p.faces[j])) add(p.faces[j]);
+            fin[b] = (int)xf.size() - off[b];
+            for (int c = c0; c < c1; ++c)
+                for (int e = hm.d_cf_off[c]; e < hm.d_cf_off[c + 1]; ++e)
+                    if (between(hm.d_cf[e] >> 1)) add(hm.d_cf[e] >> 1);
+            off[b + 1] = (int)xf.size();
+            for (int e = hm.d_cf_off[c0]; e < hm.d_cf_off[c1]; ++e) slot[e] = place[hm.d_cf[e] >> 1];
+            smem = std::max(smem, 96 * (size_t)(c1 - c0) + 40 * (size_t)(off[b + 1] - off[b]));
+        }
+        if (smem <= kDfMaxSmem && (opt.strict ? strict::o1df_sm_max_blocks_per_sm(opt.flux, smem)
+                                              : fast::o1df_sm_max_blocks_per_sm(opt.flux, smem)) >= 1) {
+            dfp.smem = smem;
+            dfp.xface_off = dupload(off, owned);
+            dfp.xfaces = dupload(xf, owned);
+            dfp.xcells = dupload(xc, owned);
+            dfp.face_in = dupload(fin, owned);
+            dfp.mail_of = dupload(mail_of, owned);
+            dfp.slot = dupload(slot, owned);
+            dfp.mail = dalloc<double2>(16 * (size_t)std::max(n_mail, 1), owned);
+        }
+    }
     df_grid = nb;
     dataflow_ok = true;
 }

@@ -91,9 +91,26 @@ struct DfPlan {
     double* wpart;            // [max_steps * n_warps * 4] per-warp partials
     int n_warps;              // cell warps, ceil(N / 32)
     int max_steps;            // steps per launch (wpart capacity)
+    // Form with the blocks' own cells and their faces' fluxes in shared memory
+    // (smem bytes a block; 0: in L2).  A block's faces are all of its cells',
+    // xfaces[xface_off[b] .. xface_off[b+1]), the face_in[b] ones that need no
+    // other block's cell first; xcells: their left and right cells, own ones
+    // as offsets from cell_off[b], others as -1 - mailbox (a boundary face's
+    // right cell as INT_MIN); slot: per cell-face entry the face's place in its
+    // cell's block; mail_of: each cell's mailbox or -1; mail: 16 words of 16
+    // bytes a mailbox.
+    size_t smem;
+    const int* xface_off;     // [nb+1]
+    const int* xfaces;        // [F + faces between blocks]
+    const int2* xcells;
+    const int* face_in;       // [nb]
+    const int* mail_of;       // [N]
+    double2* mail;
+    const int* slot;          // [E]
 };
 constexpr int kDfBlock = 512;          // threads per block (one block per SM)
 constexpr int kDfProgStride = 32;      // progress words per block (128 bytes)
+constexpr size_t kDfMaxSmem = 200u << 10;  // dynamic shared memory of the shared-memory form (17 KB more are static)
 constexpr int kDfMaxDeps = 32;         // dependency list bound per block and phase
 constexpr size_t kDfPartialBytes = 64u << 20;  // wpart budget (bounds steps per launch)
 
@@ -252,11 +269,13 @@ cudaError_t launch_o1_persistent(const O1Args& a, double4_32a* P, PersistCtl* pc
 // threads per block, at most one block per SM).
 namespace fast {
 int o1df_max_blocks_per_sm(int flux);
+int o1df_sm_max_blocks_per_sm(int flux, size_t smem);
 cudaError_t launch_o1_dataflow(const O1Args& a, double4_32a* P, PersistCtl* pc, const DfPlan& d, int nsteps,
                                int grid, cudaStream_t s);
 }  // namespace fast
 namespace strict {
 int o1df_max_blocks_per_sm(int flux);
+int o1df_sm_max_blocks_per_sm(int flux, size_t smem);
 cudaError_t launch_o1_dataflow(const O1Args& a, double4_32a* P, PersistCtl* pc, const DfPlan& d, int nsteps,
                                int grid, cudaStream_t s);
 }  // namespace strict

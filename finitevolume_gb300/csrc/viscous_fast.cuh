@@ -120,7 +120,8 @@ __device__ __forceinline__ double inviscid(const NSArgs& n, int f, int cl, int c
     vR = R.v;
     double smax;
     fvfix::State q;
-    if (ok && fvfix::flux<FLUX == FLUX_HLLC ? 1 : 0, false, true>(L, R, 0.0, 0.0, fg[6], fg[7], fg[1], n.fxc, q, cr >= 0,
+    if (ok && fvfix::flux<FLUX == FLUX_HLLC ? 1 : 0, false, true>(L, R, 0.0, 0.0, fvfix::NoCons{}, fvfix::NoCons{},
+                                                                  fg[6], fg[7], fg[1], n.fxc, q, cr >= 0,
                                                                   smax)) {
         F = st_make(q.r, q.u, q.v, q.p);
         // Equal densities: the Rusanov mass flux has no dissipation and is the

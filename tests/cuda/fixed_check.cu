@@ -3,6 +3,7 @@
 // (128-bit on the Arm machines that carry the GPU).
 //
 //   flux: random face states of several kinds, Rusanov and HLLC
+//   first: the same states as the first-order kernel's faces, conserved
 //   grad: random "cells" of 3 to 18 faces (18 takes the FP64 form), random weights,
 //         offsets and neighbours, both limiters
 // Each line: "<what> n N taken T rms_fixed A rms_fp64 B max_fixed C max_fp64 D",
@@ -15,6 +16,7 @@
 #include <vector>
 
 #define FV_KNS fast
+#include "euler_o1p.cuh"
 #include "euler_o2_fixed.cuh"
 
 using namespace fast;
@@ -28,19 +30,39 @@ __global__ void k_flux(const V* L, const V* R, const double4_32a* g, int n, fvfi
     if (i >= n) return;
     V F = {0, 0, 0, 0};
     double lam;
-    // every second face with its sound speeds given, as the first-order kernel does
-    if (i & 1)
-        took[i] = fvfix::flux<FLUX, true, false>(L[i], R[i], sqrt(gam * L[i].p / L[i].r), sqrt(gam * R[i].p / R[i].r),
-                                                 g[i].x, g[i].y, g[i].z, k, F, true, lam);
-    else
-        took[i] = fvfix::flux<FLUX, false, false>(L[i], R[i], 0.0, 0.0, g[i].x, g[i].y, g[i].z, k, F, true, lam);
+    took[i] = fvfix::flux<FLUX, false, false>(L[i], R[i], 0.0, 0.0, fvfix::NoCons{}, fvfix::NoCons{}, g[i].x, g[i].y,
+                                              g[i].z, k, F, true, lam);
     fx[i] = F;
     const V q = num_flux_p<double, FLUX>(L[i], R[i], g[i].x, g[i].y, gam, 1.0 / (gam - 1.0), 0.0, 0);
     f64[i] = {g[i].z * q.r, g[i].z * q.u, g[i].z * q.v, g[i].z * q.p};
 }
 
-static void flux_ld(int flux, const V& L, const V& R, LD nx, LD ny, LD ar, LD g, LD F[4]) {
-    const V* w[2] = {&L, &R};
+// the first-order kernel's face, from conserved states
+template <int FLUX>
+__global__ void k_first(const St* L, const St* R, const double4_32a* g, int n, fvfix::FluxConst k, double gam, V* fx, V* f64,
+                        int* took) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const Prim PL = prim_of(L[i], gam), PR = prim_of(R[i], gam);
+    V F;
+    double lam;
+    took[i] = fvfix::flux<FLUX, true, false>(fvfix::State{L[i].r, PL.u, PL.v, PL.p}, fvfix::State{R[i].r, PR.u, PR.v, PR.p},
+                                             PL.c, PR.c, L[i], R[i], g[i].x, g[i].y, g[i].z, k,
+                                             reinterpret_cast<fvfix::State&>(F), true, lam);
+    fx[i] = F;
+    const St q = g[i].z * num_flux_p<FLUX>(L[i], PL, R[i], PR, g[i].x, g[i].y, gam, 0.0, 0);
+    f64[i] = {q.r, q.ru, q.rv, q.E};
+}
+
+struct VL { LD r, u, v, p; };
+static VL wide(const V& w) { return {w.r, w.u, w.v, w.p}; }
+static VL wide(const St& s, LD g) {
+    const LD r = s.r, u = s.ru / r, v = s.rv / r;
+    return {r, u, v, (g - 1) * (s.E - r * (u * u + v * v) / 2)};
+}
+
+static void flux_ld(int flux, const VL& L, const VL& R, LD nx, LD ny, LD ar, LD g, LD F[4]) {
+    const VL* w[2] = {&L, &R};
     LD vn[2], vt[2], c[2], E[2], U[2][4], f[2][4];
     for (int s = 0; s < 2; ++s) {
         const LD r = w[s]->r, u = w[s]->u, v = w[s]->v, p = w[s]->p;
@@ -56,8 +78,8 @@ static void flux_ld(int flux, const V& L, const V& R, LD nx, LD ny, LD ar, LD g,
         return;
     }
     const LD SL = fminl(vn[0] - c[0], vn[1] - c[1]), SR = fmaxl(vn[0] + c[0], vn[1] + c[1]);
-    const LD mL = (LD)L.r * (SL - vn[0]), mR = (LD)R.r * (SR - vn[1]);
-    const LD Ss = ((LD)R.p - (LD)L.p + mL * vn[0] - mR * vn[1]) / (mL - mR);
+    const LD mL = L.r * (SL - vn[0]), mR = R.r * (SR - vn[1]);
+    const LD Ss = (R.p - L.p + mL * vn[0] - mR * vn[1]) / (mL - mR);
     const int s = SL >= 0 ? 0 : (SR <= 0 ? 1 : (Ss >= 0 ? 0 : 1));
     if (SL >= 0 || SR <= 0) {
         for (int k = 0; k < 4; ++k) F[k] = ar * f[s][k];
@@ -91,7 +113,7 @@ template <typename T> static std::vector<T> down(const T* p, size_t n) {
     return v;
 }
 
-template <int FLUX> static void check_flux(const char* name, int kind, double gam) {
+template <int FLUX> static void check_flux(const char* name, int kind, double gam, bool first) {
     const int n = 1 << 15;
     std::mt19937_64 rng(17 + kind);
     std::uniform_real_distribution<double> U(0.0, 1.0);
@@ -128,7 +150,16 @@ template <int FLUX> static void check_flux(const char* name, int kind, double ga
     V *fx, *f64;
     int* tk;
     cudaMalloc(&fx, sizeof(V) * n); cudaMalloc(&f64, sizeof(V) * n); cudaMalloc(&tk, sizeof(int) * n);
-    k_flux<FLUX><<<n / 256, 256>>>(up(L), up(R), up(g), n, k, gam, fx, f64, tk);
+    std::vector<St> UL(n), UR(n);
+    for (int i = 0; i < n; ++i)
+        for (int q = 0; q < 2; ++q) {
+            const V& w = q ? R[i] : L[i];
+            St& u = q ? UR[i] : UL[i];
+            u.r = w.r; u.ru = w.r * w.u; u.rv = w.r * w.v;
+            u.E = w.p / (gam - 1.0) + 0.5 * w.r * (w.u * w.u + w.v * w.v);
+        }
+    if (first) k_first<FLUX><<<n / 256, 256>>>(up(UL), up(UR), up(g), n, k, gam, fx, f64, tk);
+    else k_flux<FLUX><<<n / 256, 256>>>(up(L), up(R), up(g), n, k, gam, fx, f64, tk);
     auto a = down(fx, n), b = down(f64, n);
     auto took = down(tk, n);
     Err err;
@@ -141,7 +172,8 @@ template <int FLUX> static void check_flux(const char* name, int kind, double ga
     for (int i = 0; i < n; ++i) {
         if (!took[i]) continue;
         LD F[4];
-        flux_ld(FLUX, L[i], R[i], g[i].x, g[i].y, g[i].z, gam, F);
+        flux_ld(FLUX, first ? wide(UL[i], gam) : wide(L[i]), first ? wide(UR[i], gam) : wide(R[i]), g[i].x, g[i].y,
+                g[i].z, gam, F);
         const LD r = fmax(L[i].r, R[i].r), c = sqrt(gam * fmax(L[i].p / L[i].r, R[i].p / R[i].r));
         const LD q = fmaxl(c, hypot(L[i].u, L[i].v)), sc[4] = {r * q, r * q * q, r * q * q, r * q * q * q};
         const double *x = &a[i].r, *y = &b[i].r;
@@ -265,10 +297,12 @@ int main() {
         char s[64];
         const char* kinds[5] = {"smooth", "jumps", "lowmach", "aligned", "outside"};
         for (int k = 0; k < 5; ++k) {
-            snprintf(s, sizeof(s), "flux_rusanov_%s_%.2f", kinds[k], g);
-            check_flux<0>(s, k, g);
-            snprintf(s, sizeof(s), "flux_hllc_%s_%.2f", kinds[k], g);
-            check_flux<1>(s, k, g);
+            for (int first = 0; first < 2; ++first) {
+                snprintf(s, sizeof(s), "%s_rusanov_%s_%.2f", first ? "first" : "flux", kinds[k], g);
+                check_flux<0>(s, k, g, first);
+                snprintf(s, sizeof(s), "%s_hllc_%s_%.2f", first ? "first" : "flux", kinds[k], g);
+                check_flux<1>(s, k, g, first);
+            }
         }
     }
     const char* kinds[4] = {"smooth", "jumps", "stretched", "scaled"};
