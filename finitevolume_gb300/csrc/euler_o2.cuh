@@ -712,9 +712,10 @@ __device__ __forceinline__ double sound64(const V4<double>& w, double g) {
 
 // The signed sum of a cell's N face fluxes, component by component on the
 // integer pipe (the FP64 pipe bounds the update: N - 1 additions a component
-// there).
+// there).  R.ok: all four as integers.
+struct FixedState { fvfix::Fixed r, ru, rv, E; };
 template <int N>
-__device__ __forceinline__ St gather_fixed(const St* ff, const int* cf) {
+__device__ __forceinline__ bool gather_fixed(const St* ff, const int* cf, FixedState& R) {
     double x[4][N];
     int neg[N];
 #pragma unroll
@@ -724,18 +725,36 @@ __device__ __forceinline__ St gather_fixed(const St* ff, const int* cf) {
         x[0][i] = F.r; x[1][i] = F.ru; x[2][i] = F.rv; x[3][i] = F.E;
         neg[i] = ent;
     }
-    return st_make(fvfix::signed_sum<N>(x[0], neg), fvfix::signed_sum<N>(x[1], neg), fvfix::signed_sum<N>(x[2], neg),
-                   fvfix::signed_sum<N>(x[3], neg));
+    const bool a = fvfix::fixed_sum<N>(x[0], neg, R.r), b = fvfix::fixed_sum<N>(x[1], neg, R.ru);
+    const bool c = fvfix::fixed_sum<N>(x[2], neg, R.rv), d = fvfix::fixed_sum<N>(x[3], neg, R.E);
+    return a && b && c && d;
 }
-template <int N>
-__device__ __forceinline__ St gather_fixed(const float4*, const int*) { return {}; }  // FP32 flux: gather32
 
-// x / 4 by the exponent field where that is exact
+// x / 4 by the exponent field where that is exact; the product out of line,
+// as the compiler would otherwise issue it for every value
+static __device__ __noinline__ double quarter_product(double x) { return 0.25 * x; }
 __device__ __forceinline__ double quarter(double x) {
-    return fvfix::biased(fvfix::hi_word(x)) - 3u < 2040u ? fvfix::scale2(x, -2) : 0.25 * x;
+    if (fvfix::biased(fvfix::hi_word(x)) - 3u < 2040u) return fvfix::scale2(x, -2);
+    return quarter_product(x);
 }
 __device__ __forceinline__ St quarter(const St& s) {
     return st_make(quarter(s.r), quarter(s.ru), quarter(s.rv), quarter(s.E));
+}
+
+// The Shu-Osher combination of stage 1 or 2; out of line, as few cells need
+// it beside the fixed-point one below.
+template <int STAGE>
+__device__ __noinline__ St stage_f64(const St& u, const St& u0, const St& R, double dtv) {
+    const St e = u + dtv * R;
+    return STAGE == 1 ? 0.75 * u0 + 0.25 * e : (1.0 / 3.0) * u0 + (2.0 / 3.0) * e;
+}
+// The same on the integer pipe; false where
+// a component is out of range.
+template <int STAGE>
+__device__ __forceinline__ bool stage_fixed(const St& u, const St& u0, const FixedState& R, double dtv, St& un) {
+    const bool a = fvfix::rk_stage<STAGE>(u.r, u0.r, R.r, dtv, un.r), b = fvfix::rk_stage<STAGE>(u.ru, u0.ru, R.ru, dtv, un.ru);
+    const bool c = fvfix::rk_stage<STAGE>(u.rv, u0.rv, R.rv, dtv, un.rv), d = fvfix::rk_stage<STAGE>(u.E, u0.E, R.E, dtv, un.E);
+    return a && b && c && d;
 }
 
 // STAGE: 0..NST-1; NST: 1 (forward Euler) or 3 (SSP-RK3); DT: 1 global, 2 local.
@@ -748,15 +767,19 @@ __global__ void __launch_bounds__(fvgb::kMaxBlock) k_update(const O2Args a) {
         const FT* ff = static_cast<const FT*>(a.ff);
         const int e0 = a.m.cf_off[c], e1 = a.m.cf_off[c + 1];
         St R;
+        FixedState Rq;
+        bool fixed = false;  // R is in Rq
         double lam = 0.0;
         float lamf = 0.0f;
         if constexpr (std::is_same<T, float>::value) {
             R = gather32<STAGE == 0 && DT == 2>(ff, reinterpret_cast<const float*>(a.dtf), a.m.cf, e0, e1, lamf);
         } else {
             const int n = e1 - e0;
-            if (n == 4) R = gather_fixed<4>(ff, a.m.cf + e0);
-            else if (n == 3) R = gather_fixed<3>(ff, a.m.cf + e0);
-            else {
+            if (n == 4) fixed = gather_fixed<4>(ff, a.m.cf + e0, Rq);
+            else if (n == 3) fixed = gather_fixed<3>(ff, a.m.cf + e0, Rq);
+            if (fixed && (STAGE == 0 || a.forcing)) {
+                R = st_make(fvfix::value(Rq.r), fvfix::value(Rq.ru), fvfix::value(Rq.rv), fvfix::value(Rq.E));
+            } else if (!fixed) {
                 // Every cell has faces: the sum starts from the first signed flux
                 // instead of 0 + flux (one FP64 add per component less; only the
                 // sign of an exactly-zero sum can differ, and u + dt * (+-0) = u).
@@ -767,6 +790,7 @@ __global__ void __launch_bounds__(fvgb::kMaxBlock) k_update(const O2Args a) {
                     R += flip_if(ld_flux(ff, ent >> 1), ent);
                 }
             }
+            if (a.forcing) fixed = false;
             if (STAGE == 0 && DT == 2) {
                 lam = a.dtf[a.m.cf[e0] >> 1];
                 for (int e = e0 + 1; e < e1; ++e) lam += a.dtf[a.m.cf[e] >> 1];
@@ -795,12 +819,22 @@ __global__ void __launch_bounds__(fvgb::kMaxBlock) k_update(const O2Args a) {
             dtv = a.dtv[c];
         }
         const St u = ld_state(a.U, c);
-        const St e = u + dtv * R;
         St un;
-        if (NST == 1) un = e;
-        else if (STAGE == 0) { st_state(a.U0, c, u); un = e; }
-        else if (STAGE == 1) un = 0.75 * ld_state(a.U0, c) + quarter(e);
-        else un = (1.0 / 3.0) * ld_state(a.U0, c) + (2.0 / 3.0) * e;
+        if (STAGE == 0) {
+            if (NST > 1) st_state(a.U0, c, u);
+            un = u + dtv * R;
+        } else {
+            const St u0 = ld_state(a.U0, c);
+            if constexpr (std::is_same<T, float>::value) {
+                // FP64, which the loads hide (on the integer pipe 56 us a launch
+                // at 1.05M cells instead of 46)
+                const St e = u + dtv * R;
+                un = STAGE == 1 ? 0.75 * u0 + quarter(e) : (1.0 / 3.0) * u0 + (2.0 / 3.0) * e;
+            } else if (!fixed || !stage_fixed<STAGE>(u, u0, Rq, dtv, un)) {
+                if (fixed) R = st_make(fvfix::value(Rq.r), fvfix::value(Rq.ru), fvfix::value(Rq.rv), fvfix::value(Rq.E));
+                un = stage_f64<STAGE>(u, u0, R, dtv);
+            }
+        }
         st_state(a.U, c, un);
         const double g = a.gamma;
         if constexpr (std::is_same<T, float>::value) {

@@ -61,6 +61,7 @@ __device__ __forceinline__ i64 funnel(i64 hi, unsigned lo, int S) {
 template <int S>
 __device__ __forceinline__ i64 mul(const Sp& a, const Sp& b) {
     const i64 mid = madw(a.h, b.l, (i64)a.l * b.h);
+    if (S == 0) return madw(a.h, b.h, (i64)(int)(mid >> 32));
     return funnel(madw(a.h, b.h, (i64)(int)(mid >> 32)), (unsigned)mid, S);
 }
 template <int S> __device__ __forceinline__ i64 mul(i64 a, i64 b) { return mul<S>(split(a), split(b)); }
@@ -70,6 +71,8 @@ __device__ __forceinline__ i64 mul_u32(i64 v, unsigned m) {
     const u64 t = madwu((unsigned)v, m, 0);
     return funnel((i64)madwu((unsigned)((u64)v >> 32), m, t >> 32), (unsigned)t, S);
 }
+
+__device__ __forceinline__ i64 iabs(i64 x) { return x < 0 ? -x : x; }
 
 __device__ __forceinline__ int hi_word(double x) { return __double2hiint(x); }
 __device__ __forceinline__ int biased(int hi) { return (hi >> 20) & 0x7ff; }
@@ -163,7 +166,6 @@ __device__ __forceinline__ i64 recip(i64 D) {
     const i64 t = (i64)q.l * R0;
     return ((i64)R0 << 32) + funnel(madw(q.h, R0, (i64)(int)(t >> 32)), (unsigned)t, 2);
 }
-__device__ __forceinline__ i64 iabs(i64 x) { return x < 0 ? -x : x; }
 
 // Flux times the face length: FLUX 0 Rusanov, 1 HLLC, on primitive inputs
 // (r, u, v, p) and, with C, the sound speeds and the conserved states, whose
@@ -344,24 +346,54 @@ __device__ __forceinline__ bool sound_speed(double r, double p, double g, double
     return true;
 }
 
+// m * 2^k
+struct Fixed { i64 m; int k; };
+__device__ __forceinline__ double value(const Fixed& x) { return to_double(x.m, x.k); }
+
 // The signed sum of N FP64 values (bit 0 of neg[i] flips the sign of x[i]) in
-// fixed point: exact but for bits below 2^-59 of the largest, one FP64
-// instruction instead of N - 1.
+// fixed point: exact but for bits below 2^-59 of the largest.  False where a
+// value is not finite, or all are zero or below 2^-873.
 template <int N>
-__device__ __forceinline__ double signed_sum(const double (&x)[N], const int (&neg)[N]) {
+__device__ __forceinline__ bool fixed_sum(const double (&x)[N], const int (&neg)[N], Fixed& s) {
     int E = 0;
 #pragma unroll
     for (int i = 0; i < N; ++i) E = max(E, biased(hi_word(x[i])));
-    if ((unsigned)(E - 150) > 1750u) {  // all zero, tiny, huge or not finite
-        double s = 0.0;
+    s.m = 0;
 #pragma unroll
-        for (int i = 0; i < N; ++i) s += neg[i] & 1 ? -x[i] : x[i];
-        return s;
-    }
-    i64 s = 0;
+    for (int i = 0; i < N; ++i) s.m += to_fixed<59>(x[i], E, -(neg[i] & 1));
+    s.k = E - 1023 - 59;
+    return (unsigned)(E - 150) <= 1750u;
+}
+template <int N>
+__device__ __forceinline__ double signed_sum(const double (&x)[N], const int (&neg)[N]) {
+    Fixed q;
+    if (fixed_sum<N>(x, neg, q)) return value(q);
+    double s = 0.0;
 #pragma unroll
-    for (int i = 0; i < N; ++i) s += to_fixed<59>(x[i], E, -(neg[i] & 1));
-    return to_double(s, E - 1023 - 59);
+    for (int i = 0; i < N; ++i) s += neg[i] & 1 ? -x[i] : x[i];
+    return s;
+}
+// One component of a Shu-Osher stage, with e = u + dtv R: stage 1 (3 u0 + e) / 4,
+// stage 2 (u0 + 2 e) / 3, as integers in units of 2^-59 of the largest term's
+// binade (an FP64 form rounds three or four times at 2^-53).  False out of
+// range.
+template <int STAGE>
+__device__ __forceinline__ bool rk_stage(double u, double u0, const Fixed& R, double dtv, double& un) {
+    const int ed = (int)((unsigned)hi_word(dtv) >> 20);  // sign included: must be clear
+    const i64 mag = iabs(R.m);
+    const int lz = mag ? __clzll(mag) : 63;
+    const int er = R.k + 64 - lz + ed;  // above the biased exponent of dtv R
+    const int E = max(max(biased(hi_word(u)), biased(hi_word(u0))), er);
+    // dtv R: R's leading bit at 2^62 times dtv's at 2^62, >> 64: below 2^61 in
+    // units of 2^(er - 1023 - 61)
+    const i64 p = mul<0>(split(R.m << (lz - 1)), split((i64)(top_bits(dtv) >> 1)));
+    i64 q;
+    asm("shr.s64 %0, %1, %2;" : "=l"(q) : "l"(p), "r"(E - er + 1));
+    const i64 a = to_fixed<59>(u0, E), e = to_fixed<59>(u, E) + ((q + 1) >> 1);
+    // rounded, not floored: a floor's bias would add up over the steps
+    const i64 s = STAGE == 1 ? (a + a + a + e + 2) >> 2 : mul<2>(split(a + e + e + 1), split(0x1555555555555555ll));
+    un = to_double(s, E - 1023 - 59);
+    return (unsigned)(E - 150) <= 1750u && (unsigned)(ed - 123) < 1800u && lz > 0;
 }
 
 // num / den * 2^52, rounded, for 0 < num <= den, den in [2^56, 2^62): three
