@@ -101,56 +101,67 @@ __global__ void __launch_bounds__(fvgb::kFaceBlock) k_face_o1(const O1Args a) {
     }
 }
 
-// Fold one block's four squared-residual sums into partials[blockIdx];
-// the last block to arrive folds all partials (fixed order) into the
-// norms, records the history row, and re-arms the control block.
-__device__ __forceinline__ void finish_norms(double s0, double s1, double s2, double s3, StepCtl* ctl,
-                                             double* partials, double* hist, int hist_cap) {
+// One block's four squared-residual sums into partials[blockIdx].
+__device__ __forceinline__ void block_partial(double s0, double s1, double s2, double s3, double* partials) {
     // up to 512 threads per block (launch shapes are tunable)
     __shared__ double red[16][4];
-    __shared__ bool last;
-    const int nw = blockDim.x >> 5;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const double ws = warp_sum4(s0, s1, s2, s3);
     if ((lane & 7) == 0) red[w][lane >> 3] = ws;
     __syncthreads();
     if (threadIdx.x < 4) {
         double v = 0.0;
-        for (int i = 0; i < nw; ++i) v += red[i][threadIdx.x];
+        for (int i = 0; i < (int)(blockDim.x >> 5); ++i) v += red[i][threadIdx.x];
         partials[blockIdx.x * 4 + threadIdx.x] = v;
     }
+}
+
+// All n blocks' partials, by one block and in fixed order, into the norms;
+// records the history row and re-arms the control block.
+__device__ __forceinline__ void fold_partials(int n, StepCtl* ctl, const double* partials, double* hist,
+                                              int hist_cap) {
+    __shared__ double red[16][4];
+    const int nw = blockDim.x >> 5;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double t[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int b = threadIdx.x; b < n; b += blockDim.x) {
+        const volatile double* p = partials + 4 * b;
+        t[0] += p[0]; t[1] += p[1]; t[2] += p[2]; t[3] += p[3];
+    }
+    const double ts = warp_sum4(t[0], t[1], t[2], t[3]);
+    if ((lane & 7) == 0) red[w][lane >> 3] = ts;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double n4[4];
+        int bad = 0;
+        for (int k = 0; k < 4; ++k) {
+            double v = 0.0;
+            for (int i = 0; i < nw; ++i) v += red[i][k];
+            n4[k] = sqrt(v);
+            if (!isfinite(n4[k])) bad = 1;
+            ctl->norms[k] = n4[k];
+        }
+        const int row = ctl->step % hist_cap;
+        for (int k = 0; k < 4; ++k) hist[row * 4 + k] = n4[k];
+        if (bad) ctl->nonfinite = 1;
+        ctl->step += 1;
+        ctl->done_blocks = 0u;
+        ctl->dt_bits = (unsigned long long)__double_as_longlong(DBL_MAX);
+    }
+}
+
+// Both in one kernel: the last block to finish folds.
+__device__ __forceinline__ void finish_norms(double s0, double s1, double s2, double s3, StepCtl* ctl,
+                                             double* partials, double* hist, int hist_cap) {
+    __shared__ bool last;
+    block_partial(s0, s1, s2, s3, partials);
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) last = (atomicAdd(&ctl->done_blocks, 1u) == gridDim.x - 1);
     __syncthreads();
     if (!last) return;
     __threadfence();
-    double t[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) {
-        const volatile double* p = partials + 4 * b;
-        t[0] += p[0]; t[1] += p[1]; t[2] += p[2]; t[3] += p[3];
-    }
-    const double ts = warp_sum4(t[0], t[1], t[2], t[3]);
-    __syncthreads();
-    if ((lane & 7) == 0) red[w][lane >> 3] = ts;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double n[4];
-        int bad = 0;
-        for (int k = 0; k < 4; ++k) {
-            double v = 0.0;
-            for (int i = 0; i < nw; ++i) v += red[i][k];
-            n[k] = sqrt(v);
-            if (!isfinite(n[k])) bad = 1;
-            ctl->norms[k] = n[k];
-        }
-        const int row = ctl->step % hist_cap;
-        for (int k = 0; k < 4; ++k) hist[row * 4 + k] = n[k];
-        if (bad) ctl->nonfinite = 1;
-        ctl->step += 1;
-        ctl->done_blocks = 0u;
-        ctl->dt_bits = (unsigned long long)__double_as_longlong(DBL_MAX);
-    }
+    fold_partials((int)gridDim.x, ctl, partials, hist, hist_cap);
 }
 
 template <bool LOCAL>

@@ -849,7 +849,13 @@ __global__ void __launch_bounds__(fvgb::kMaxBlock) k_update(const O2Args a) {
     }
     // Batched solves reduce per instance instead (k_batch_norms); a.r2 is
     // uniform over the grid, so the block-wide reduction is all-or-nothing.
-    if (STAGE == 0 && !a.r2) finish_norms(s0, s1, s2, s3, a.ctl, a.partials, a.hist, a.hist_cap);
+    if (a.r2) return;
+    // With three stages the fold waits for the next update, whose first block
+    // does it beside the others' work (the grid is the same): stage 0 then
+    // has no fence, no counter and no last block that works alone.
+    if (STAGE == 0 && NST == 1) finish_norms(s0, s1, s2, s3, a.ctl, a.partials, a.hist, a.hist_cap);
+    if (STAGE == 0 && NST == 3) block_partial(s0, s1, s2, s3, a.partials);
+    if (STAGE == 1 && blockIdx.x == 0) fold_partials((int)gridDim.x, a.ctl, a.partials, a.hist, a.hist_cap);
 }
 
 // Residual only (multigrid restriction): the same signed gather as
