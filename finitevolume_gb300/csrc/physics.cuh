@@ -34,6 +34,10 @@ __device__ __forceinline__ double rmax(double a, double b) { return (a < b) ? b 
 __device__ __forceinline__ float rmax(float a, float b) { return (a < b) ? b : a; }
 __device__ __forceinline__ double rmin(double a, double b) { return (b < a) ? b : a; }
 
+// A line that the thread will read behind a chain of other loads, asked for at
+// once: costs no register.
+__device__ __forceinline__ void prefetch(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
 // One 256-bit access per state (32-byte aligned): as two 128-bit ones a warp's
 // gather takes twice the L1 cycles, each half touching every line.
 __device__ __forceinline__ St ld_state(const St* __restrict__ U, int i) {
