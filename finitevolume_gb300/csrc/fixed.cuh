@@ -33,7 +33,7 @@ using i64 = long long;
 using u64 = unsigned long long;
 
 // v = h * 2^32 + l with l signed, so that all partial products are
-// signed 32 x 32.
+// signed 32 x 32; v below 2^63 - 2^31, as h rounds up.
 struct Sp { int h, l; };
 __device__ __forceinline__ Sp split(i64 v) {
     const int l = (int)v;
@@ -330,8 +330,13 @@ __device__ __forceinline__ bool flux(const W& L, const W& R, double cLd, double 
     return true;
 }
 
-// Sound speed sqrt(g p / r) within an ulp, with one FP64 instruction (the
-// FP64 form takes ten); false outside the ranges.
+// a * b >> 60 to one unit: mul<4> with the low halves' product
+__device__ __forceinline__ i64 mul_low(const Sp& a, const Sp& b) {
+    const i64 mid = madw(a.h, b.l, madw(a.l, b.h, (i64)a.l * b.l >> 32));
+    return funnel(madw(a.h, b.h, (i64)(int)(mid >> 32)), (unsigned)mid, 4);
+}
+// Sound speed sqrt(g p / r) rounded once but for 2^-56 of it, with one FP64
+// instruction (the FP64 form takes ten); false outside the ranges.
 __device__ __forceinline__ bool sound_speed(double r, double p, double g, double& c) {
     const int er = (int)((unsigned)hi_word(r) >> 20), ep = (int)((unsigned)hi_word(p) >> 20);
     const int eg = (int)((unsigned)hi_word(g) >> 20) - 1023;  // 0 or 1: gamma in [1, 4)
@@ -339,10 +344,10 @@ __device__ __forceinline__ bool sound_speed(double r, double p, double g, double
     // r = m 2^er, p = q 2^(er + 2 kc) with q in [1, 4): c = sqrt(g q / m) 2^kc
     const int kc = (ep - er) >> 1, odd = (ep - er) & 1;
     const float y = rsqrt_f((float)g * mant_float(p, odd) * mant_float(r, 0));
-    const i64 m4 = shr_short(top_bits(r), 5), g2 = shr_short(top_bits(g), 4 - eg), q8 = shr_short(top_bits(p), 6 - odd);
-    const i64 gq = mul<4>(g2, q8);    // g q / 16
-    const i64 x = mul<4>(gq, m4);     // g q m / 64
-    c = scale2(__ll2double_rn(sound(gq, x, (unsigned)__float2int_rn(y * 134217728.0f))), kc + 1 - 60);  // Q24 of 8 y
+    const i64 m4 = shr_short(top_bits(r), 5), g2 = shr_short(top_bits(g), 4 - eg), q2 = shr_short(top_bits(p), 4 - odd);
+    const i64 gq = mul_low(split(g2), split(q2));  // g q / 4, below 4
+    const i64 x = mul_low(split(gq), split(m4));   // g q m / 16, below 2
+    c = scale2(__ll2double_rn(sound(gq, x, (unsigned)__float2int_rn(y * 67108864.0f))), kc - 60);  // Q24 of 4 y
     return true;
 }
 
@@ -384,16 +389,17 @@ __device__ __forceinline__ bool rk_stage(double u, double u0, const Fixed& R, do
     const int lz = mag ? __clzll(mag) : 63;
     const int er = R.k + 64 - lz + ed;  // above the biased exponent of dtv R
     const int E = max(max(biased(hi_word(u)), biased(hi_word(u0))), er);
-    // dtv R: R's leading bit at 2^62 times dtv's at 2^62, >> 64: below 2^61 in
-    // units of 2^(er - 1023 - 61)
-    const i64 p = mul<0>(split(R.m << (lz - 1)), split((i64)(top_bits(dtv) >> 1)));
+    // dtv R: R's leading bit at 2^61 times dtv's at 2^61 (one place higher,
+    // a mantissa of ones would overflow split's high half), >> 62: below 2^62
+    // in units of 2^(er - 1023 - 62)
+    const i64 p = mul<2>(split(R.m << (lz - 2)), split((i64)(top_bits(dtv) >> 2)));
     i64 q;
     asm("shr.s64 %0, %1, %2;" : "=l"(q) : "l"(p), "r"(E - er + 1));
     const i64 a = to_fixed<59>(u0, E), e = to_fixed<59>(u, E) + ((q + 1) >> 1);
     // rounded, not floored: a floor's bias would add up over the steps
     const i64 s = STAGE == 1 ? (a + a + a + e + 2) >> 2 : mul<2>(split(a + e + e + 1), split(0x1555555555555555ll));
     un = to_double(s, E - 1023 - 59);
-    return (unsigned)(E - 150) <= 1750u && (unsigned)(ed - 123) < 1800u && lz > 0;
+    return (unsigned)(E - 150) <= 1750u && (unsigned)(ed - 123) < 1800u && lz > 1;
 }
 
 // num / den * 2^52, rounded, for 0 < num <= den, den in [2^56, 2^62): three
