@@ -101,12 +101,12 @@ __global__ void __launch_bounds__(fvgb::kFaceBlock) k_face_o1(const O1Args a) {
     }
 }
 
-// One block's four squared-residual sums into partials[blockIdx].
-__device__ __forceinline__ void block_partial(double s0, double s1, double s2, double s3, double* partials) {
+// One block's four squared-residual sums, from its warps' (ws, as warp_sum4
+// leaves them), into partials[blockIdx].
+__device__ __forceinline__ void block_partial(double ws, double* partials) {
     // up to 512 threads per block (launch shapes are tunable)
     __shared__ double red[16][4];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const double ws = warp_sum4(s0, s1, s2, s3);
     if ((lane & 7) == 0) red[w][lane >> 3] = ws;
     __syncthreads();
     if (threadIdx.x < 4) {
@@ -151,10 +151,9 @@ __device__ __forceinline__ void fold_partials(int n, StepCtl* ctl, const double*
 }
 
 // Both in one kernel: the last block to finish folds.
-__device__ __forceinline__ void finish_norms(double s0, double s1, double s2, double s3, StepCtl* ctl,
-                                             double* partials, double* hist, int hist_cap) {
+__device__ __forceinline__ void finish_norms(double ws, StepCtl* ctl, double* partials, double* hist, int hist_cap) {
     __shared__ bool last;
-    block_partial(s0, s1, s2, s3, partials);
+    block_partial(ws, partials);
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) last = (atomicAdd(&ctl->done_blocks, 1u) == gridDim.x - 1);
@@ -183,7 +182,7 @@ __global__ void __launch_bounds__(fvgb::kCellBlock) k_cell_o1(const O1Args a) {
         const St u = ld_state(a.U, c);
         st_state(a.U, c, u + (dt / a.m.vol[c]) * R);
     }
-    finish_norms(s0, s1, s2, s3, a.ctl, a.partials, a.hist, a.hist_cap);
+    finish_norms(warp_sum4(s0, s1, s2, s3), a.ctl, a.partials, a.hist, a.hist_cap);
 }
 
 template <int FLUX>

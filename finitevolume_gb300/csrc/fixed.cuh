@@ -402,6 +402,48 @@ __device__ __forceinline__ bool rk_stage(double u, double u0, const Fixed& R, do
     return (unsigned)(E - 150) <= 1750u && (unsigned)(ed - 123) < 1800u && lz > 1;
 }
 
+// a / s for a > 0 and a sum s > 0 of the above, rounded once but for 2^-55 of
+// it; false out of range.
+__device__ __forceinline__ bool quotient(double a, const Fixed& s, double& q) {
+    const int ea = (int)((unsigned)hi_word(a) >> 20);  // sign included: must be clear
+    if ((unsigned)(ea - 123) >= 1800u || s.m <= 0) return false;
+    const int lz = __clzll(s.m);  // at least 2
+    const i64 D = lz >= 3 ? s.m << (lz - 3) : s.m >> 1;  // in [1, 2) of Q60, times 2^(s.k + 63 - lz)
+    const i64 x = mul_low(split((i64)(top_bits(a) >> 3)), split(recip(D)));  // Q58
+    q = to_double(x, ea - 1023 - (s.k + 63 - lz) - 58);
+    return abs(ea - 1023 - (s.k + 63 - lz)) < 900;
+}
+// The sums over a warp of x^2 for four values a lane (all 32 lanes call it):
+// the k-th in the lanes 8 k to 8 k + 7, as warp_sum4's.  Squares as integers
+// in units of 2^-57 of the warp's largest binade (below 2^59, the sum below
+// 2^64), rounded and added exactly: one FP64 instruction instead of ten.
+// False (on all lanes) where a value is not finite or its square out of range.
+__device__ __forceinline__ bool warp_squares4(const double (&x)[4], double& sum) {
+    u64 v[4];
+    int E[4], bad = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int e = biased(hi_word(x[k]));
+        E[k] = __reduce_max_sync(0xffffffffu, e);
+        bad |= E[k] > 1500 || (E[k] != 0 && E[k] < 550);
+        const Sp m = split((i64)(top_bits(x[k]) >> 3));  // Q60, in [1, 2)
+        v[k] = e == 0 ? 0 : (shr((u64)mul<1>(m, m) << 1, 2 * (E[k] - e)) + 1) >> 1;
+    }
+    const int lane = threadIdx.x & 31;
+    const bool h16 = lane & 16, h8 = lane & 8;
+    u64 a = h16 ? v[2] : v[0], b = h16 ? v[3] : v[1];
+    a += __shfl_xor_sync(0xffffffffu, h16 ? v[0] : v[2], 16);
+    b += __shfl_xor_sync(0xffffffffu, h16 ? v[1] : v[3], 16);
+    u64 s = h8 ? b : a;
+    s += __shfl_xor_sync(0xffffffffu, h8 ? a : b, 8);
+    s += __shfl_xor_sync(0xffffffffu, s, 4);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    const int e = h16 ? (h8 ? E[3] : E[2]) : (h8 ? E[1] : E[0]);
+    sum = s == 0 ? 0.0 : scale2(__ull2double_rn(s), 2 * (e - 1023) - 57);
+    return bad == 0;
+}
+
 // num / den * 2^52, rounded, for 0 < num <= den, den in [2^56, 2^62): three
 // quotient digits of 20, 20 and 12 bits, each from the float quotient of
 // the exact remainder (within 3/4 of a unit).

@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(fvgb::kCellBlock) k_ns_cell(const O1Args a) {
         s0 = R.r * R.r; s1 = R.ru * R.ru; s2 = R.rv * R.rv; s3 = R.E * R.E;
         st_state(a.U, c, ld_state(a.U, c) + (dt * fvconv::rcp_nr3(a.m.vol[c])) * R);
     }
-    finish_norms(s0, s1, s2, s3, a.ctl, a.partials, a.hist, a.hist_cap);
+    finish_norms(warp_sum4(s0, s1, s2, s3), a.ctl, a.partials, a.hist, a.hist_cap);
 }
 #else
 __global__ void __launch_bounds__(fvgb::kCellBlock) k_ns_prim(const NSArgs a) {

@@ -6,6 +6,9 @@
 //          with all mantissa bits set, fluxes with all of them set, sums that
 //          cancel, step factors and states of very different sizes
 //   sound: sound speeds (kind 0)
+//   dt: a step factor over a sum of wave speeds (kind 0)
+//   squares: a warp's sums of squares; kinds: like sizes, sizes 2^30 apart,
+//            one value far above the others, mantissas of all ones, one zero column
 // Each line: "<what> kind K n N taken T rms_fixed A rms_fp64 B max_fixed C max_fp64 D",
 // errors relative to the largest term.
 #include <cmath>
@@ -47,6 +50,30 @@ __global__ void k_sound(const In* in, int n, Out* out) {
     out[i].took = fvfix::sound_speed(r, p, g, c);
     out[i].fx = c;
     out[i].f64 = sqrt(g * p / r);
+}
+
+__global__ void k_dt(const In* in, int n, Out* out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    double x[4], s = 0.0, q = 0.0;
+    int none[4] = {0, 0, 0, 0};
+    for (int k = 0; k < 4; ++k) s += x[k] = fabs(in[i].x[k]);
+    fvfix::Fixed R;
+    const bool ok = fvfix::fixed_sum<4>(x, none, R) && fvfix::quotient(in[i].dtv, R, q);
+    out[i].took = ok;
+    out[i].fx = q;
+    out[i].f64 = in[i].dtv / s;
+}
+
+// n lanes, whole warps; the sum of value k of a warp in its lanes 8 k to 8 k + 7
+__global__ void k_squares(const In* in, int n, Out* out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    double x[4], s = 0.0;
+    for (int k = 0; k < 4; ++k) x[k] = in[i].x[k];
+    out[i].took = fvfix::warp_squares4(x, s);
+    out[i].fx = s;
+    out[i].f64 = warp_sum4(x[0] * x[0], x[1] * x[1], x[2] * x[2], x[3] * x[3]);
 }
 
 template <class K, class Ref>
@@ -109,7 +136,29 @@ int main() {
             if (st == 1) run("stage1", kind, in, k_stage<1>, ref);
             else run("stage2", kind, in, k_stage<2>, ref);
         }
+        std::vector<In> sq(32 * 4000);
+        for (size_t i = 0; i < sq.size(); ++i) {
+            for (int k = 0; k < 4; ++k) {
+                double& x = sq[i].x[k];
+                x = U(rng) * (kind == 1 ? std::exp2(15 * U(rng)) : kind == 2 && i % 32 == 5 ? 1e6 : 1.0);
+                if (kind == 3) x = full(x);
+                if (kind == 4 && k == 2) x = 0.0;
+            }
+        }
+        run("squares", kind, sq, k_squares, [&](const In& q, LD& s) {
+            const size_t i = &q - sq.data(), w = i & ~(size_t)31;
+            s = 0;
+            for (int l = 0; l < 32; ++l) { const LD x = sq[w + l].x[i / 8 % 4]; s += x * x; }
+            const LD sum = s;
+            if (s == 0) s = 1;
+            return sum;
+        });
         if (kind != 0) continue;
+        run("dt", kind, in, k_dt, [&](const In& q, LD& s) {
+            LD t = 0;
+            for (double x : q.x) t += fabsl(x);
+            return s = q.dtv / t;
+        });
         for (In& q : in) q.u = 1.2 + 0.9 * (1.0 + U(rng));
         run("sound", kind, in, k_sound, [&](const In& q, LD& s) {
             return s = sqrtl((LD)q.u * fabsl(q.x[1]) / fabsl(q.x[0]));
