@@ -128,6 +128,12 @@ __device__ __forceinline__ V4<double> ghost_fast(const O2Args& a, int f, int cel
     return {w.r, w.u - 2.0 * Vn * nx, w.v - 2.0 * Vn * ny, w.p};
 }
 
+// A third boundary face of one cell: rare, out of line
+static __device__ __noinline__ V4<double> ghost_more(const O2Args& a, int f, int c) {
+    const double4_32a q = a.m.fgeom[f];
+    return ghost_fast(a, f, c, WStore<double>::ld(static_cast<const St*>(a.W), c), q.x, q.y);
+}
+
 // One variable k of one cell.  The four lanes of a cell meet at the votes:
 // an FP64 cell is one for all its variables, and a face state that is not
 // positive falls back to the cell's.  N: the cell's face count (3 or 4, its
@@ -139,17 +145,30 @@ __device__ __forceinline__ void grad_lane(const O2Args& a, int c, int k, int e0,
     const double* W = static_cast<const double*>(a.W);
     const int n = N ? N : e1 - e0;
     const double wc = __ldg(W + 4 * (size_t)c + k);
-    // values across the faces (boundary: the mean of the cell's and the ghost's)
-    auto boundary = [&](int f) -> double {
+    // Values across the faces; a boundary face's is the mean of the cell's and
+    // the ghost's.  A ghost is a long FP64 chain (2 to 3 us) and a warp's cells
+    // have their boundary faces at different places: each lane forms the ghost
+    // of one face, all at once, and the quad shares them.
+    auto ghost = [&](int f) -> V4<double> {
         const double4_32a q = a.m.fgeom[f];
-        const V4<double> gh = ghost_fast(a, f, c, WStore<double>::ld(static_cast<const St*>(a.W), c), q.x, q.y);
-        return 0.5 * (wc + (k == 0 ? gh.r : (k == 1 ? gh.u : (k == 2 ? gh.v : gh.p))));
+        return ghost_fast(a, f, c, WStore<double>::ld(static_cast<const St*>(a.W), c), q.x, q.y);
     };
-    double wn[N ? N : 1], wb = 0.0;
-    int eb = -1;
+    auto mean = [&](double r, double u, double v, double p) {
+        return 0.5 * (wc + (k == 0 ? r : (k == 1 ? u : (k == 2 ? v : p))));
+    };
+    auto share = [&](const V4<double>& g, int lane) {
+        return mean(__shfl_sync(quad, g.r, lane, 4), __shfl_sync(quad, g.u, lane, 4), __shfl_sync(quad, g.v, lane, 4),
+                    __shfl_sync(quad, g.p, lane, 4));
+    };
+    double wn[N ? N : 1], wb0 = 0.0, wb1 = 0.0;
+    int b0 = -1, b1 = -1;
     auto across = [&](int e) -> double {  // N = 0 only
         const int nb = a.cnb[e];
-        return nb >= 0 ? __ldg(W + 4 * (size_t)nb + k) : (e == eb ? wb : boundary(-1 - nb));
+        if (nb >= 0) return __ldg(W + 4 * (size_t)nb + k);
+        if (e == b0) return wb0;
+        if (e == b1) return wb1;
+        const V4<double> g = ghost_more(a, -1 - nb, c);
+        return mean(g.r, g.u, g.v, g.p);
     };
     int E = biased(hi_word(wc));
     if constexpr (N != 0) {
@@ -160,18 +179,29 @@ __device__ __forceinline__ void grad_lane(const O2Args& a, int c, int k, int e0,
 #pragma unroll
         for (int i = 0; i < N; ++i) wn[i] = __ldg(W + 4 * (size_t)(nb[i] < 0 ? c : nb[i]) + k);
         if (any < 0) {
+            V4<double> g = {0.0, 0.0, 0.0, 0.0};
+            const int mine = k < N ? a.cnb[e0 + k] : 0;
+            if (mine < 0) g = ghost(-1 - mine);
 #pragma unroll
             for (int i = 0; i < N; ++i)
-                if (nb[i] < 0) wn[i] = boundary(-1 - nb[i]);
+                if (nb[i] < 0) wn[i] = share(g, i);
         }
 #pragma unroll
         for (int i = 0; i < N; ++i) E = max(E, biased(hi_word(wn[i])));
     } else {
         for (int e = e0; e < e1; ++e) {
-            const double w = across(e);
-            if (eb < 0 && a.cnb[e] < 0) { eb = e; wb = w; }
-            E = max(E, biased(hi_word(w)));
+            if (a.cnb[e] >= 0) continue;
+            if (b0 < 0) b0 = e;
+            else if (b1 < 0) b1 = e;
         }
+        if (b0 >= 0) {
+            V4<double> g = {0.0, 0.0, 0.0, 0.0};
+            const int mine = k == 0 ? b0 : (k == 1 ? b1 : -1);
+            if (mine >= 0) g = ghost(-1 - a.cnb[mine]);
+            wb0 = share(g, 0);
+            wb1 = share(g, 1);
+        }
+        for (int e = e0; e < e1; ++e) E = max(E, biased(hi_word(across(e))));
     }
     const int S = a.fxs[c];
     // out of range: the arithmetic below still runs, its result is not used
