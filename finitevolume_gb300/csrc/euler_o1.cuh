@@ -131,20 +131,17 @@ __device__ __forceinline__ void fold_partials(int n, StepCtl* ctl, const double*
     const double ts = warp_sum4(t[0], t[1], t[2], t[3]);
     if ((lane & 7) == 0) red[w][lane >> 3] = ts;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double n4[4];
-        int bad = 0;
-        for (int k = 0; k < 4; ++k) {
-            double v = 0.0;
-            for (int i = 0; i < nw; ++i) v += red[i][k];
-            n4[k] = sqrt(v);
-            if (!isfinite(n4[k])) bad = 1;
-            ctl->norms[k] = n4[k];
-        }
-        const int row = ctl->step % hist_cap;
-        for (int k = 0; k < 4; ++k) hist[row * 4 + k] = n4[k];
+    if (threadIdx.x < 4) {
+        const int k = threadIdx.x, step = ctl->step;
+        double v = 0.0;
+        for (int i = 0; i < nw; ++i) v += red[i][k];
+        v = sqrt(v);
+        ctl->norms[k] = v;
+        hist[step % hist_cap * 4 + k] = v;
+        const int bad = __any_sync(0xfu, !isfinite(v));
+        if (k != 0) return;
         if (bad) ctl->nonfinite = 1;
-        ctl->step += 1;
+        ctl->step = step + 1;
         ctl->done_blocks = 0u;
         ctl->dt_bits = (unsigned long long)__double_as_longlong(DBL_MAX);
     }

@@ -780,7 +780,12 @@ __device__ __forceinline__ bool stage_fixed(const St& u, const St& u0, const Fix
 template <typename T, int STAGE, int NST, int DT>
 __global__ void __launch_bounds__(fvgb::kMaxBlock) k_update(const O2Args a) {
     using FT = typename std::conditional<std::is_same<T, double>::value, St, float4>::type;
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    // Stage 1's first block is not the update's (see below).
+    if (STAGE == 1 && blockIdx.x == 0) {
+        if (!a.r2) fold_partials((int)gridDim.x - 1, a.ctl, a.partials, a.hist, a.hist_cap);
+        return;
+    }
+    const int c = (blockIdx.x - (STAGE == 1)) * blockDim.x + threadIdx.x;
     double res[4] = {0.0, 0.0, 0.0, 0.0};
     if (c < a.m.n_cells && (!a.active || a.active[a.cell_inst[c]])) {
         const FT* ff = static_cast<const FT*>(a.ff);
@@ -881,9 +886,9 @@ __global__ void __launch_bounds__(fvgb::kMaxBlock) k_update(const O2Args a) {
     // Batched solves reduce per instance instead (k_batch_norms); a.r2 is
     // uniform over the grid, so the block-wide reduction is all-or-nothing.
     if (a.r2) return;
-    // With three stages the fold waits for the next update, whose first block
-    // does it beside the others' work (the grid is the same): stage 0 then
-    // has no fence, no counter and no last block that works alone.
+    // With three stages the fold waits for the next update, in which one more
+    // block does it beside the others' work: stage 0 then has no fence, no
+    // counter and no last block that works alone.
     if (STAGE == 0) {
         double ws;
         if (!fvfix::warp_squares4(res, ws))
@@ -891,7 +896,6 @@ __global__ void __launch_bounds__(fvgb::kMaxBlock) k_update(const O2Args a) {
         if (NST == 1) finish_norms(ws, a.ctl, a.partials, a.hist, a.hist_cap);
         else block_partial(ws, a.partials);
     }
-    if (STAGE == 1 && blockIdx.x == 0) fold_partials((int)gridDim.x, a.ctl, a.partials, a.hist, a.hist_cap);
 }
 
 // Residual only (multigrid restriction): the same signed gather as

@@ -39,7 +39,7 @@ void face(const O2Args& a, int dt, int bs, cudaStream_t s) {
 
 template <int ST, int NST>
 void update(const O2Args& a, int local, int bs, cudaStream_t s) {
-    const int cb = (a.m.n_cells + bs - 1) / bs;
+    const int cb = (a.m.n_cells + bs - 1) / bs + (ST == 1);  // stage 1: and one for the norms
     if (local) k_update<R, ST, NST, 2><<<cb, bs, 0, s>>>(a);
     else k_update<R, ST, NST, 1><<<cb, bs, 0, s>>>(a);
 }
