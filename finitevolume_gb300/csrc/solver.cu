@@ -109,9 +109,16 @@ void Solver::init(const HostMesh& hm, const fv_bc_t* bcs, int n_bcs, double g, d
     cfg.limiter = opt.limiter;
     cfg.stages = opt.rk_stages;
     cfg.local_dt = opt.dt_mode == FV_DT_LOCAL;
-    cfg.blk_grad = cfg.blk_face = cfg.blk_cell = 256;
     gamma = g;
     N = hm.n_cells;
+    // Small blocks spread a small mesh over more SMs and end a large one's last
+    // wave sooner; the update's also set the length of the norms' fold, which
+    // on large meshes outweighs that.  256 / 256 / 256 against 128 / 128 and the
+    // update's 128 or 256 (ms, Venkatakrishnan, HLLC): 2k cells, 20 steps 1.18,
+    // 1.10, -; 131k, 8 steps 1.35, 1.28, 1.30; 262k 2.30, 2.21, 2.23 (FP32, 20
+    // steps 1.16, 1.13, 1.11); 1.05M 7.58, 7.40, 7.36 (FP32 8.28, 8.33, 8.15).
+    cfg.blk_grad = cfg.blk_face = 128;
+    cfg.blk_cell = N <= 200000 ? 128 : 256;
     F = hm.n_faces;
     perm = hm.perm;
     wall_faces.clear();

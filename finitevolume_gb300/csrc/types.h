@@ -212,7 +212,7 @@ struct O2Config {
     int stages;    // 1 or 3
     int local_dt;  // 1 local, 0 global
     // launch shapes (threads per block, 128..512, multiple of 32), chosen by
-    // the autotuner; 256 by default
+    // the autotuner; Solver::init chooses the default
     int blk_grad, blk_face, blk_cell;
 };
 
