@@ -17,6 +17,7 @@
 // Included by kernels_fast.cu and kernels_strict.cu with FV_KNS defined.
 #pragma once
 
+#include "fixed.cuh"
 #include "physics.cuh"
 
 namespace FV_KNS {
@@ -51,6 +52,14 @@ __device__ __forceinline__ double warp_sum4(double v0, double v1, double v2, dou
 #pragma unroll
     for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
+}
+
+// The warp's sums of the squares of four values, placed the same: on the
+// integer pipe where the values allow it.
+__device__ __forceinline__ double warp_squares(const double (&x)[4]) {
+    double s;
+    if (fvfix::warp_squares4(x, s)) return s;
+    return warp_sum4(x[0] * x[0], x[1] * x[1], x[2] * x[2], x[3] * x[3]);
 }
 
 // Per-face wave-speed estimate max(|Vn|+c) of EulerFVMSolver::compute_dt

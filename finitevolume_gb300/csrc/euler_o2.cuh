@@ -890,9 +890,7 @@ __global__ void __launch_bounds__(fvgb::kMaxBlock) k_update(const O2Args a) {
     // block does it beside the others' work: stage 0 then has no fence, no
     // counter and no last block that works alone.
     if (STAGE == 0) {
-        double ws;
-        if (!fvfix::warp_squares4(res, ws))
-            ws = warp_sum4(res[0] * res[0], res[1] * res[1], res[2] * res[2], res[3] * res[3]);
+        const double ws = warp_squares(res);
         if (NST == 1) finish_norms(ws, a.ctl, a.partials, a.hist, a.hist_cap);
         else block_partial(ws, a.partials);
     }

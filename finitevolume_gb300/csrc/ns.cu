@@ -122,14 +122,14 @@ __global__ void __launch_bounds__(fvgb::kFaceBlock) k_ns_face(const NSArgs a) {
 // The Euler cell pass with the fluxes summed on the integer pipe.
 __global__ void __launch_bounds__(fvgb::kCellBlock) k_ns_cell(const O1Args a) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+    double res[4] = {0.0, 0.0, 0.0, 0.0};
     if (c < a.m.n_cells) {
         const double dt = __longlong_as_double((long long)a.ctl->dt_bits);
         const St R = gather_any(a.ff, a.m.cf, a.m.cf_off[c], a.m.cf_off[c + 1]);
-        s0 = R.r * R.r; s1 = R.ru * R.ru; s2 = R.rv * R.rv; s3 = R.E * R.E;
+        res[0] = R.r; res[1] = R.ru; res[2] = R.rv; res[3] = R.E;
         st_state(a.U, c, ld_state(a.U, c) + (dt * fvconv::rcp_nr3(a.m.vol[c])) * R);
     }
-    finish_norms(warp_sum4(s0, s1, s2, s3), a.ctl, a.partials, a.hist, a.hist_cap);
+    finish_norms(warp_squares(res), a.ctl, a.partials, a.hist, a.hist_cap);
 }
 #else
 __global__ void __launch_bounds__(fvgb::kCellBlock) k_ns_prim(const NSArgs a) {
@@ -276,14 +276,19 @@ __global__ void k_ns_wall(const NSArgs a, const int* __restrict__ faces, int n, 
 namespace fvgb {
 
 void FV_NS_FN(ns_launch_step)(const NSArgs& a, const O1Args& cell, cudaStream_t s) {
+#ifdef FV_NS_FAST
+    constexpr int bs = 128;  // shorter last waves than 256
+#else
+    constexpr int bs = kCellBlock;
+#endif
     const int cb = (a.g.n_cells + kCellBlock - 1) / kCellBlock;
-    const int fb = (a.g.n_faces + kFaceBlock - 1) / kFaceBlock;
-    FV_KNS::k_ns_prim<<<cb, kCellBlock, 0, s>>>(a);
-    FV_KNS::k_ns_grad<<<cb, kCellBlock, 0, s>>>(a);
+    const int gb = (a.g.n_cells + bs - 1) / bs, fb = (a.g.n_faces + bs - 1) / bs;
+    FV_KNS::k_ns_prim<<<gb, bs, 0, s>>>(a);
+    FV_KNS::k_ns_grad<<<gb, bs, 0, s>>>(a);
     switch (a.flux) {
-        case 1: FV_KNS::k_ns_face<1><<<fb, kFaceBlock, 0, s>>>(a); break;
-        case 2: FV_KNS::k_ns_face<2><<<fb, kFaceBlock, 0, s>>>(a); break;
-        default: FV_KNS::k_ns_face<0><<<fb, kFaceBlock, 0, s>>>(a); break;
+        case 1: FV_KNS::k_ns_face<1><<<fb, bs, 0, s>>>(a); break;
+        case 2: FV_KNS::k_ns_face<2><<<fb, bs, 0, s>>>(a); break;
+        default: FV_KNS::k_ns_face<0><<<fb, bs, 0, s>>>(a); break;
     }
 #ifdef FV_NS_FAST
     FV_KNS::k_ns_cell<<<cb, kCellBlock, 0, s>>>(cell);

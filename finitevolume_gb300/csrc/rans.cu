@@ -433,7 +433,7 @@ __global__ void __launch_bounds__(fvgb::kCellBlock) k_sa_cell(const RansArgs a) 
         const double vol = a.vol[c], nut = a.nut[c];
         const St u = ld_state(a.ns.U, c);
         Rn += vol * sa_source(a, nut, nut * (u.r * a.inv_mu), fabs(gv.x - gu.y), a.walld[c], gn.x, gn.y);
-        s[0] = R.r * R.r; s[1] = R.ru * R.ru; s[2] = R.rv * R.rv; s[3] = R.E * R.E; s[4] = Rn * Rn;
+        s[0] = R.r; s[1] = R.ru; s[2] = R.rv; s[3] = R.E; s[4] = Rn * Rn;
         const double k = __longlong_as_double((long long)ctl->dt_bits) * fvconv::rcp_nr3(vol);
         st_state(a.ns.U, c, u + k * R);
         a.nut[c] = nut + k * Rn;
@@ -464,7 +464,8 @@ __global__ void __launch_bounds__(fvgb::kCellBlock) k_sa_cell(const RansArgs a) 
     __shared__ bool last;
     const int w = threadIdx.x >> 5;
 #ifdef FV_NS_FAST
-    const double s4 = warp_sum4(s[0], s[1], s[2], s[3]);
+    const double res[4] = {s[0], s[1], s[2], s[3]};
+    const double s4 = warp_squares(res);
     s[4] = warp_sum(s[4]);
     const int lane = threadIdx.x & 31;
     if ((lane & 7) == 0) red[w][lane >> 3] = s4;
@@ -498,22 +499,22 @@ __global__ void __launch_bounds__(fvgb::kCellBlock) k_sa_cell(const RansArgs a) 
     if ((threadIdx.x & 31) == 0)
         for (int q = 0; q < 5; ++q) red[w][q] = t[q];
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double nrm[5];
-        int bad = 0;
-        for (int q = 0; q < 5; ++q) {
-            double v = 0.0;
-            for (int i = 0; i < fvgb::kCellBlock / 32; ++i) v += red[i][q];
-            nrm[q] = sqrt(v);
-            if (!isfinite(nrm[q])) bad = 1;
+    if (threadIdx.x < 5) {
+        const int q = threadIdx.x, step = ctl->step, row = step % a.hist_cap;
+        double v = 0.0;
+        for (int i = 0; i < fvgb::kCellBlock / 32; ++i) v += red[i][q];
+        v = sqrt(v);
+        if (q < 4) {
+            ctl->norms[q] = v;
+            a.hist[row * 4 + q] = v;
+        } else {
+            a.nut_hist[row] = v;
+            a.nut_norm[0] = v;
         }
-        for (int q = 0; q < 4; ++q) ctl->norms[q] = nrm[q];
-        const int row = ctl->step % a.hist_cap;
-        for (int q = 0; q < 4; ++q) a.hist[row * 4 + q] = nrm[q];
-        a.nut_hist[row] = nrm[4];
-        a.nut_norm[0] = nrm[4];
+        const int bad = __any_sync(0x1fu, !isfinite(v));
+        if (q != 0) return;
         if (bad) ctl->nonfinite = 1;
-        ctl->step += 1;
+        ctl->step = step + 1;
         ctl->done_blocks = 0u;
         ctl->dt_bits = (unsigned long long)__double_as_longlong(DBL_MAX);
     }
@@ -556,14 +557,19 @@ void rans_wall_distance(const RansArgs& a, const double4_32a* seg, int n_seg, cu
 #endif
 
 void FV_NS_FN(rans_launch_step)(const RansArgs& a, cudaStream_t s) {
+#ifdef FV_NS_FAST
+    constexpr int bs = 128;  // shorter last waves than 256
+#else
+    constexpr int bs = kCellBlock;
+#endif
     const int cb = (a.ns.g.n_cells + kCellBlock - 1) / kCellBlock;
-    const int fb = (a.ns.g.n_faces + kFaceBlock - 1) / kFaceBlock;
-    FV_KNS::k_sa_prim<<<cb, kCellBlock, 0, s>>>(a);
-    FV_KNS::k_sa_grad<<<cb, kCellBlock, 0, s>>>(a);
+    const int gb = (a.ns.g.n_cells + bs - 1) / bs, fb = (a.ns.g.n_faces + bs - 1) / bs;
+    FV_KNS::k_sa_prim<<<gb, bs, 0, s>>>(a);
+    FV_KNS::k_sa_grad<<<gb, bs, 0, s>>>(a);
     switch (a.ns.flux) {
-        case 1: FV_KNS::k_sa_face<1><<<fb, kFaceBlock, 0, s>>>(a); break;
-        case 2: FV_KNS::k_sa_face<2><<<fb, kFaceBlock, 0, s>>>(a); break;
-        default: FV_KNS::k_sa_face<0><<<fb, kFaceBlock, 0, s>>>(a); break;
+        case 1: FV_KNS::k_sa_face<1><<<fb, bs, 0, s>>>(a); break;
+        case 2: FV_KNS::k_sa_face<2><<<fb, bs, 0, s>>>(a); break;
+        default: FV_KNS::k_sa_face<0><<<fb, bs, 0, s>>>(a); break;
     }
     FV_KNS::k_sa_cell<<<cb, kCellBlock, 0, s>>>(a);
 }

@@ -158,7 +158,7 @@ __device__ __forceinline__ void min_candidate(double cand, fvgb::StepCtl* ctl) {
     __syncthreads();
     if (threadIdx.x == 0) {
         double v = smin[0];
-        for (int w = 1; w < fvgb::kFaceBlock / 32; ++w) v = fmin(v, smin[w]);
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) v = fmin(v, smin[w]);
         atomicMin(&ctl->dt_bits, (unsigned long long)__double_as_longlong(v));
     }
 }
