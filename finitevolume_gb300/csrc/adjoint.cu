@@ -706,13 +706,50 @@ __global__ void k_fwd_cell3(const AdjArgs a, St* __restrict__ dR) {
     st_state(dR, c, r);
 }
 
+// Norm of the stage-0 pseudo-time residual: the blocks' partials folded in a
+// fixed order by one block, the four norms appended to the history.
+struct AdjFold {
+    const double* partials;
+    int nblk;
+    double* hist;
+    int* counter;
+    int cap;
+};
+__device__ __forceinline__ void fold_norms(const AdjFold& q) {
+    __shared__ double red[8][4];
+    double t[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int b = threadIdx.x; b < q.nblk; b += blockDim.x) {
+        const double4_32a p = ld4(q.partials + 4 * (size_t)b);
+        t[0] += p.x; t[1] += p.y; t[2] += p.z; t[3] += p.w;
+    }
+    const double ws = warp_sum4(t[0], t[1], t[2], t[3]);
+    const int lane = threadIdx.x & 31;
+    if ((lane & 7) == 0) red[threadIdx.x >> 5][lane >> 3] = ws;
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        const int it = *q.counter;
+        double v = 0.0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v += red[w][threadIdx.x];
+        if (it < q.cap) q.hist[4 * it + threadIdx.x] = sqrt(v);
+        __syncwarp(0xfu);
+        if (threadIdx.x == 0) *q.counter = it + 1;
+    }
+}
+__global__ void __launch_bounds__(256) k_adj_norms(const AdjFold q) { fold_norms(q); }
+
 // ---------------------------------------------------------------------------
 // Cotangent map: Ubar = (dR/dU)^T lam, fsbar = (dR/dfs)^T lam.
 // Bound: the flux Jacobians (256 B a face) where they do not fit in L2, else
 // FP64 issue; they are read a row of four per 256-bit load (as scalars, 32
 // lanes each on a line of its own, the pass took 43 us at 250k faces).
-__global__ void k_bwd_face(const AdjArgs a, const St* __restrict__ lam) {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+// With fold.nblk its first block folds the previous stage's norms instead,
+// beside the others (as a launch of its own 7.5 us an iteration).
+__global__ void __launch_bounds__(256) k_bwd_face(const AdjArgs a, const St* __restrict__ lam, const AdjFold fold) {
+    if (fold.nblk && blockIdx.x == 0) {
+        fold_norms(fold);
+        return;
+    }
+    const int f = (blockIdx.x - (fold.nblk != 0)) * blockDim.x + threadIdx.x;
     if (f >= a.n_faces) return;
     const int L = a.fl[f], R = a.fr[f];
     // R_L -= F_f, R_R += F_f
@@ -740,7 +777,7 @@ __global__ void k_bwd_face(const AdjArgs a, const St* __restrict__ lam) {
 // order 1: finishes Ubar here (MODE 0: write Ubar; 1..3: RK stage 0..2).
 __device__ __forceinline__ void finish_cell(const AdjArgs& a, int c, const double wbar[4], int mode,
                                             St* __restrict__ out, St* __restrict__ lam, St* __restrict__ lam0,
-                                            const St* __restrict__ rhs, double* __restrict__ r2) {
+                                            const St* __restrict__ rhs, double* __restrict__ res) {
     // (dW/dU)^T wbar (prim_jac), with one reciprocal
     const V4<double> w = ldW(a.W, c);
     const double ir = fvconv::rcp_nr3(w.r), m1 = wbar[1] * ir, m2 = wbar[2] * ir, g3 = (a.gamma - 1.0) * wbar[3];
@@ -761,7 +798,7 @@ __device__ __forceinline__ void finish_cell(const AdjArgs& a, int c, const doubl
         st_state(lam0, c, l);
         n = e;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) r2[k] = r[k] * r[k];
+        for (int k = 0; k < 4; ++k) res[k] = r[k];
     } else if (mode == 2) {
         n = 0.75 * ld_state(lam0, c) + 0.25 * e;
     } else {
@@ -770,25 +807,11 @@ __device__ __forceinline__ void finish_cell(const AdjArgs& a, int c, const doubl
     st_state(lam, c, n);
 }
 
-__device__ __forceinline__ void block_partials(double r2[4], double* partials) {
-    __shared__ double red[8][4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) r2[k] = warp_sum(r2[k]);
-    if ((threadIdx.x & 31) == 0)
-        for (int k = 0; k < 4; ++k) red[threadIdx.x >> 5][k] = r2[k];
-    __syncthreads();
-    if (threadIdx.x == 0)
-        for (int k = 0; k < 4; ++k) {
-            double v = 0.0;
-            for (int w = 0; w < 8; ++w) v += red[w][k];
-            partials[4 * blockIdx.x + k] = v;
-        }
-}
 
 __global__ void __launch_bounds__(256) k_bwd_cell1(const AdjArgs a, int mode, St* out, St* lam, St* lam0,
                                                    const St* rhs, double* partials) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    double r2[4] = {0.0, 0.0, 0.0, 0.0};
+    double res[4] = {0.0, 0.0, 0.0, 0.0};
     if (c < a.n_cells) {
         double wb[4] = {0.0, 0.0, 0.0, 0.0}, gx[4] = {0.0, 0.0, 0.0, 0.0}, gy[4] = {0.0, 0.0, 0.0, 0.0};
         for (int e = a.cf_off[c]; e < a.cf_off[c + 1]; ++e) {
@@ -854,17 +877,17 @@ __global__ void __launch_bounds__(256) k_bwd_cell1(const AdjArgs a, int mode, St
             st4(gub, gux[0], guy[0], gux[1], guy[1]);
             st4(gub + 4, gux[2], guy[2], gux[3], guy[3]);
         } else {
-            finish_cell(a, c, wb, mode, out, lam, lam0, rhs, r2);
+            finish_cell(a, c, wb, mode, out, lam, lam0, rhs, res);
         }
     }
-    if (a.order == 1 && mode == 1) block_partials(r2, partials);
+    if (a.order == 1 && mode == 1) block_partial(warp_squares(res), partials);
 }
 
 // Gradient cotangent to W-bar (gather through twin entries), then Ubar.
 __global__ void __launch_bounds__(256) k_bwd_cell2(const AdjArgs a, int mode, St* out, St* lam, St* lam0,
                                                    const St* rhs, double* partials) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    double r2[4] = {0.0, 0.0, 0.0, 0.0};
+    double res[4] = {0.0, 0.0, 0.0, 0.0};
     if (c < a.n_cells) {
         const St w0 = ld_state(a.Wbar, c);
         double wb[4] = {w0.r, w0.ru, w0.rv, w0.E};
@@ -903,32 +926,9 @@ __global__ void __launch_bounds__(256) k_bwd_cell2(const AdjArgs a, int mode, St
                 }
             }
         }
-        finish_cell(a, c, wb, mode, out, lam, lam0, rhs, r2);
+        finish_cell(a, c, wb, mode, out, lam, lam0, rhs, res);
     }
-    if (mode == 1) block_partials(r2, partials);
-}
-
-// Norm of the stage-0 pseudo-time residual: block partials folded in block
-// order by one block (deterministic); appended to the history.
-__global__ void __launch_bounds__(256) k_adj_norms(const double* partials, int nblk, double* hist, int* counter,
-                                                   int cap) {
-    __shared__ double red[256][4];
-    double t[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int b = threadIdx.x; b < nblk; b += 256)
-        for (int k = 0; k < 4; ++k) t[k] += partials[4 * b + k];
-    for (int k = 0; k < 4; ++k) red[threadIdx.x][k] = t[k];
-    __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-        if (threadIdx.x < w)
-            for (int k = 0; k < 4; ++k) red[threadIdx.x][k] += red[threadIdx.x + w][k];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        const int it = *counter;
-        if (it < cap)
-            for (int k = 0; k < 4; ++k) hist[4 * it + k] = sqrt(red[0][k]);
-        *counter = it + 1;
-    }
+    if (mode == 1) block_partial(warp_squares(res), partials);
 }
 
 // ---------------------------------------------------------------------------
@@ -1215,7 +1215,7 @@ const HostMesh& host_mesh_of(const fv_mesh_s* m);
 
 namespace {
 
-constexpr int kB = 256;
+constexpr int kB = 128;
 inline int blocks(int n) { return (n + kB - 1) / kB; }
 
 void check_launch() { FV_CUDA(cudaGetLastError()); }
@@ -1293,19 +1293,21 @@ void linearise(fv_adjoint_s* A) {
     A->linearised = true;
 }
 
+adjk::AdjFold norm_fold(fv_adjoint_s* A) { return {A->partials, blocks(A->N), A->hist, A->counter, A->hist_cap}; }
+
+// Stage 1 (mode 1) leaves its norms' partials; stage 2, which follows it in
+// every iteration, folds them.
 void backward(fv_adjoint_s* A, const St* lam, int mode, St* out) {
     fvgb::Solver& s = A->solver->s;
     AdjArgs& a = A->a;
-    adjk::k_bwd_face<<<blocks(A->F), kB, 0, s.stream>>>(a, lam);
+    adjk::AdjFold fold = norm_fold(A);
+    if (mode != 2) fold.nblk = 0;
+    adjk::k_bwd_face<<<blocks(A->F) + (mode == 2), kB, 0, s.stream>>>(a, lam, fold);
     check_launch();
     adjk::k_bwd_cell1<<<blocks(A->N), kB, 0, s.stream>>>(a, mode, out, A->lam, A->lam0, A->rhs, A->partials);
     check_launch();
     if (a.order == 2) {
         adjk::k_bwd_cell2<<<blocks(A->N), kB, 0, s.stream>>>(a, mode, out, A->lam, A->lam0, A->rhs, A->partials);
-        check_launch();
-    }
-    if (mode == 1) {
-        adjk::k_adj_norms<<<1, 256, 0, s.stream>>>(A->partials, blocks(A->N), A->hist, A->counter, A->hist_cap);
         check_launch();
     }
 }
@@ -1910,6 +1912,8 @@ int fv_adjoint_solve_gmres(fv_adjoint_t A, const double* dJdU, int32_t restart, 
         FV_CUDA(cudaMemcpyAsync(lam, A->kx, sizeof(double) * n, cudaMemcpyDeviceToDevice, s.stream));
         FV_CUDA(cudaMemsetAsync(A->counter, 0, sizeof(int), s.stream));
         backward(A, A->lam, 1, nullptr);
+        adjk::k_adj_norms<<<1, 256, 0, A->solver->s.stream>>>(norm_fold(A));
+        check_launch();
         double r4[4];
         FV_CUDA(cudaMemcpyAsync(r4, A->hist, sizeof(double) * 4, cudaMemcpyDeviceToHost, s.stream));
         FV_CUDA(cudaMemcpyAsync(lam, A->kx, sizeof(double) * n, cudaMemcpyDeviceToDevice, s.stream));
