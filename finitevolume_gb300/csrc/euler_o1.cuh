@@ -62,6 +62,16 @@ __device__ __forceinline__ double warp_squares(const double (&x)[4]) {
     return warp_sum4(x[0] * x[0], x[1] * x[1], x[2] * x[2], x[3] * x[3]);
 }
 
+// The warp's residual sums for the norms (strict: the squares' FP64 sums).
+__device__ __forceinline__ double warp_norms(const St& R) {
+#ifdef FV_STRICT_ORDER
+    return warp_sum4(R.r * R.r, R.ru * R.ru, R.rv * R.rv, R.E * R.E);
+#else
+    const double x[4] = {R.r, R.ru, R.rv, R.E};
+    return warp_squares(x);
+#endif
+}
+
 // Per-face wave-speed estimate max(|Vn|+c) of EulerFVMSolver::compute_dt
 // (src/EulerFVMSolver.cpp:140-150).
 __device__ __forceinline__ double face_smax(const St& UL, const St& UR, bool interior, double nx, double ny,
@@ -172,7 +182,7 @@ __device__ __forceinline__ void finish_norms(double ws, StepCtl* ctl, double* pa
 template <bool LOCAL>
 __global__ void __launch_bounds__(fvgb::kCellBlock) k_cell_o1(const O1Args a) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+    St res = st_make(0.0, 0.0, 0.0, 0.0);
     if (c < a.m.n_cells) {
         double dt = LOCAL ? 0.0 : __longlong_as_double((long long)a.ctl->dt_bits);
         St R = st_make(0.0, 0.0, 0.0, 0.0);
@@ -184,11 +194,11 @@ __global__ void __launch_bounds__(fvgb::kCellBlock) k_cell_o1(const O1Args a) {
             if (LOCAL) dt += a.dtf[f];
         }
         if (LOCAL) dt = a.ctl->cfl * a.m.vol[c] / dt;
-        s0 = R.r * R.r; s1 = R.ru * R.ru; s2 = R.rv * R.rv; s3 = R.E * R.E;
+        res = R;
         const St u = ld_state(a.U, c);
         st_state(a.U, c, u + (dt / a.m.vol[c]) * R);
     }
-    finish_norms(warp_sum4(s0, s1, s2, s3), a.ctl, a.partials, a.hist, a.hist_cap);
+    finish_norms(warp_norms(res), a.ctl, a.partials, a.hist, a.hist_cap);
 }
 
 template <int FLUX>

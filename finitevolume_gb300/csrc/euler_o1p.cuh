@@ -10,13 +10,13 @@
 // barrier:
 //
 //   prologue   per-cell primitives P = (u, v, p, c) of the current state
-//   per step   face phase: fluxes (and the CFL candidate or lambda*A),
-//                 block 0 also folds the previous step's norm partials
+//   per step   face phase: fluxes (and the CFL candidate or lambda*A); every
+//                 kNormRing steps their norm partials are folded
 //              barrier
 //              cell phase: signed gather, U += dt/V R, the new P, and one
 //                 norm partial per 256-cell tile
 //              barrier
-//   epilogue   block 0 folds the last step's partials
+//   epilogue   the last steps' partials are folded
 //
 // P is the reference's own per-side quantities (u = rho_u/rho, v, the
 // pressure and sound speed expressions of EulerState.h:58-82), formed once
@@ -295,11 +295,11 @@ __device__ __forceinline__ double face_phase_face(const O1Args& a, const double4
 }
 
 #ifndef FV_STRICT_ORDER
-// The signed sum of a cell's N face fluxes and, with LOCAL, the sum of its
-// faces' lambda * length, on the integer pipe (fvfix::signed_sum).
+// The signed sum of a cell's N face fluxes and, with LOCAL, the step factor
+// cfl over the sum of its faces' lambda * length, on the integer pipe.
 // face(i, lam): the flux and lambda * length of the cell's i-th face.
 template <int N, bool LOCAL, class Face>
-__device__ __forceinline__ St gather_cell(const int* cf, const Face& face, double& lam) {
+__device__ __forceinline__ St gather_cell(const int* cf, const Face& face, double cfl, double& coef) {
     double x[4][N], l[N];
     int neg[N], none[N];
 #pragma unroll
@@ -309,41 +309,46 @@ __device__ __forceinline__ St gather_cell(const int* cf, const Face& face, doubl
         neg[i] = cf[i];
         none[i] = 0;
     }
-    if (LOCAL) lam = fvfix::signed_sum<N>(l, none);
+    fvfix::Fixed lam;
+    if (LOCAL && !(fvfix::fixed_sum<N>(l, none, lam) && fvfix::quotient(cfl, lam, coef)))
+        coef = cfl * fvconv::rcp_nr3(fvfix::signed_sum<N>(l, none));
     return st_make(fvfix::signed_sum<N>(x[0], neg), fvfix::signed_sum<N>(x[1], neg), fvfix::signed_sum<N>(x[2], neg),
                    fvfix::signed_sum<N>(x[3], neg));
 }
 #endif
 
-// One cell of the cell phase: the signed gather of its face fluxes, U + dt/V R
-// (returned) from its state u, the new primitives q, and the squares of R for
-// the norms.
+// One cell of the cell phase: the signed gather R of its face fluxes, U + dt/V R
+// (returned) from its state u, and the new primitives q.
 template <bool LOCAL, class Face>
 __device__ __forceinline__ St cell_compute(const O1Args& a, int c, const Face& face, const St& u, double g, double cfl,
-                                           double dt_g, Prim& q, double& s0, double& s1, double& s2, double& s3) {
+                                           double dt_g, Prim& q, St& Rs) {
     double dt = dt_g;
-    St Rs = st_make(0.0, 0.0, 0.0, 0.0);
+    Rs = st_make(0.0, 0.0, 0.0, 0.0);
     const int e0 = a.m.cf_off[c], n = a.m.cf_off[c + 1] - e0;
     const int* cf = a.m.cf + e0;
-    double lam = 0.0;
-#ifndef FV_STRICT_ORDER
-    if (n == 4) Rs = gather_cell<4, LOCAL>(cf, face, lam);
-    else if (n == 3) Rs = gather_cell<3, LOCAL>(cf, face, lam);
-    else
-#endif
-    for (int i = 0; i < n; ++i) {
-        double l;
-        Rs += flip_if(face(i, l), cf[i]);
-        if (LOCAL) lam += l;
-    }
-    double coef;  // dt / V
+    double lam = 0.0, coef = 0.0;  // coef: dt / V
+    auto any = [&]() {
+        for (int i = 0; i < n; ++i) {
+            double l;
+            Rs += flip_if(face(i, l), cf[i]);
+            if (LOCAL) lam += l;
+        }
+    };
 #ifdef FV_STRICT_ORDER
+    any();
     if (LOCAL) dt = cfl * a.m.vol[c] / lam;
     coef = dt / a.m.vol[c];
 #else
-    coef = LOCAL ? cfl * fvconv::rcp_nr3(lam) : dt * fvconv::rcp_nr3(a.m.vol[c]);
+    if (n == 4) {
+        Rs = gather_cell<4, LOCAL>(cf, face, cfl, coef);
+    } else if (n == 3) {
+        Rs = gather_cell<3, LOCAL>(cf, face, cfl, coef);
+    } else {
+        any();
+        if (LOCAL) coef = cfl * fvconv::rcp_nr3(lam);
+    }
+    if (!LOCAL) coef = dt * fvconv::rcp_nr3(a.m.vol[c]);
 #endif
-    s0 = Rs.r * Rs.r; s1 = Rs.ru * Rs.ru; s2 = Rs.rv * Rs.rv; s3 = Rs.E * Rs.E;
     const St un = u + coef * Rs;
     q = prim_of(un, g);
     return un;
@@ -351,7 +356,7 @@ __device__ __forceinline__ St cell_compute(const O1Args& a, int c, const Face& f
 
 template <bool LOCAL>
 __device__ __forceinline__ void cell_phase_cell(const O1Args& a, double4_32a* P, int c, double g, double cfl,
-                                                double dt_g, double& s0, double& s1, double& s2, double& s3) {
+                                                double dt_g, St& R) {
     const int* cf = a.m.cf + a.m.cf_off[c];
     Prim q;
     const St un = cell_compute<LOCAL>(
@@ -361,7 +366,7 @@ __device__ __forceinline__ void cell_phase_cell(const O1Args& a, double4_32a* P,
             if (LOCAL) l = __ldcg(a.dtf + f);
             return ld_state_cg(a.ff, f);
         },
-        ld_state_cg(a.U, c), g, cfl, dt_g, q, s0, s1, s2, s3);
+        ld_state_cg(a.U, c), g, cfl, dt_g, q, R);
     st_state(a.U, c, un);
     st_prim(P, c, q);
 }
@@ -400,11 +405,11 @@ __device__ __forceinline__ bool grid_barrier(PersistCtl* pc, unsigned int expect
     return ok != 0;
 }
 
-// Block 0 folds one step's tile partials exactly as finish_norms' last
+// One block folds one step's tile partials exactly as finish_norms' last
 // block does (tiles strided over the block's threads, transposed warp sums,
-// warps in order), records the history row and advances the step counter.
-__device__ __forceinline__ void fold_step_norms(StepCtl* ctl, const double* partials, int n_tiles, double* hist,
-                                                int hist_cap) {
+// warps in order) and records the history row, and with `last` the norms.
+__device__ __forceinline__ void fold_step_norms(StepCtl* ctl, const double* partials, int n_tiles, double* row,
+                                                bool last) {
     __shared__ double red[fvgb::kCellBlock / 32][4];
     constexpr int nw = fvgb::kCellBlock / 32;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -417,20 +422,13 @@ __device__ __forceinline__ void fold_step_norms(StepCtl* ctl, const double* part
     __syncthreads();
     if ((lane & 7) == 0) red[w][lane >> 3] = ts;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double n[4];
-        int bad = 0;
-        for (int k = 0; k < 4; ++k) {
-            double v = 0.0;
-            for (int i = 0; i < nw; ++i) v += red[i][k];
-            n[k] = sqrt(v);
-            if (!isfinite(n[k])) bad = 1;
-            ctl->norms[k] = n[k];
-        }
-        const int row = ctl->step % hist_cap;
-        for (int k = 0; k < 4; ++k) hist[row * 4 + k] = n[k];
-        if (bad) ctl->nonfinite = 1;
-        ctl->step += 1;
+    if (threadIdx.x < 4) {
+        double v = 0.0;
+        for (int i = 0; i < nw; ++i) v += red[i][threadIdx.x];
+        v = sqrt(v);
+        row[threadIdx.x] = v;
+        if (last) ctl->norms[threadIdx.x] = v;
+        if (!isfinite(v)) ctl->nonfinite = 1;
     }
     __syncthreads();
 }
@@ -444,6 +442,13 @@ __global__ void __launch_bounds__(fvgb::kCellBlock) k_o1_persistent(const O1Args
     const int n_tiles = (a.m.n_cells + fvgb::kCellBlock - 1) / fvgb::kCellBlock;
     const int F = a.m.n_faces, N = a.m.n_cells;
 
+    const int step0 = a.ctl->step;
+    auto fold_ring = [&](int from, int to) {
+        for (int j = from + blockIdx.x; j < to; j += nb)
+            fold_step_norms(a.ctl, a.partials + (size_t)(j % fvgb::kNormRing) * n_tiles * 4, n_tiles,
+                            a.hist + (size_t)((step0 + j) % a.hist_cap) * 4, j == nsteps - 1);
+    };
+
     // prologue: primitives of the current state; both dt slots armed
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < N; c += nb * blockDim.x)
         st_prim(P, c, prim_of(ld_state_cg(a.U, c), g));
@@ -453,10 +458,11 @@ __global__ void __launch_bounds__(fvgb::kCellBlock) k_o1_persistent(const O1Args
 
     for (int s = 0; s < nsteps; ++s) {
         const int slot = s & 1;
-        if (blockIdx.x == 0 && s > 0) {
-            fold_step_norms(a.ctl, a.partials, n_tiles, a.hist, a.hist_cap);
-            if (threadIdx.x == 0) pc->dt_slot[slot ^ 1] = (unsigned long long)__double_as_longlong(DBL_MAX);
-        }
+        if (blockIdx.x == 0 && s > 0 && threadIdx.x == 0)
+            pc->dt_slot[slot ^ 1] = (unsigned long long)__double_as_longlong(DBL_MAX);
+        // Norms: the partials of kNormRing steps, then a block for each step (a
+        // fold takes one block 4 to 5 us, for which all others wait).
+        if (s > 0 && s % fvgb::kNormRing == 0) fold_ring(s - fvgb::kNormRing, s);
         // face phase
         const double cfl = a.ctl->cfl;
         double cand = DBL_MAX;
@@ -482,24 +488,25 @@ __global__ void __launch_bounds__(fvgb::kCellBlock) k_o1_persistent(const O1Args
         const double dt_g = LOCAL ? 0.0 : __longlong_as_double((long long)*(volatile unsigned long long*)&pc->dt_slot[slot]);
         for (int tile = blockIdx.x; tile < n_tiles; tile += nb) {
             const int c = tile * fvgb::kCellBlock + threadIdx.x;
-            double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-            if (c < N) cell_phase_cell<LOCAL>(a, P, c, g, cfl, dt_g, s0, s1, s2, s3);
+            St R = st_make(0.0, 0.0, 0.0, 0.0);
+            if (c < N) cell_phase_cell<LOCAL>(a, P, c, g, cfl, dt_g, R);
             // the tile's partial: finish_norms' block reduction
             __shared__ double red[fvgb::kCellBlock / 32][4];
             const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-            const double ws = warp_sum4(s0, s1, s2, s3);
+            const double ws = warp_norms(R);
             if ((lane & 7) == 0) red[w][lane >> 3] = ws;
             __syncthreads();
             if (threadIdx.x < 4) {
                 double v = 0.0;
                 for (int i = 0; i < fvgb::kCellBlock / 32; ++i) v += red[i][threadIdx.x];
-                a.partials[tile * 4 + threadIdx.x] = v;
+                a.partials[((size_t)(s % fvgb::kNormRing) * n_tiles + tile) * 4 + threadIdx.x] = v;
             }
             __syncthreads();
         }
         if (!grid_barrier(pc, expected)) return;
     }
-    if (blockIdx.x == 0 && nsteps > 0) fold_step_norms(a.ctl, a.partials, n_tiles, a.hist, a.hist_cap);
+    fold_ring((nsteps - 1) / fvgb::kNormRing * fvgb::kNormRing, nsteps);
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.ctl->step = step0 + nsteps;
 }
 
 // ---------------------------------------------------------------------------
@@ -667,9 +674,9 @@ __global__ void __launch_bounds__(fvgb::kDfBlock, 1) k_o1_dataflow(const O1Args 
         double* wp = d.wpart + (size_t)s * d.n_warps * 4;
         for (int cw = c0 / 32 + warp; cw * 32 < c1; cw += nwarps) {
             const int c = cw * 32 + lane;
-            double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-            if (c < N) cell_phase_cell<true>(a, P, c, g, cfl, 0.0, s0, s1, s2, s3);
-            const double ws = warp_sum4(s0, s1, s2, s3);
+            St R = st_make(0.0, 0.0, 0.0, 0.0);
+            if (c < N) cell_phase_cell<true>(a, P, c, g, cfl, 0.0, R);
+            const double ws = warp_norms(R);
             if ((lane & 7) == 0) wp[(size_t)cw * 4 + (lane >> 3)] = ws;
         }
         df_publish(d.prog, 2u * s + 2u);
@@ -768,7 +775,7 @@ __global__ void __launch_bounds__(fvgb::kDfBlock, 1) k_o1_dataflow_sm(const O1Ar
     const int nf_in = d.face_in[b];    // faces that need no other block's cell, first
     double2* sU = sm;                  // own states
     double2* sP = sU + 2 * nc;         // their primitives
-    double2* sN = sP + 2 * nc;         // squared residuals
+    double2* sN = sP + 2 * nc;         // residuals
     double2* sF = sN + 2 * nc;         // fluxes of the own cells' faces
     double* sL = reinterpret_cast<double*>(sF + 2 * nf);  // their lambda * length
     const int step0 = a.ctl->step;
@@ -843,7 +850,7 @@ __global__ void __launch_bounds__(fvgb::kDfBlock, 1) k_o1_dataflow_sm(const O1Ar
         for (int i = threadIdx.x; i < nc; i += fvgb::kDfBlock) {
             const int c = c0 + i, e0 = a.m.cf_off[c];
             Prim q;
-            double s0, s1, s2, s3;
+            St R;
             const St un = cell_compute<true>(
                 a, c,
                 [&](int m, double& l) {
@@ -851,13 +858,13 @@ __global__ void __launch_bounds__(fvgb::kDfBlock, 1) k_o1_dataflow_sm(const O1Ar
                     l = sL[k];
                     return ld_shared(sF, k);
                 },
-                ld_shared(sU, i), g, cfl, 0.0, q, s0, s1, s2, s3);
+                ld_shared(sU, i), g, cfl, 0.0, q, R);
             const int m = d.mail_of[c];
             if (last) st_state(a.U, c, un);
             else if (m >= 0) mail_put(d.mail + 16 * (size_t)m + 8 * ((s + 1) & 1), un, q, s + 2ull);
             st_shared(sU, i, un.r, un.ru, un.rv, un.E);
             st_shared(sP, i, q.u, q.v, q.p, q.c);
-            st_shared(sN, i, s0, s1, s2, s3);
+            st_shared(sN, i, R.r, R.ru, R.rv, R.E);
         }
         __syncthreads();
 
@@ -868,7 +875,7 @@ __global__ void __launch_bounds__(fvgb::kDfBlock, 1) k_o1_dataflow_sm(const O1Ar
         for (int cw = nwarps - 1 - warp; cw * 32 < nc; cw += nwarps) {
             St n = st_make(0.0, 0.0, 0.0, 0.0);
             if (cw * 32 + lane < nc) n = ld_shared(sN, cw * 32 + lane);
-            const double ws = warp_sum4(n.r, n.ru, n.rv, n.E);
+            const double ws = warp_norms(n);
             if ((lane & 7) == 0) wp[(size_t)(c0 / 32 + cw) * 4 + (lane >> 3)] = ws;
         }
     }

@@ -170,8 +170,10 @@ void Solver::init(const HostMesh& hm, const fv_bc_t* bcs, int n_bcs, double g, d
     if (!(general && cfg.fp32)) ff = dalloc<St>(F, owned);
     dtf = dalloc<double>(F, owned);
     n_cell_blocks = (N + kCellBlock - 1) / kCellBlock;
-    // sized for the smallest tunable cell block
-    partials = dalloc<double>(4 * (size_t)((N + kMinBlock - 1) / kMinBlock), owned);
+    // sized for the smallest tunable cell block, or the persistent kernel's steps
+    partials = dalloc<double>(4 * std::max<size_t>((N + kMinBlock - 1) / kMinBlock,
+                                                   general || viscous ? 0 : (size_t)kNormRing * n_cell_blocks),
+                              owned);
     ctl = dalloc<StepCtl>(1, owned);
     StepCtl c0;
     std::memset(&c0, 0, sizeof(c0));

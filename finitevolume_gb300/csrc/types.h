@@ -231,6 +231,7 @@ constexpr int kNormChunk = 1024;
 
 constexpr int kCellBlock = 256;
 constexpr int kFaceBlock = 256;
+constexpr int kNormRing = 8;    // steps of the persistent first-order kernel whose norm partials are kept
 constexpr int kMaxBlock = 512;  // largest tunable block of the second-order kernels
 constexpr int kMinBlock = 128;  // smallest (sizes the norm partials)
 
