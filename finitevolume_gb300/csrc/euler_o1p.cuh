@@ -180,16 +180,14 @@ __device__ __forceinline__ double face_smax_p(const Prim& PL, const Prim& PR, bo
 // ghost's primitives too: its sound speed is |cb| (p_b = rho_b cb^2 / g),
 // and the boundary density rho_s (cb^2 / (g s))^(1/(g-1)) with the upwind
 // side's entropy s = p_s / rho_s^g is rho_s |cb / c_s|^(2/(g-1)), taken by
-// pow_near1.  This is the longest dependent chain of the face phase and a
+// pow_near1; the freestream's primitives are prepared (O1Args::fsp).  This is the longest dependent chain of the face phase and a
 // few blocks own all the farfield faces, so no division, square root or
 // library power depends on the interior state here.
-__device__ __forceinline__ void char_farfield_p(const St& UL, const Prim& PL, const double* sinf, double nx,
-                                                double ny, double g, St& UR, Prim& PR) {
-    const double rf = sinf[0], irf = fvconv::rcp_nr3(rf), uf = sinf[1] * irf, vf = sinf[2] * irf;
-    const double pf = (g - 1.0) * (sinf[3] - 0.5 * rf * (uf * uf + vf * vf));
-    const double cf = sqrt(g * pf * irf);
+__device__ __forceinline__ void char_farfield_p(const St& UL, const Prim& PL, const double* sinf, const double* fsp,
+                                                double nx, double ny, double g, St& UR, Prim& PR) {
+    const double rf = fsp[0], uf = fsp[1], vf = fsp[2], pf = fsp[3], cf = fsp[4], icf = fsp[5];
     const double vni = PL.u * nx + PL.v * ny, vnf = uf * nx + vf * ny;
-    const double ici = fvconv::rcp_nr3(PL.c), icf = fvconv::rcp_nr3(cf);  // off the chain
+    const double ici = fvconv::rcp_nr3(PL.c);  // off the chain
     if (vnf <= -cf) {  // supersonic inflow
         UR = st_make(sinf[0], sinf[1], sinf[2], sinf[3]);
         PR.u = uf; PR.v = vf; PR.p = pf; PR.c = cf;
@@ -210,7 +208,7 @@ __device__ __forceinline__ void char_farfield_p(const St& UL, const Prim& PL, co
     const double vt = out ? PL.v - vni * ny : vf - vnf * ny;
     const double rb = rs * fvconv::pow_near1(fabs(cb) * ics, k);
     const double ub = ut + vnb * nx, vb = vt + vnb * ny;
-    const double pb = rb * cb * cb * (1.0 / g);
+    const double pb = rb * cb * cb * fsp[6];
     UR = st_make(rb, rb * ub, rb * vb, pb * (1.0 / (g - 1.0)) + 0.5 * rb * (ub * ub + vb * vb));
     PR.u = ub; PR.v = vb; PR.p = pb; PR.c = fabs(cb);
 }
@@ -221,11 +219,11 @@ __device__ __forceinline__ void char_farfield_p(const St& UL, const Prim& PL, co
 // normal velocity reversed); outflow the interior itself; the fixed
 // farfield and the no-slip wall through ghost_state.  Same states as
 // ghost_state + prim_of up to rounding, with short dependent chains.
-__device__ __forceinline__ void ghost_p(const BCTable& bc, int patch, const St& UL, const Prim& PL, double nx,
-                                        double ny, double g, St& UR, Prim& PR) {
+__device__ __forceinline__ void ghost_p(const BCTable& bc, const double* fsp, int patch, const St& UL, const Prim& PL,
+                                        double nx, double ny, double g, St& UR, Prim& PR) {
     const int t = bc.type[patch];
     if (t == BC_CHAR) {
-        char_farfield_p(UL, PL, bc.st[patch], nx, ny, g, UR, PR);
+        char_farfield_p(UL, PL, bc.st[patch], fsp + 8 * patch, nx, ny, g, UR, PR);
     } else if (t == BC_WALL) {
         const double Vn = PL.u * nx + PL.v * ny;
         PR.u = PL.u - 2.0 * Vn * nx;
@@ -252,7 +250,7 @@ __device__ __forceinline__ St face_compute(const O1Args& a, int f, bool interior
                                            const Prim& PL, St UR, Prim PR, double g, double cfl, double& dt) {
     if (!interior) {
 #ifndef FV_STRICT_ORDER
-        ghost_p(a.bc, a.m.fpatch[f], UL, PL, geo.x, geo.y, g, UR, PR);
+        ghost_p(a.bc, a.fsp, a.m.fpatch[f], UL, PL, geo.x, geo.y, g, UR, PR);
 #else
         UR = ghost_state(a.bc, a.m.fpatch[f], UL, geo.x, geo.y, g);
         PR = prim_of(UR, g);

@@ -132,6 +132,20 @@ __device__ __forceinline__ double pow_near1(double x, double k) {
     const double xm = x - 1.0;
     const double axm = fabs(xm);
     if (!(axm <= 0.125)) return pow(x, k);
+    // k within 4e-15 of a whole number n up to 8 (2 / (gamma - 1) = 5 for
+    // gamma = 1.4): x^n by squarings, five roundings at most, times
+    // x^(k - n) = 1 + (k - n) (x - 1) (what is left out is below 2^-54).
+    const int n = __double2int_rn(k);
+    const double r = k - n;
+    if (n >= 1 && n <= 8 && fabs(r) <= 4e-15) {
+        const double x2 = x * x, x4 = x2 * x2;
+        double p = fma(r, xm, 1.0);
+        if (n & 1) p *= x;
+        if (n & 2) p *= x2;
+        if (n & 4) p *= x4;
+        if (n & 8) p *= x4 * x4;
+        return p;
+    }
     const double z = xm * rcp_nr3(x + 1.0);
     const double z2 = z * z;
     if (axm <= 1.0 / 64.0) {

@@ -210,6 +210,20 @@ void Solver::init(const HostMesh& hm, const fv_bc_t* bcs, int n_bcs, double g, d
         }
     }
 
+    // Farfield primitives, per patch or per instance of a batch (O2Args::fsp)
+    auto upload_farfield = [&]() {
+        const double* st = batch ? batch_freestream : &bc.st[0][0];
+        std::vector<double> q;
+        for (int i = 0; i < (batch ? n_inst : kMaxPatches); ++i, st += 4) {
+            const bool has = st[0] != 0.0;  // patches without a farfield state stay zero
+            const double r = st[0], u = has ? st[1] / r : 0.0, v = has ? st[2] / r : 0.0;
+            const double p = (gamma - 1.0) * (st[3] - 0.5 * r * (u * u + v * v));
+            const double c = has ? std::sqrt(gamma * p / r) : 0.0;
+            for (double x : {r, u, v, p, c, has ? 1.0 / c : 0.0, 1.0 / gamma, 0.0}) q.push_back(x);
+        }
+        fsp = dupload(q, owned);
+    };
+    if (!general && !viscous && !opt.strict) upload_farfield();
     if (general) {
         HostMesh h2 = hm;  // the per-entry geometry is derived on a copy
         h2.build_o2_geometry();
@@ -261,18 +275,7 @@ void Solver::init(const HostMesh& hm, const fv_bc_t* bcs, int n_bcs, double g, d
         // The fixed-point passes cover the Rusanov and HLLC fluxes, and with a
         // limiter the least-squares gradients.
         fixed = !cfg.fp32 && cfg.flux != FV_FLUX_EXACT && fixed_gamma() && (cfg.order == 1 || cfg.limiter != 0);
-        if (fixed) {
-            const double* st = batch ? batch_freestream : &bc.st[0][0];
-            std::vector<double> q;
-            for (int i = 0; i < (batch ? n_inst : kMaxPatches); ++i, st += 4) {
-                const bool has = st[0] != 0.0;  // patches without a farfield state stay zero
-                const double r = st[0], u = has ? st[1] / r : 0.0, v = has ? st[2] / r : 0.0;
-                const double p = (gamma - 1.0) * (st[3] - 0.5 * r * (u * u + v * v));
-                const double c = has ? std::sqrt(gamma * p / r) : 0.0;
-                for (double x : {r, u, v, p, c, has ? 1.0 / c : 0.0, 1.0 / gamma, 0.0}) q.push_back(x);
-            }
-            fsp = dupload(q, owned);
-        }
+        if (fixed) upload_farfield();
         if (fixed && cfg.order == 2 && cfg.gradient == 0) {
             fxa = dalloc<int4>(h2.d_cf.size(), owned);
             fxr = dalloc<int4>(h2.d_cf.size(), owned);
@@ -513,6 +516,7 @@ O1Args Solver::o1_args() const {
     a.flux = opt.flux;
     a.local_dt = opt.dt_mode == FV_DT_LOCAL;
     a.fixed = !opt.strict && fixed_gamma();
+    a.fsp = fsp;
     a.fxc = flux_const();
     return a;
 }

@@ -129,6 +129,7 @@ struct O1Args {
     int flux;          // 0 Rusanov, 1 HLLC, 2 exact
     int local_dt;
     int fixed;         // the persistent kernel's default build takes its fluxes in fixed point
+    const double* fsp = nullptr;  // its farfield states (as O2Args::fsp)
     fvfix::FluxConst fxc;
 };
 
