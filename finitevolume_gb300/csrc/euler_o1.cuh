@@ -31,6 +31,14 @@ __device__ __forceinline__ double warp_min(double v) {
     for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
     return v;
 }
+// The same for values that are not negative, by their bit patterns (integer
+// pipe); NaN counts as above all numbers.
+__device__ __forceinline__ double warp_min_pos(double v) {
+    unsigned long long b = (unsigned long long)__double_as_longlong(v);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) b = min(b, __shfl_xor_sync(0xffffffffu, b, o));
+    return __longlong_as_double((long long)b);
+}
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -109,7 +117,7 @@ __global__ void __launch_bounds__(fvgb::kFaceBlock) k_face_o1(const O1Args a) {
     }
     if (!LOCAL) {
         __shared__ double smin[fvgb::kFaceBlock / 32];
-        cand = warp_min(cand);
+        cand = warp_min_pos(cand);
         if ((threadIdx.x & 31) == 0) smin[threadIdx.x >> 5] = cand;
         __syncthreads();
         if (threadIdx.x == 0) {

@@ -471,7 +471,7 @@ __global__ void __launch_bounds__(fvgb::kCellBlock) k_o1_persistent(const O1Args
             cand = fmin(cand, face_phase_face<FLUX, LOCAL>(a, P, f, g, cfl));
         if (!LOCAL) {
             __shared__ double smin[fvgb::kCellBlock / 32];
-            cand = warp_min(cand);
+            cand = warp_min_pos(cand);
             if ((threadIdx.x & 31) == 0) smin[threadIdx.x >> 5] = cand;
             __syncthreads();
             if (threadIdx.x == 0) {

@@ -613,7 +613,7 @@ __device__ __forceinline__ V4<T> num_flux_p(const V4<T>& L, const V4<T>& R, T nx
 // The block's smallest candidate into the step's global-dt minimum.
 __device__ __forceinline__ void block_min_dt(double cand, StepCtl* ctl) {
     __shared__ double smin[fvgb::kMaxBlock / 32];
-    cand = warp_min(cand);
+    cand = warp_min_pos(cand);
     if ((threadIdx.x & 31) == 0) smin[threadIdx.x >> 5] = cand;
     __syncthreads();
     if (threadIdx.x == 0) {

@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(fvgb::kMaxBlock, 2) k_face_fx(const O2Args a) 
                 Smax = rmax(Smax, fabs(wrc.u * nx + wrc.v * ny) + cs[R]);
             }
             if (DT == 2) a.dtf[f] = Smax * ar;
-            else cand = a.ctl->cfl * q.w / Smax;
+            else cand = (a.ctl->cfl * q.w) * fvconv::rcp_nr3(Smax);
         }
     }
     if (DT == 1) block_min_dt(cand, a.ctl);

@@ -78,7 +78,7 @@ template <int FLUX>
 __global__ void __launch_bounds__(fvgb::kFaceBlock) k_ns_face(const NSArgs a) {
     // from the last face down: the boundary faces start first
     const int f = (gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x;
-    double cand = DBL_MAX;
+    double rate = 0.0;
     if (f < a.g.n_faces) {
         const int cl = a.fl[f], cr = a.g.fr[f];
         const bool bnd = cr < 0;
@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(fvgb::kFaceBlock) k_ns_face(const NSArgs a) {
         const double smax = inviscid<FLUX>(a, f, cl, cr, fg, rL, wl, rR, wr, F, uR, vR);
         // compute_dt: Smax + 2 nu / nd with the larger of the cells' mu / rho
         const double nu = (a.mu > 0.0) ? a.mu * rmax(wl.w, wr.w) : 0.0;
-        cand = (a.ctl->cfl * fg[5]) * fvconv::rcp_nr3(smax + 2.0 * nu * fg[0]);
+        rate = (smax + 2.0 * nu * fg[0]) * fg[0];
         const int p = bnd ? a.fpatch[f] : 0;
         if (!bnd || a.bc.type[p] == BC_NOSLIP) {
             if (bnd) {
@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(fvgb::kFaceBlock) k_ns_face(const NSArgs a) {
         }
         st_state(a.ff, f, F);
     }
-    min_candidate(cand, a.ctl);
+    max_rate(rate, a.ctl);
 }
 
 // The Euler cell pass with the fluxes summed on the integer pipe.
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(fvgb::kFaceBlock) k_ns_face(const NSArgs a) {
         st_state(a.ff, f, area * (inv - visc));
     }
     __shared__ double smin[fvgb::kFaceBlock / 32];
-    cand = warp_min(cand);
+    cand = warp_min_pos(cand);
     if ((threadIdx.x & 31) == 0) smin[threadIdx.x >> 5] = cand;
     __syncthreads();
     if (threadIdx.x == 0) {

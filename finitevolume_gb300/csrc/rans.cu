@@ -223,7 +223,7 @@ template <int FLUX>
 __global__ void __launch_bounds__(fvgb::kFaceBlock) k_sa_face(const RansArgs a) {
     // from the last face down: the boundary faces start first
     const int f = (gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x;
-    double cand = DBL_MAX;
+    double rate = 0.0;
     if (f < a.ns.g.n_faces) {
         const fvgb::NSArgs& n = a.ns;
         const int cl = n.fl[f], cr = n.g.fr[f];
@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(fvgb::kFaceBlock) k_sa_face(const RansArgs a) 
         double uR, vR;
         const double smax = inviscid<FLUX>(n, f, cl, cr, fg, rL, wl, rR, wr, F, uR, vR);
         const double nu_eff = ((n.mu > 0.0) ? rmax(nuL.x, nuR.x) : 0.0) + rmax(nuL.y, nuR.y);
-        cand = (n.ctl->cfl * fg[5]) * fvconv::rcp_nr3(smax + 2.0 * nu_eff * fg[0]);
+        rate = (smax + 2.0 * nu_eff * fg[0]) * fg[0];
 
         // nu-tilde upwinded by the mean velocity of the inviscid state pair
         const double Vn = 0.5 * ((wl.x + uR) * fg[6] + (wl.y + vR) * fg[7]);
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(fvgb::kFaceBlock) k_sa_face(const RansArgs a) 
         st_state(n.ff, f, F);
         a.nut_ff[f] = nut_flux;
     }
-    min_candidate(cand, a.ns.ctl);
+    max_rate(rate, a.ns.ctl);
 }
 
 template <int N> __device__ __forceinline__ double gather_nut(const double* ff, const int* cf) {
@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(fvgb::kFaceBlock) k_sa_face(const RansArgs a) 
         a.nut_ff[f] = nut_adv + nut_diff;
     }
     __shared__ double smin[fvgb::kFaceBlock / 32];
-    cand = warp_min(cand);
+    cand = warp_min_pos(cand);
     if ((threadIdx.x & 31) == 0) smin[threadIdx.x >> 5] = cand;
     __syncthreads();
     if (threadIdx.x == 0) {

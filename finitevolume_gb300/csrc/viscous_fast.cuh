@@ -150,16 +150,22 @@ __device__ __forceinline__ void traction(const double* fg, double ux, double uy,
     ty = xy * nx + (2.0 * vy - div) * ny;
 }
 
-// Block minimum of the faces' time-step candidates into the step's slot.
-__device__ __forceinline__ void min_candidate(double cand, fvgb::StepCtl* ctl) {
-    __shared__ double smin[fvgb::kFaceBlock / 32];
-    cand = warp_min(cand);
-    if ((threadIdx.x & 31) == 0) smin[threadIdx.x >> 5] = cand;
+// The block's largest wave rate (a face's wave speed over its length scale,
+// not negative; NaN does not count), as the time step cfl / rate, into the
+// step's slot: one reciprocal a block instead of one a face.
+__device__ __forceinline__ void max_rate(double rate, fvgb::StepCtl* ctl) {
+    __shared__ unsigned long long smax[fvgb::kFaceBlock / 32];
+    unsigned long long b = (unsigned long long)__double_as_longlong(rate);
+    if (b > 0x7ff0000000000000ull) b = 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
+    if ((threadIdx.x & 31) == 0) smax[threadIdx.x >> 5] = b;
     __syncthreads();
     if (threadIdx.x == 0) {
-        double v = smin[0];
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) v = fmin(v, smin[w]);
-        atomicMin(&ctl->dt_bits, (unsigned long long)__double_as_longlong(v));
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) b = max(b, smax[w]);
+        if (b == 0) return;
+        const double dt = ctl->cfl * fvconv::rcp_nr3(__longlong_as_double((long long)b));
+        atomicMin(&ctl->dt_bits, (unsigned long long)__double_as_longlong(dt));
     }
 }
 
