@@ -52,7 +52,11 @@ __device__ __forceinline__ double boundary_field(const NSArgs& a, int face, int 
 // a face (370 in the strict order), 55 a cell for the gradients (155).
 __global__ void __launch_bounds__(fvgb::kCellBlock) k_ns_prim(const NSArgs a) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < a.g.n_cells) a.prim[c] = prim_visc(ld_state(a.U, c), a.gamma, a.inv_R);
+    if (c >= a.g.n_cells) return;
+    const St s = ld_state(a.U, c);
+    double p;
+    a.prim[c] = prim_visc(s, a.gamma, a.inv_R, p);
+    a.rp[c] = make_double2(s.r, p);
 }
 
 __global__ void __launch_bounds__(fvgb::kCellBlock) k_ns_grad(const NSArgs a) {
@@ -85,12 +89,12 @@ __global__ void __launch_bounds__(fvgb::kFaceBlock) k_ns_face(const NSArgs a) {
         const double* fg = a.g.fgrad + 8 * (size_t)f;
         const double4_32a wl = a.prim[cl];
         double4_32a wr = bnd ? wl : a.prim[cr];
-        const double rL = a.U[cl].r, rR = bnd ? rL : a.U[cr].r;
+        const double2 qL = a.rp[cl], qR = bnd ? qL : a.rp[cr];
         St F;
         double uR, vR;
-        const double smax = inviscid<FLUX>(a, f, cl, cr, fg, rL, wl, rR, wr, F, uR, vR);
+        const double smax = inviscid<FLUX>(a, f, cl, cr, fg, qL, wl, qR, wr, F, uR, vR);
         // compute_dt: Smax + 2 nu / nd with the larger of the cells' mu / rho
-        const double nu = (a.mu > 0.0) ? a.mu * rmax(wl.w, wr.w) : 0.0;
+        const double nu = (a.mu > 0.0) ? a.mu * max_pos(wl.w, wr.w) : 0.0;
         rate = (smax + 2.0 * nu * fg[0]) * fg[0];
         const int p = bnd ? a.fpatch[f] : 0;
         if (!bnd || a.bc.type[p] == BC_NOSLIP) {
@@ -120,14 +124,14 @@ __global__ void __launch_bounds__(fvgb::kFaceBlock) k_ns_face(const NSArgs a) {
 }
 
 // The Euler cell pass with the fluxes summed on the integer pipe.
-__global__ void __launch_bounds__(fvgb::kCellBlock) k_ns_cell(const O1Args a) {
+__global__ void __launch_bounds__(fvgb::kCellBlock) k_ns_cell(const O1Args a, const double* __restrict__ inv_vol) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     double res[4] = {0.0, 0.0, 0.0, 0.0};
     if (c < a.m.n_cells) {
         const double dt = __longlong_as_double((long long)a.ctl->dt_bits);
         const St R = gather_any(a.ff, a.m.cf, a.m.cf_off[c], a.m.cf_off[c + 1]);
         res[0] = R.r; res[1] = R.ru; res[2] = R.rv; res[3] = R.E;
-        st_state(a.U, c, ld_state(a.U, c) + (dt * fvconv::rcp_nr3(a.m.vol[c])) * R);
+        st_state(a.U, c, ld_state(a.U, c) + (dt * inv_vol[c]) * R);
     }
     finish_norms(warp_squares(res), a.ctl, a.partials, a.hist, a.hist_cap);
 }
@@ -291,7 +295,7 @@ void FV_NS_FN(ns_launch_step)(const NSArgs& a, const O1Args& cell, cudaStream_t 
         default: FV_KNS::k_ns_face<0><<<fb, bs, 0, s>>>(a); break;
     }
 #ifdef FV_NS_FAST
-    FV_KNS::k_ns_cell<<<cb, kCellBlock, 0, s>>>(cell);
+    FV_KNS::k_ns_cell<<<cb, kCellBlock, 0, s>>>(cell, a.inv_vol);
 #else
     FV_KNS::k_cell_o1<false><<<cb, kCellBlock, 0, s>>>(cell);
 #endif

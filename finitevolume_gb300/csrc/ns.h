@@ -22,6 +22,9 @@ struct NSArgs {
     int fixed;                 // default build: inviscid fluxes in fixed point (fixed.cuh)
     fvfix::FluxConst fxc;
     double inv_R;              // 1 / gas_constant
+    // default build: density and pressure per cell, 1 / volume
+    double2* rp;
+    const double* inv_vol;
 };
 
 // Strict (no FMA contraction, reference evaluation order) and _fast

@@ -77,15 +77,13 @@ __device__ __forceinline__ double inv_root6(double z) {
 }
 
 // sa_source of the strict build with its divisions as reciprocals shared
-// between terms; chi = nut / nu.
-__device__ __forceinline__ double sa_source(const RansArgs& a, double nut, double chi, double omega, double d,
-                                            double gx, double gy) {
+// between terms; chi = nut / nu, chi_fv1 = nu_t / nu, id = 1 / d.
+__device__ __forceinline__ double sa_source(const RansArgs& a, double nut, double chi, double chi_fv1, double omega,
+                                            double id, double gx, double gy) {
     const double cb1 = a.sa[0], cw2 = a.sa[4], cv2 = a.sa[7], cv3 = a.sa[8];
     const bool pos = nut > 0.0;
     chi = pos ? chi : 0.0;
-    const double fv1 = pos ? sa_fv1_chi(chi, a.cv1_3) : 0.0;
-    const double fv2 = 1.0 - chi * fvconv::rcp_nr3(1.0 + chi * fv1);
-    const double id = fvconv::rcp_nr3(d);
+    const double fv2 = 1.0 - chi * fvconv::rcp_nr3(1.0 + (pos ? chi_fv1 : 0.0));
     const double q = nut * ((id * id) * a.inv_kappa2), s_bar = q * fv2;
     double s_tilde;
     if (s_bar >= -cv2 * omega) s_tilde = omega + s_bar;
@@ -106,7 +104,9 @@ __global__ void __launch_bounds__(fvgb::kCellBlock) k_sa_prim(const RansArgs a) 
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= a.ns.g.n_cells) return;
     const St s = ld_state(a.ns.U, c);
-    double4_32a w = prim_visc(s, a.ns.gamma, a.ns.inv_R);
+    double p;
+    double4_32a w = prim_visc(s, a.ns.gamma, a.ns.inv_R, p);
+    a.ns.rp[c] = make_double2(s.r, p);
     const double nu = a.ns.mu * w.w;
     w.w = a.nut[c];
     a.ns.prim[c] = w;
@@ -162,6 +162,7 @@ __global__ void k_sa_wall_distance(const RansArgs a, const double4_32a* __restri
         best = rmin(best, d2);
     }
     a.walld[c] = sqrt(best);
+    if (a.inv_walld) a.inv_walld[c] = 1.0 / sqrt(best);
 }
 
 __global__ void __launch_bounds__(fvgb::kCellBlock) k_sa_prim(const RansArgs a) {
@@ -233,11 +234,12 @@ __global__ void __launch_bounds__(fvgb::kFaceBlock) k_sa_face(const RansArgs a) 
         const double4_32a wl = n.prim[cl];
         double4_32a wr = bnd ? wl : n.prim[cr];
         const double2 nuL = a.nu[cl], nuR = bnd ? nuL : a.nu[cr];
-        const double rL = n.U[cl].r, rR = bnd ? rL : n.U[cr].r;
+        const double2 qL = n.rp[cl], qR = bnd ? qL : n.rp[cr];
+        const double rL = qL.x, rR = qR.x;
         St F;
         double uR, vR;
-        const double smax = inviscid<FLUX>(n, f, cl, cr, fg, rL, wl, rR, wr, F, uR, vR);
-        const double nu_eff = ((n.mu > 0.0) ? rmax(nuL.x, nuR.x) : 0.0) + rmax(nuL.y, nuR.y);
+        const double smax = inviscid<FLUX>(n, f, cl, cr, fg, qL, wl, qR, wr, F, uR, vR);
+        const double nu_eff = ((n.mu > 0.0) ? max_pos(nuL.x, nuR.x) : 0.0) + max_pos(nuL.y, nuR.y);
         rate = (smax + 2.0 * nu_eff * fg[0]) * fg[0];
 
         // nu-tilde upwinded by the mean velocity of the inviscid state pair
@@ -430,11 +432,12 @@ __global__ void __launch_bounds__(fvgb::kCellBlock) k_sa_cell(const RansArgs a) 
         else
             for (int e = e0; e < e1; ++e) Rn += (a.cf[e] & 1) ? -a.nut_ff[a.cf[e] >> 1] : a.nut_ff[a.cf[e] >> 1];
         const double2 gu = a.grad[4 * c], gv = a.grad[4 * c + 1], gn = a.grad[4 * c + 3];
-        const double vol = a.vol[c], nut = a.nut[c];
+        const double nut = a.nut[c];
         const St u = ld_state(a.ns.U, c);
-        Rn += vol * sa_source(a, nut, nut * (u.r * a.inv_mu), fabs(gv.x - gu.y), a.walld[c], gn.x, gn.y);
-        s[0] = R.r; s[1] = R.ru; s[2] = R.rv; s[3] = R.E; s[4] = Rn * Rn;
-        const double k = __longlong_as_double((long long)ctl->dt_bits) * fvconv::rcp_nr3(vol);
+        const double inv_nu = u.r * a.inv_mu;
+        Rn += a.vol[c] * sa_source(a, nut, nut * inv_nu, a.nu[c].y * inv_nu, fabs(gv.x - gu.y), a.inv_walld[c], gn.x, gn.y);
+        s[0] = R.r; s[1] = R.ru; s[2] = R.rv; s[3] = R.E; s[4] = Rn;
+        const double k = __longlong_as_double((long long)ctl->dt_bits) * a.ns.inv_vol[c];
         st_state(a.ns.U, c, u + k * R);
         a.nut[c] = nut + k * Rn;
     }
@@ -466,7 +469,8 @@ __global__ void __launch_bounds__(fvgb::kCellBlock) k_sa_cell(const RansArgs a) 
 #ifdef FV_NS_FAST
     const double res[4] = {s[0], s[1], s[2], s[3]};
     const double s4 = warp_squares(res);
-    s[4] = warp_sum(s[4]);
+    const double res_nut[4] = {s[4], 0.0, 0.0, 0.0};
+    s[4] = warp_squares(res_nut);
     const int lane = threadIdx.x & 31;
     if ((lane & 7) == 0) red[w][lane >> 3] = s4;
     if (lane == 0) red[w][4] = s[4];

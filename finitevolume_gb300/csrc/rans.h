@@ -16,6 +16,7 @@ struct RansArgs {
     double2* nu;           // [N] molecular and eddy kinematic viscosity
     double2* grad;         // [4N] gradients of u, v, T, nu-tilde
     double* walld;         // [N] distance to the nearest no-slip wall
+    double* inv_walld;     // [N] its reciprocal (default build, else null)
     double* partials;      // [5 * cell blocks]
     double* hist;          // [hist_cap * 4] mean-flow norms
     double* nut_hist;      // [hist_cap] nu-tilde norms

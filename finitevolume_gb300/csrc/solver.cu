@@ -365,6 +365,12 @@ void Solver::init(const HostMesh& hm, const fv_bc_t* bcs, int n_bcs, double g, d
         a.ff = ff;
         a.prim = dalloc<double4_32a>(N, owned);
         a.grad = dalloc<double2>(3 * (size_t)N, owned);
+        if (!opt.strict) {
+            a.rp = dalloc<double2>(N, owned);
+            std::vector<double> iv(N);
+            for (int c = 0; c < N; ++c) iv[c] = 1.0 / hm.d_vol[c];
+            a.inv_vol = dupload(iv, owned);
+        }
         a.ctl = ctl;
         a.bc = bc;
         a.gamma = gamma;
@@ -395,6 +401,7 @@ void Solver::init(const HostMesh& hm, const fv_bc_t* bcs, int n_bcs, double g, d
         r.nu = dalloc<double2>(N, owned);
         r.grad = dalloc<double2>(4 * (size_t)N, owned);
         r.walld = dalloc<double>(N, owned);
+        r.inv_walld = opt.strict ? nullptr : dalloc<double>(N, owned);
         r.partials = dalloc<double>(5 * (size_t)n_cell_blocks, owned);
         r.nut_norm = dupload(std::vector<double>(1, 0.0), owned);
         for (int p = 0; p < kMaxPatches; ++p) r.farfield_nut[p] = p < hm.n_patches ? bcs[p].nut : 0.0;
@@ -423,6 +430,7 @@ void Solver::init(const HostMesh& hm, const fv_bc_t* bcs, int n_bcs, double g, d
         if (seg.empty()) {
             // no wall: infinite distance, as compute_wall_distance
             h2d_sync(r.walld, std::vector<double>(N, INFINITY).data(), sizeof(double) * N);
+            if (r.inv_walld) h2d_sync(r.inv_walld, std::vector<double>(N, 0.0).data(), sizeof(double) * N);
         } else {
             double4_32a* d_seg = dupload(seg, owned);
             RansArgs tmp = rans_args();

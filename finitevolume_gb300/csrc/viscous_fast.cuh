@@ -15,19 +15,25 @@ namespace FV_KNS {
 using fvgb::GradDev;
 using fvgb::NSArgs;
 
-// u, v, T and 1/rho of a conserved state
-__device__ __forceinline__ double4_32a prim_visc(const St& s, double g, double inv_R) {
+// u, v, T and 1/rho of a conserved state, and its pressure
+__device__ __forceinline__ double4_32a prim_visc(const St& s, double g, double inv_R, double& p) {
     const double ir = fvconv::rcp_nr3(s.r);
     double4_32a w;
     w.x = s.ru * ir;
     w.y = s.rv * ir;
-    w.z = ((g - 1.0) * (s.E - 0.5 * (s.ru * w.x + s.rv * w.y))) * (ir * inv_R);
+    p = (g - 1.0) * (s.E - 0.5 * (s.ru * w.x + s.rv * w.y));
+    w.z = p * (ir * inv_R);
     w.w = ir;
     return w;
 }
 
 __device__ __forceinline__ double comp(const double4_32a& w, int k) {
     return k == 0 ? w.x : (k == 1 ? w.y : (k == 2 ? w.z : w.w));
+}
+
+// The larger of two values that are not negative, by their bit patterns
+__device__ __forceinline__ double max_pos(double a, double b) {
+    return __double_as_longlong(a) < __double_as_longlong(b) ? b : a;
 }
 
 // Gradients of the first NV components of prim; bvec(face): the boundary
@@ -88,17 +94,17 @@ __device__ __noinline__ double inviscid_f64(const NSArgs& n, int f, int cl, int 
     return face_smax(UL, UR, cr >= 0, geo.x, geo.y, n.gamma);
 }
 
-// rL, rR: the cells' densities (rR unused on a boundary face); fg: the fast
-// fgrad row.  uR, vR: the velocity of the right state (a boundary face's
+// qL, qR: the cells' densities and pressures (qR unused on a boundary face);
+// fg: the fast fgrad row.  uR, vR: the velocity of the right state (a boundary face's
 // ghost).
 template <int FLUX>
-__device__ __forceinline__ double inviscid(const NSArgs& n, int f, int cl, int cr, const double* fg, double rL,
-                                           const double4_32a& wl, double rR, const double4_32a& wr, St& F, double& uR,
-                                           double& vR) {
-    fvfix::State L = {rL, wl.x, wl.y, rL * (wl.z * n.gas_constant)}, R;
+__device__ __forceinline__ double inviscid(const NSArgs& n, int f, int cl, int cr, const double* fg,
+                                           const double2& qL, const double4_32a& wl, const double2& qR,
+                                           const double4_32a& wr, St& F, double& uR, double& vR) {
+    fvfix::State L = {qL.x, wl.x, wl.y, qL.y}, R;
     bool ok = FLUX != FLUX_EXACT && n.fixed;
     if (cr >= 0) {
-        R = {rR, wr.x, wr.y, rR * (wr.z * n.gas_constant)};
+        R = {qR.x, wr.x, wr.y, qR.y};
     } else {
         const int p = n.fpatch[f], t = n.bc.type[p];
         R = L;
