@@ -14,8 +14,9 @@
 // Bound: FP64 issue in the face pass (8 instructions a face: the difference,
 // the quotient as five multiply-adds with the prepared reciprocal, two
 // products), launches below about 100k cells.  260k cells: face pass 16 ->
-// 14 us (division -> quotient), cell pass 66 -> 11 us (its last block folded
-// the block partials with one thread, and every cell divided dt by V).
+// 14 us (division -> quotient), cell pass 66 -> 8 us (its last block folded
+// the block partials with one thread, every cell divided dt by V, and the norm
+// took six of twelve FP64 instructions, now one, fvfix::warp_squares).
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
@@ -25,6 +26,7 @@
 
 #include "../../include/fv_gb300.h"
 #include "errors.h"
+#include "fixed.cuh"
 #include "fpconv.cuh"
 #include "mesh_host.h"
 #include "types.h"
@@ -96,11 +98,12 @@ __global__ void __launch_bounds__(kCellBlock) k_diff_cell(const DiffArgs a, int 
             const int ent = a.cf[e];
             r += flip1(a.ff[ent >> 1], ent);
         }
-        s = r * r;
+        s = r;
         a.phi[c] += a.coef[c] * r;
     }
     __shared__ double red[kCellBlock / 32];
-    s = wsum(s);
+    double q;
+    s = fvfix::warp_squares(s, q) ? q : wsum(s * s);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
     __syncthreads();
     if (threadIdx.x == 0) {

@@ -413,22 +413,36 @@ __device__ __forceinline__ bool quotient(double a, const Fixed& s, double& q) {
     q = to_double(x, ea - 1023 - (s.k + 63 - lz) - 58);
     return abs(ea - 1023 - (s.k + 63 - lz)) < 900;
 }
+// x^2 in units of 2^(2 (E - 1023) - 57), E the warp's largest biased exponent:
+// rounded, below 2^59, so that 32 of them add up exactly in 64 bits.  All 32
+// lanes call it; false (on all) where a value is not finite or its square out
+// of range.
+__device__ __forceinline__ bool warp_square(double x, u64& v, int& E) {
+    const int e = biased(hi_word(x));
+    E = __reduce_max_sync(0xffffffffu, e);
+    const Sp m = split((i64)(top_bits(x) >> 3));  // Q60, in [1, 2)
+    v = e == 0 ? 0 : (shr((u64)mul<1>(m, m) << 1, 2 * (E - e)) + 1) >> 1;
+    return E <= 1500 && (E == 0 || E >= 550);
+}
+// The sum of x^2 over a warp, in every lane; as above.
+__device__ __forceinline__ bool warp_squares(double x, double& sum) {
+    u64 s;
+    int E;
+    const bool ok = warp_square(x, s, E);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    sum = s == 0 ? 0.0 : scale2(__ull2double_rn(s), 2 * (E - 1023) - 57);
+    return ok;
+}
 // The sums over a warp of x^2 for four values a lane (all 32 lanes call it):
-// the k-th in the lanes 8 k to 8 k + 7, as warp_sum4's.  Squares as integers
-// in units of 2^-57 of the warp's largest binade (below 2^59, the sum below
-// 2^64), rounded and added exactly: one FP64 instruction instead of ten.
-// False (on all lanes) where a value is not finite or its square out of range.
+// the k-th in the lanes 8 k to 8 k + 7, as warp_sum4's; one FP64 instruction
+// instead of ten.
 __device__ __forceinline__ bool warp_squares4(const double (&x)[4], double& sum) {
     u64 v[4];
-    int E[4], bad = 0;
+    int E[4];
+    bool ok = true;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int e = biased(hi_word(x[k]));
-        E[k] = __reduce_max_sync(0xffffffffu, e);
-        bad |= E[k] > 1500 || (E[k] != 0 && E[k] < 550);
-        const Sp m = split((i64)(top_bits(x[k]) >> 3));  // Q60, in [1, 2)
-        v[k] = e == 0 ? 0 : (shr((u64)mul<1>(m, m) << 1, 2 * (E[k] - e)) + 1) >> 1;
-    }
+    for (int k = 0; k < 4; ++k) ok &= warp_square(x[k], v[k], E[k]);
     const int lane = threadIdx.x & 31;
     const bool h16 = lane & 16, h8 = lane & 8;
     u64 a = h16 ? v[2] : v[0], b = h16 ? v[3] : v[1];
@@ -441,7 +455,7 @@ __device__ __forceinline__ bool warp_squares4(const double (&x)[4], double& sum)
     s += __shfl_xor_sync(0xffffffffu, s, 1);
     const int e = h16 ? (h8 ? E[3] : E[2]) : (h8 ? E[1] : E[0]);
     sum = s == 0 ? 0.0 : scale2(__ull2double_rn(s), 2 * (e - 1023) - 57);
-    return bad == 0;
+    return ok;
 }
 
 // num / den * 2^52, rounded, for 0 < num <= den, den in [2^56, 2^62): three

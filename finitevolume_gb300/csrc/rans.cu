@@ -469,8 +469,8 @@ __global__ void __launch_bounds__(fvgb::kCellBlock) k_sa_cell(const RansArgs a) 
 #ifdef FV_NS_FAST
     const double res[4] = {s[0], s[1], s[2], s[3]};
     const double s4 = warp_squares(res);
-    const double res_nut[4] = {s[4], 0.0, 0.0, 0.0};
-    s[4] = warp_squares(res_nut);
+    double s_nut;
+    s[4] = fvfix::warp_squares(s[4], s_nut) ? s_nut : warp_sum(s[4] * s[4]);
     const int lane = threadIdx.x & 31;
     if ((lane & 7) == 0) red[w][lane >> 3] = s4;
     if (lane == 0) red[w][4] = s[4];
