@@ -29,14 +29,17 @@
 // normal velocity of the Rusanov flux from P instead of a division per face
 // side, and the local-dt update factor dt/V = cfl / sum lambda A by one
 // reciprocal, and the ghost states from P with short dependent chains
-// (ghost_p); it agrees with the reference within 1e-10.  In both builds the
-// norm partials are formed over the same 256-cell tiles and folded in the
-// same order as k_cell_o1's, so the residual history is bit-identical to
-// the two-kernel path too.
+// (ghost_p), and takes fluxes and sums on the integer pipe (fixed.cuh); it
+// agrees with the reference within 1e-10.  In both builds the norm partials
+// are formed over the same 256-cell tiles and folded in the same order as
+// k_cell_o1's, so in the strict build the residual history is bit-identical
+// to the two-kernel path too.
 //
-// With local dt a step has no global dependency, and the dataflow form
-// (k_o1_dataflow, further down) replaces the grid barriers by waits on the
-// few blocks that share faces with each block.
+// With local dt a step has no global dependency, and the dataflow forms
+// (k_o1_dataflow_sm; k_o1_dataflow in the strict build, further down) replace
+// the grid barriers by waits on the few blocks that share faces with each
+// block.  Where they do not apply the default build runs the barrier form's
+// phases as launches of their own (k_o1_split_*).
 //
 // The grid barrier is a counter plus a generation word.  Every wait (grid
 // barrier or neighbour progress) is bounded (PersistCtl::limit, in SM clock
@@ -432,7 +435,7 @@ __device__ __forceinline__ void fold_step_norms(StepCtl* ctl, const double* part
 }
 
 template <int FLUX, bool LOCAL>
-__global__ void __launch_bounds__(fvgb::kCellBlock) k_o1_persistent(const O1Args a, double4_32a* __restrict__ P,
+__global__ void __launch_bounds__(fvgb::kCellBlock, FLUX == FLUX_EXACT ? 2 : 3) k_o1_persistent(const O1Args a, double4_32a* __restrict__ P,
                                                                      PersistCtl* __restrict__ pc, int nsteps) {
     const double g = a.gamma;
     const int nb = gridDim.x;
@@ -633,6 +636,7 @@ __device__ __forceinline__ void df_fold(const O1Args& a, const DfPlan& d, int s,
     __syncthreads();
 }
 
+#ifdef FV_STRICT_ORDER  // (the default build uses the form below or k_o1_split_*)
 template <int FLUX>
 __global__ void __launch_bounds__(fvgb::kDfBlock, 1) k_o1_dataflow(const O1Args a, double4_32a* __restrict__ P,
                                                                   PersistCtl* __restrict__ pc, const DfPlan d,
@@ -684,6 +688,7 @@ __global__ void __launch_bounds__(fvgb::kDfBlock, 1) k_o1_dataflow(const O1Args 
     for (int s = b; s < nsteps; s += nb) df_fold(a, d, s, (step0 + s) % a.hist_cap, s == nsteps - 1);
     if (b == 0 && threadIdx.x == 0) a.ctl->step = step0 + nsteps;
 }
+#endif
 
 // The same with the block's own cells and the fluxes of all their faces in
 // shared memory, for blocks that fit (DfPlan::smem).  A face between two
@@ -701,7 +706,7 @@ __global__ void __launch_bounds__(fvgb::kDfBlock, 1) k_o1_dataflow(const O1Args 
 //
 // Bound: the dependent chain of one step (mailbox round trip, a face's flux, a
 // cell's update) below about 20k cells, FP64 issue above.  32k cells,
-// Rusanov: see the launch rule.
+// Rusanov: 8.7 us a step (states and fluxes in L2 with progress words 15.2).
 __device__ __forceinline__ void mail_store(double2* w, double v, unsigned long long tag) {
     const unsigned long long b = (unsigned long long)__double_as_longlong(v);
     asm volatile("{.reg .b128 q; mov.b128 q, {%1, %2}; st.relaxed.gpu.global.b128 [%0], q;}" ::"l"(w), "l"(b), "l"(tag)
@@ -892,6 +897,7 @@ static int o1df_sm_blocks_per_sm(size_t smem) {
     return nb;
 }
 
+#ifdef FV_STRICT_ORDER
 template <int FLUX>
 static int o1df_blocks_per_sm() {
     int nb = 0;
@@ -899,6 +905,7 @@ static int o1df_blocks_per_sm() {
         return 0;
     return nb;
 }
+#endif
 
 template <int FLUX>
 static cudaError_t launch_o1df(const O1Args& a, double4_32a* P, PersistCtl* pc, const DfPlan& d, int nsteps,
@@ -914,8 +921,129 @@ static cudaError_t launch_o1df(const O1Args& a, double4_32a* P, PersistCtl* pc, 
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     if (d.smem) return cudaLaunchKernelEx(&cfg, k_o1_dataflow_sm<FLUX>, a, pc, d, nsteps);
+#ifdef FV_STRICT_ORDER
     return cudaLaunchKernelEx(&cfg, k_o1_dataflow<FLUX>, a, P, pc, d, nsteps);
+#else
+    return cudaErrorInvalidValue;
+#endif
 }
+
+#ifndef FV_STRICT_ORDER
+// ---------------------------------------------------------------------------
+// The barrier form's phases as launches of their own: the launch boundary is
+// the barrier.  Registers are then a phase's own (24 to 32 warps an SM; the
+// persistent kernel runs 16 to 24), cells come through L1, which holds them for
+// the neighbouring faces, and the norms' fold runs beside a face pass.  Same
+// arithmetic, tiles and folds as the barrier form's.
+//
+// Bound: FP64 issue and latency (HLLC, global dt, us a step): 500k cells 82
+// (barrier form 108), 131k 26 (43), 32k 15 (20), 2k 12 (15, launches and the
+// farfield's chain).  64 registers for Rusanov, 84 for the others, which spill
+// at 64 (HLLC 1.13 ms for 40 steps of 131k cells at 84, 1.21 at 64, 1.20 at 128).
+__device__ __forceinline__ Prim ld_prim_l1(const double4_32a* P, int i) {
+    const St p = ld_state(reinterpret_cast<const St*>(P), i);
+    Prim o;
+    o.u = p.r; o.v = p.ru; o.p = p.rv; o.c = p.E;
+    return o;
+}
+
+__global__ void __launch_bounds__(fvgb::kCellBlock) k_o1_split_prim(const O1Args a, double4_32a* __restrict__ P,
+                                                                   PersistCtl* __restrict__ pc) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c < a.m.n_cells) st_prim(P, c, prim_of(ld_state(a.U, c), a.gamma));
+    if (c < 2) pc->dt_slot[c] = (unsigned long long)__double_as_longlong(DBL_MAX);
+}
+
+// The first `folds` blocks fold the norms of the steps from fold0 on.
+template <int FLUX, bool LOCAL>
+__global__ void __launch_bounds__(fvgb::kCellBlock, FLUX == FLUX_RUSANOV ? 4 : 3) k_o1_split_face(const O1Args a, const double4_32a* __restrict__ P,
+                                                                      PersistCtl* __restrict__ pc, int s, int fold0,
+                                                                      int folds, int nsteps) {
+    const int F = a.m.n_faces;
+    if ((int)blockIdx.x < folds) {
+        const int j = fold0 + blockIdx.x, n_tiles = (a.m.n_cells + fvgb::kCellBlock - 1) / fvgb::kCellBlock;
+        fold_step_norms(a.ctl, a.partials + (size_t)(j % fvgb::kNormRing) * n_tiles * 4, n_tiles,
+                        a.hist + (size_t)((a.ctl->step + j) % a.hist_cap) * 4, j == nsteps - 1);
+        return;
+    }
+    // from the last face down: the boundary faces have the longest chains
+    const int f = F - 1 - (int)((blockIdx.x - folds) * blockDim.x + threadIdx.x);
+    double cand = DBL_MAX;
+    if (f >= 0) {
+        const int L = a.m.fl[f], R = a.m.fr[f], Rs = R >= 0 ? R : L;
+        double dt;
+        const St Fl = face_compute<FLUX, LOCAL>(a, f, R >= 0, a.m.fgeom[f], ld_state(a.U, L), ld_prim_l1(P, L),
+                                                ld_state(a.U, Rs), ld_prim_l1(P, Rs), a.gamma, a.ctl->cfl, dt);
+        st_state(a.ff, f, Fl);
+        if (LOCAL) a.dtf[f] = dt;
+        else cand = dt;
+    }
+    if (!LOCAL) {
+        __shared__ double smin[fvgb::kCellBlock / 32];
+        cand = warp_min_pos(cand);
+        if ((threadIdx.x & 31) == 0) smin[threadIdx.x >> 5] = cand;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double v = smin[0];
+            for (int w = 1; w < (int)(blockDim.x >> 5); ++w) v = fmin(v, smin[w]);
+            atomicMin(&pc->dt_slot[s & 1], (unsigned long long)__double_as_longlong(v));
+        }
+    }
+}
+
+template <bool LOCAL>
+__global__ void __launch_bounds__(fvgb::kCellBlock, 4) k_o1_split_cell(const O1Args a, double4_32a* __restrict__ P,
+                                                                      PersistCtl* __restrict__ pc, int s) {
+    const int c = blockIdx.x * fvgb::kCellBlock + threadIdx.x;
+    const double dt_g = LOCAL ? 0.0 : __longlong_as_double((long long)pc->dt_slot[s & 1]);
+    St R = st_make(0.0, 0.0, 0.0, 0.0);
+    if (c < a.m.n_cells) {
+        const int* cf = a.m.cf + a.m.cf_off[c];
+        Prim q;
+        const St un = cell_compute<LOCAL>(
+            a, c,
+            [&](int i, double& l) {
+                const int f = cf[i] >> 1;
+                if (LOCAL) l = a.dtf[f];
+                return ld_state(a.ff, f);
+            },
+            ld_state(a.U, c), a.gamma, a.ctl->cfl, dt_g, q, R);
+        st_state(a.U, c, un);
+        st_prim(P, c, q);
+    }
+    if (!LOCAL && c == 0) pc->dt_slot[(s & 1) ^ 1] = (unsigned long long)__double_as_longlong(DBL_MAX);
+    __shared__ double red[fvgb::kCellBlock / 32][4];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const double ws = warp_norms(R);
+    if ((lane & 7) == 0) red[w][lane >> 3] = ws;
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        double v = 0.0;
+        for (int i = 0; i < fvgb::kCellBlock / 32; ++i) v += red[i][threadIdx.x];
+        a.partials[((size_t)(s % fvgb::kNormRing) * gridDim.x + blockIdx.x) * 4 + threadIdx.x] = v;
+    }
+}
+
+static __global__ void k_o1_split_done(StepCtl* ctl, int nsteps) { ctl->step += nsteps; }
+
+template <int FLUX, bool LOCAL>
+static cudaError_t launch_o1_split(const O1Args& a, double4_32a* P, PersistCtl* pc, int nsteps, cudaStream_t st) {
+    constexpr int B = fvgb::kCellBlock, ring = fvgb::kNormRing;
+    const int cb = (a.m.n_cells + B - 1) / B, fb = (a.m.n_faces + 127) / 128;
+    k_o1_split_prim<<<cb, B, 0, st>>>(a, P, pc);
+    for (int s = 0; s < nsteps; ++s) {
+        const int folds = s > 0 && s % ring == 0 ? ring : 0;
+        // (a fold takes a block of kCellBlock threads: those steps have them)
+        if (folds) k_o1_split_face<FLUX, LOCAL><<<folds + (a.m.n_faces + B - 1) / B, B, 0, st>>>(a, P, pc, s, s - ring, folds, nsteps);
+        else k_o1_split_face<FLUX, LOCAL><<<fb, 128, 0, st>>>(a, P, pc, s, 0, 0, nsteps);
+        k_o1_split_cell<LOCAL><<<cb, B, 0, st>>>(a, P, pc, s);
+    }
+    const int rest = nsteps > 0 ? (nsteps - 1) % ring + 1 : 0;  // the last steps' norms: a launch of folds alone
+    if (rest) k_o1_split_face<FLUX, LOCAL><<<rest, B, 0, st>>>(a, P, pc, 0, nsteps - rest, rest, nsteps);
+    k_o1_split_done<<<1, 1, 0, st>>>(a.ctl, nsteps);
+    return cudaGetLastError();
+}
+#endif
 
 template <int FLUX, bool LOCAL>
 static int o1p_blocks_per_sm() {
@@ -961,6 +1089,7 @@ int o1p_max_blocks_per_sm(int flux, int local) {
         default: return ::FV_KNS::o1p_blocks_per_sm<2, true>();
     }
 }
+#ifdef FV_STRICT_ORDER
 int o1df_max_blocks_per_sm(int flux) {
     switch (flux) {
         case 0: return ::FV_KNS::o1df_blocks_per_sm<0>();
@@ -968,6 +1097,7 @@ int o1df_max_blocks_per_sm(int flux) {
         default: return ::FV_KNS::o1df_blocks_per_sm<2>();
     }
 }
+#endif
 int o1df_sm_max_blocks_per_sm(int flux, size_t smem) {
     switch (flux) {
         case 0: return ::FV_KNS::o1df_sm_blocks_per_sm<0>(smem);
@@ -983,6 +1113,18 @@ cudaError_t launch_o1_dataflow(const O1Args& a, double4_32a* P, PersistCtl* pc, 
         default: return ::FV_KNS::launch_o1df<2>(a, P, pc, d, nsteps, grid, s);
     }
 }
+#ifndef FV_STRICT_ORDER
+cudaError_t launch_o1_split(const O1Args& a, double4_32a* P, PersistCtl* pc, int nsteps, cudaStream_t s) {
+    switch (a.flux * 2 + (a.local_dt ? 1 : 0)) {
+        case 0: return ::FV_KNS::launch_o1_split<0, false>(a, P, pc, nsteps, s);
+        case 1: return ::FV_KNS::launch_o1_split<0, true>(a, P, pc, nsteps, s);
+        case 2: return ::FV_KNS::launch_o1_split<1, false>(a, P, pc, nsteps, s);
+        case 3: return ::FV_KNS::launch_o1_split<1, true>(a, P, pc, nsteps, s);
+        case 4: return ::FV_KNS::launch_o1_split<2, false>(a, P, pc, nsteps, s);
+        default: return ::FV_KNS::launch_o1_split<2, true>(a, P, pc, nsteps, s);
+    }
+}
+#endif
 cudaError_t launch_o1_persistent(const O1Args& a, double4_32a* P, PersistCtl* pc, int nsteps, int grid,
                                  cudaStream_t s) {
     switch (a.flux * 2 + (a.local_dt ? 1 : 0)) {

@@ -719,11 +719,21 @@ bool dataflow_plan(const HostMesh& hm, const int* patch_type, int sms, DataflowP
 }
 
 void Solver::build_dataflow(const HostMesh& hm, int sms) {
-    const int per_sm = opt.strict ? strict::o1df_max_blocks_per_sm(opt.flux) : fast::o1df_max_blocks_per_sm(opt.flux);
-    if (per_sm < 1) return;
+    if (opt.strict && strict::o1df_max_blocks_per_sm(opt.flux) < 1) return;
     DataflowPlan p;
     if (!dataflow_plan(hm, bc.type, sms, p)) return;
     const int nb = p.nb, Wn = (N + 31) / 32;
+    // The shared-memory form where every block's cells (96 bytes each) and
+    // their faces (40) fit: up to about 1,100 cells a block, 170k a mesh.
+    // Larger meshes are bound by the work itself: the default build runs the
+    // barrier form's phases as launches there (262k cells, Rusanov, 40 steps:
+    // 1.62 ms against 1.97 for the states in L2; 131k 1.04 against 1.06 here),
+    // the strict build keeps the states in L2.
+    size_t own = 0;
+    for (int b = 0; b < nb; ++b)
+        own = std::max(own, 96 * (size_t)(p.cell_off[b + 1] - p.cell_off[b]) +
+                                40 * (size_t)(p.face_off[b + 1] - p.face_off[b]));
+    if (!opt.strict && own > kDfMaxSmem) return;
     std::vector<int> df = p.dep_face, dc = p.dep_cell;
     if (df.empty()) df.push_back(0);
     if (dc.empty()) dc.push_back(0);
@@ -741,14 +751,7 @@ void Solver::build_dataflow(const HostMesh& hm, int sms) {
     dfp.prog = dalloc<unsigned int>((size_t)nb * kDfProgStride, owned);
     dfp.wpart = dalloc<double>((size_t)dfp.max_steps * Wn * 4, owned);
     dfp.n_warps = Wn;
-    // The shared-memory form where every block's cells (96 bytes each) and
-    // their faces (40) fit: up to about 1,100 cells a block, 170k a mesh.
-    // Larger meshes keep their states in L2 and are bound by the work itself.
     dfp.smem = 0;
-    size_t own = 0;
-    for (int b = 0; b < nb; ++b)
-        own = std::max(own, 96 * (size_t)(p.cell_off[b + 1] - p.cell_off[b]) +
-                                40 * (size_t)(p.face_off[b + 1] - p.face_off[b]));
     if (own <= kDfMaxSmem) {
         std::vector<int> block_of(N), mail_of(N, -1), off(nb + 1, 0), xf, fin(nb, 0), slot(hm.d_cf.size(), -1), place(F);
         std::vector<int2> xc;
@@ -795,6 +798,7 @@ void Solver::build_dataflow(const HostMesh& hm, int sms) {
             dfp.mail = dalloc<double2>(16 * (size_t)std::max(n_mail, 1), owned);
         }
     }
+    if (!opt.strict && !dfp.smem) return;
     df_grid = nb;
     dataflow_ok = true;
 }
@@ -814,12 +818,14 @@ void Solver::launch_steps(int k, std::vector<int>* classes, std::vector<cudaEven
     // The error flag is cleared once per fv_step (reset_wait_error), so
     // that a wait that ran out in an early launch is still reported.
     const O1Args a = o1_args();
-    const bool df = persistent_form() == 2;
+    const bool df = persistent_form() == 2, split = split_form();
     for (int done = 0; done < k;) {
         const int n = df ? std::min(k - done, dfp.max_steps) : k;
         FV_CUDA(cudaMemsetAsync(pctl, 0, sizeof(int), stream));
         cudaError_t rc;
-        if (df)
+        if (split)
+            rc = fast::launch_o1_split(a, Pc, pctl, n, stream);
+        else if (df)
             rc = opt.strict ? strict::launch_o1_dataflow(a, Pc, pctl, dfp, n, df_grid, stream)
                             : fast::launch_o1_dataflow(a, Pc, pctl, dfp, n, df_grid, stream);
         else
@@ -851,6 +857,12 @@ void Solver::set_wait_limit(long long cycles, int phantom) {
     FV_CUDA(cudaStreamSynchronize(stream));
     h2d_sync(reinterpret_cast<char*>(pctl) + offsetof(PersistCtl, phantom), &phantom, sizeof(int), stream);
     h2d_sync(reinterpret_cast<char*>(pctl) + offsetof(PersistCtl, limit), &cycles, sizeof(long long), stream);
+    const bool set = cycles != kDefaultWaitCycles || phantom != 0;
+    if (set != wait_limit_set) {
+        for (auto& kv : graphs) cudaGraphExecDestroy(kv.second);
+        graphs.clear();
+    }
+    wait_limit_set = set;
 }
 
 void Solver::reset_wait_error() {
@@ -926,7 +938,7 @@ void Solver::step_async(int n) {
         return;
     }
     if (persistent) reset_wait_error();
-    const int chunk = persistent ? kPersistChunk : kGraphChunk;
+    const int chunk = persistent && !split_form() ? kPersistChunk : kGraphChunk;
     int q = n / chunk, r = n % chunk;
     if (q) {
         cudaGraphExec_t ge = graph_for(chunk);

@@ -138,6 +138,10 @@ struct Solver {
     // barriers, one block per SM (DfPlan).  Used unless barrier_form.
     bool dataflow_ok = false;
     bool barrier_form = false;
+    // The default build runs the barrier form's phases as launches of their
+    // own, unless set_persistent asked for that form or a wait limit is set.
+    bool wait_limit_set = false;
+    bool split_form() const { return persistent && !opt.strict && persistent_form() == 1 && !barrier_form && !wait_limit_set; }
     int df_grid = 0;
     DfPlan dfp{};
     static constexpr int kPersistChunk = 256;

@@ -377,8 +377,9 @@ class EulerFVMSolver:
     def set_persistent(self, on=True) -> None:
         """First-order forward-Euler FP64 path: one persistent cooperative
         launch per chunk of steps (on, the default where supported; with
-        local dt in its dataflow form), two kernels per step (off), or
-        ``"barrier"`` for the grid-barrier form of the persistent kernel."""
+        local dt in its dataflow form, else as the grid-barrier form, whose
+        phases the default build launches one by one), two kernels per step
+        (off), or ``"barrier"`` for the grid-barrier form in one launch."""
         mode = 2 if on == "barrier" else (1 if on else 0)
         capi.check(capi.lib().fv_solver_set_persistent(self._h, mode))
 

@@ -245,8 +245,11 @@ int fv_solver_set_launch(fv_solver_t s, const int32_t blocks[3]);
  * supports cooperative launch; on = 0 selects the two-kernel path.  With
  * local time stepping the kernel runs in a dataflow form: one block per SM
  * owns a range of cells, and each phase waits only for the blocks it shares
- * faces with instead of for the whole grid (same results again); on = 2
- * keeps the grid-barrier form.  fv_solver_persistent reports the form in
+ * faces with instead of for the whole grid (same results again), on meshes
+ * whose cells and fluxes fit in the SMs' shared memory (about 170k cells;
+ * strict mode: any).  Elsewhere the default build runs the phases of the
+ * grid-barrier form as launches of their own while no wait limit is set;
+ * on = 2 keeps the one launch.  fv_solver_persistent reports the form in
  * use (0 two-kernel path, 1 grid-barrier form, 2 dataflow form) and its
  * grid size (either pointer may be NULL).  No reference counterpart (the
  * reference's loops are OpenMP). */
