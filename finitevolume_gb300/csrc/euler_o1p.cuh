@@ -245,10 +245,10 @@ __device__ __forceinline__ void ghost_p(const BCTable& bc, const double* fsp, in
 #endif
 
 // One face of the face phase: its flux times the face length and, in dt, with
-// local dt lambda * length, else the face's global-dt candidate cfl * (CFL
-// length) / max(|Vn| + c).  UR, PR: the right cell of an internal face (a
+// MODE 1 (local dt) lambda * length, 0 the face's global-dt candidate cfl * (CFL
+// length) / lambda, 2 lambda = max(|Vn| + c) itself.  UR, PR: the right cell of an internal face (a
 // boundary face's ghost is formed here).
-template <int FLUX, bool LOCAL>
+template <int FLUX, int MODE>
 __device__ __forceinline__ St face_compute(const O1Args& a, int f, bool interior, const double4_32a& geo, const St& UL,
                                            const Prim& PL, St UR, Prim PR, double g, double cfl, double& dt) {
     if (!interior) {
@@ -267,14 +267,14 @@ __device__ __forceinline__ St face_compute(const O1Args& a, int f, bool interior
         double lam;
         if (fvfix::flux<FLUX == FLUX_HLLC ? 1 : 0, true, true>(L4, R4, PL.c, PR.c, UL, UR, geo.x, geo.y, geo.z, a.fxc,
                                                                F, interior, lam)) {
-            dt = LOCAL ? lam * geo.z : cfl * geo.w * fvconv::rcp_nr3(lam);
+            dt = MODE == 2 ? lam : MODE == 1 ? lam * geo.z : cfl * geo.w * fvconv::rcp_nr3(lam);
             return st_make(F.r, F.u, F.v, F.p);
         }
     }
 #endif
     const St Fl = num_flux_p<FLUX>(UL, PL, UR, PR, geo.x, geo.y, g, a.exact_tol, a.exact_max_iter);
     const double Smax = face_smax_p(PL, PR, interior, geo.x, geo.y);
-    dt = LOCAL ? Smax * geo.z : cfl * geo.w / Smax;
+    dt = MODE == 2 ? Smax : MODE == 1 ? Smax * geo.z : cfl * geo.w / Smax;
     return geo.z * Fl;
 }
 
@@ -936,8 +936,8 @@ static cudaError_t launch_o1df(const O1Args& a, double4_32a* P, PersistCtl* pc, 
 // the neighbouring faces, and the norms' fold runs beside a face pass.  Same
 // arithmetic, tiles and folds as the barrier form's.
 //
-// Bound: FP64 issue and latency (HLLC, global dt, us a step): 500k cells 82
-// (barrier form 108), 131k 26 (43), 32k 15 (20), 2k 12 (15, launches and the
+// Bound: FP64 issue and latency (HLLC, global dt, us a step): 500k cells 79
+// (barrier form 108), 131k 25 (43), 32k 14 (20), 2k 12 (16, launches and the
 // farfield's chain).  64 registers for Rusanov, 84 for the others, which spill
 // at 64 (HLLC 1.13 ms for 40 steps of 131k cells at 84, 1.21 at 64, 1.20 at 128).
 __device__ __forceinline__ Prim ld_prim_l1(const double4_32a* P, int i) {
@@ -968,27 +968,17 @@ __global__ void __launch_bounds__(fvgb::kCellBlock, FLUX == FLUX_RUSANOV ? 4 : 3
     }
     // from the last face down: the boundary faces have the longest chains
     const int f = F - 1 - (int)((blockIdx.x - folds) * blockDim.x + threadIdx.x);
-    double cand = DBL_MAX;
+    double dt = 0.0, len = 0.0;
     if (f >= 0) {
         const int L = a.m.fl[f], R = a.m.fr[f], Rs = R >= 0 ? R : L;
-        double dt;
-        const St Fl = face_compute<FLUX, LOCAL>(a, f, R >= 0, a.m.fgeom[f], ld_state(a.U, L), ld_prim_l1(P, L),
-                                                ld_state(a.U, Rs), ld_prim_l1(P, Rs), a.gamma, a.ctl->cfl, dt);
+        const double4_32a geo = a.m.fgeom[f];
+        const St Fl = face_compute<FLUX, LOCAL ? 1 : 2>(a, f, R >= 0, geo, ld_state(a.U, L), ld_prim_l1(P, L),
+                                                        ld_state(a.U, Rs), ld_prim_l1(P, Rs), a.gamma, 0.0, dt);
         st_state(a.ff, f, Fl);
         if (LOCAL) a.dtf[f] = dt;
-        else cand = dt;
+        len = geo.w;
     }
-    if (!LOCAL) {
-        __shared__ double smin[fvgb::kCellBlock / 32];
-        cand = warp_min_pos(cand);
-        if ((threadIdx.x & 31) == 0) smin[threadIdx.x >> 5] = cand;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double v = smin[0];
-            for (int w = 1; w < (int)(blockDim.x >> 5); ++w) v = fmin(v, smin[w]);
-            atomicMin(&pc->dt_slot[s & 1], (unsigned long long)__double_as_longlong(v));
-        }
-    }
+    if (!LOCAL) block_min_step(f >= 0, dt, len, a.ctl->cfl, &pc->dt_slot[s & 1]);
 }
 
 template <bool LOCAL>
