@@ -734,21 +734,11 @@ void Solver::build_dataflow(const HostMesh& hm, int sms) {
         own = std::max(own, 96 * (size_t)(p.cell_off[b + 1] - p.cell_off[b]) +
                                 40 * (size_t)(p.face_off[b + 1] - p.face_off[b]));
     if (!opt.strict && own > kDfMaxSmem) return;
-    std::vector<int> df = p.dep_face, dc = p.dep_cell;
-    if (df.empty()) df.push_back(0);
-    if (dc.empty()) dc.push_back(0);
-    dfp.faces = dupload(p.faces, owned);
-    dfp.face_off = dupload(p.face_off, owned);
     dfp.cell_off = dupload(p.cell_off, owned);
-    dfp.dep_face = dupload(df, owned);
-    dfp.dep_face_off = dupload(p.dep_face_off, owned);
-    dfp.dep_cell = dupload(dc, owned);
-    dfp.dep_cell_off = dupload(p.dep_cell_off, owned);
     // the per-warp partials of every step of a launch: up to kPersistChunk
     // steps, fewer on a large mesh (kDfPartialBytes)
     const size_t per_step = (size_t)Wn * 4 * sizeof(double);
     dfp.max_steps = (int)std::max<size_t>(8, std::min<size_t>(kPersistChunk, kDfPartialBytes / per_step));
-    dfp.prog = dalloc<unsigned int>((size_t)nb * kDfProgStride, owned);
     dfp.wpart = dalloc<double>((size_t)dfp.max_steps * Wn * 4, owned);
     dfp.n_warps = Wn;
     dfp.smem = 0;
@@ -789,16 +779,34 @@ void Solver::build_dataflow(const HostMesh& hm, int sms) {
         if (smem <= kDfMaxSmem && (opt.strict ? strict::o1df_sm_max_blocks_per_sm(opt.flux, smem)
                                               : fast::o1df_sm_max_blocks_per_sm(opt.flux, smem)) >= 1) {
             dfp.smem = smem;
-            dfp.xface_off = dupload(off, owned);
-            dfp.xfaces = dupload(xf, owned);
-            dfp.xcells = dupload(xc, owned);
-            dfp.face_in = dupload(fin, owned);
-            dfp.mail_of = dupload(mail_of, owned);
-            dfp.slot = dupload(slot, owned);
+            // one upload; the pairs first, for their alignment
+            std::vector<int> all;
+            all.reserve(2 * xc.size() + off.size() + xf.size() + fin.size() + mail_of.size() + slot.size());
+            for (const int2& q : xc) { all.push_back(q.x); all.push_back(q.y); }
+            for (const std::vector<int>* v : {&off, &xf, &fin, &mail_of, &slot}) all.insert(all.end(), v->begin(), v->end());
+            const int* d = dupload(all, owned);
+            dfp.xcells = reinterpret_cast<const int2*>(d);
+            dfp.xface_off = d + 2 * xc.size();
+            dfp.xfaces = dfp.xface_off + off.size();
+            dfp.face_in = dfp.xfaces + xf.size();
+            dfp.mail_of = dfp.face_in + fin.size();
+            dfp.slot = dfp.mail_of + mail_of.size();
             dfp.mail = dalloc<double2>(16 * (size_t)std::max(n_mail, 1), owned);
         }
     }
-    if (!opt.strict && !dfp.smem) return;
+    if (!dfp.smem) {
+        if (!opt.strict) return;
+        std::vector<int> df = p.dep_face, dc = p.dep_cell;
+        if (df.empty()) df.push_back(0);
+        if (dc.empty()) dc.push_back(0);
+        dfp.faces = dupload(p.faces, owned);
+        dfp.face_off = dupload(p.face_off, owned);
+        dfp.dep_face = dupload(df, owned);
+        dfp.dep_face_off = dupload(p.dep_face_off, owned);
+        dfp.dep_cell = dupload(dc, owned);
+        dfp.dep_cell_off = dupload(p.dep_cell_off, owned);
+        dfp.prog = dalloc<unsigned int>((size_t)nb * kDfProgStride, owned);
+    }
     df_grid = nb;
     dataflow_ok = true;
 }
