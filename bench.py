@@ -1038,9 +1038,10 @@ def main():
             "kernel_ms_per_step": {k: round(m / args.steps, 4) for k, m in zip(roofline.KERNEL_NAMES, ms)},
             "stage": {"survey_bytes_B2": stage_alg, "ms": round(stage_ms, 4),
                       "achieved_GBs": round(stage_alg / (stage_ms / 1e3) / 1e9, 1)}}
-    # What actually bounds it: FP64-pipe issue (ncu instruction count per
-    # cell of this kernel x cells / live launch time, against the GB300
-    # DFMA rate of 0.51e12 thread instructions/s measured on the box).
+    # The FP64 pipe's share (ncu instruction count per cell of this kernel x
+    # cells / live launch time, against the GB300 DFMA rate of 0.51e12 thread
+    # instructions/s): no longer the bound of the gradient and face passes,
+    # whose arithmetic runs on the integer pipe.
     inst = roofline.MEASURED_FP64_INST_PER_CELL.get(kname)
     if inst is not None:
         ach_inst = inst * n_cells / (per_launch_ms / 1e3) / 1e9

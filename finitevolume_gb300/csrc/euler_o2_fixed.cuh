@@ -4,10 +4,10 @@
 // ranges of the fixed-point one.
 //
 // Measured on the GB300 (1.05M-cell O-grid, Venkatakrishnan, HLLC, time per
-// launch): gradients and limiter 417 us in FP64 (the FP64 pipe 86% busy), 165
-// here; face fluxes 387 us in FP64 (88% busy), 87 here.  On 2k cells, where a
+// launch): gradients and limiter 417 us in FP64 (the FP64 pipe 86% busy), 146
+// here; face fluxes 387 us in FP64 (88% busy), 81 here.  On 2k cells, where a
 // launch is one wave and the length of a thread's dependent chain counts
-// (FP64 64 clocks an operation, integers 5 to 13), 32 and 21 us became 12
+// (FP64 64 clocks an operation, integers 5 to 13), 32 and 21 us became 10
 // and 8.5.  Errors against 128-bit arithmetic are no larger than the FP64
 // forms' (tests/cuda/fixed_check.cu).
 #pragma once
@@ -321,7 +321,9 @@ __device__ __noinline__ V4<double> face_flux_f64(const V4<double>& L, const V4<d
 
 // Face fluxes, one thread per face; blocks take the faces from the last one
 // down, so that the boundary faces (FP64 ghost states, the longest chains)
-// start first.
+// start first.  Bound by integer issue and latency (ALU 70%, issue 60%): 64
+// registers for 32 warps an SM (72 registers, 24 warps: 84 us for 81, with
+// the local time step 111 for 92).
 template <int FLUX, int ORDER, int DT>
 __global__ void __launch_bounds__(fvgb::kMaxBlock, 2) k_face_fx(const O2Args a) {
     const int f = (gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x;

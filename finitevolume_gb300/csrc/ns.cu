@@ -48,8 +48,11 @@ __device__ __forceinline__ double boundary_field(const NSArgs& a, int face, int 
 }
 
 #ifdef FV_NS_FAST
-// Default build (viscous_fast.cuh).  Bound: FP64 issue, about 75 instructions
-// a face (370 in the strict order), 55 a cell for the gradients (155).
+// Default build (viscous_fast.cuh).  Bound: FP64 issue (73% busy), 73
+// instructions a face (370 in the strict order), 48 a cell for the gradients
+// (155), 14 for the cell pass.  130k cells: face pass 45.5 us, gradients 17,
+// cell pass 13, primitives 6 (a step 258 us with the strict order's
+// operations contracted, 77 so).
 __global__ void __launch_bounds__(fvgb::kCellBlock) k_ns_prim(const NSArgs a) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= a.g.n_cells) return;

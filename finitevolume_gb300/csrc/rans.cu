@@ -49,9 +49,10 @@ __device__ __forceinline__ double sa_fv1(double nut, double nu, const double* c)
 __device__ __forceinline__ double sa_nut(double nut, double nu, const double* c) { return nut * sa_fv1(nut, nu, c); }
 
 #ifdef FV_NS_FAST
-// Default build (viscous_fast.cuh).  Bound: FP64 issue, about 105
-// instructions a face (430 in the strict order), 65 a cell for the gradients
-// (155), 90 for the cell pass (245), 27 for the primitives (67).
+// Default build (viscous_fast.cuh).  Bound: FP64 issue (76 to 82% busy), 100
+// instructions a face (430 in the strict order), 49 a cell for the gradients
+// (155), 74 for the cell pass (245), 24 for the primitives (67).  245k cells:
+// 79, 28, 53 and 15 us.
 
 // nu_t = nut fv1(chi) with chi = nut / nu
 __device__ __forceinline__ double sa_fv1_chi(double chi, double cv1_3) {

@@ -60,18 +60,16 @@ KERNEL_NAMES = ("gradients", "faces", "update")
 # DRAM bytes per cell per launch measured by ncu (dram__bytes_read.sum +
 # dram__bytes_write.sum, one launch of each kernel class) on the 968,907-cell
 # NACA0012 mixed mesh; the captures are summarised under profiles/.  In
-# FP64 the gradient pass writes the per-entry limiter increments that the
-# face pass reads (32 B per entry each way), which puts both above their
-# algorithmic bytes on purpose: the FP64 kernels are bound by FP64 issue,
-# not by DRAM, and the increments save the face pass one multiply-add per
-# variable and side.
-MEASURED_TRAFFIC_PER_CELL = {"gradients": 382.0, "faces": 401.3, "update": 207.2}
-MEASURED_TRAFFIC_PER_CELL_FP32 = {"gradients": 146.3, "faces": 165.1, "update": 147.7}
+# FP64 the gradient pass writes each cell face's reconstructed state (32 B per
+# entry), which the face pass reads instead of the cells' states and gradients.
+MEASURED_TRAFFIC_PER_CELL = {"gradients": 386.4, "faces": 314.2, "update": 223.7}
+MEASURED_TRAFFIC_PER_CELL_FP32 = {"gradients": 144.2, "faces": 166.8, "update": 151.5}
 
 # FP64-pipe thread instructions per cell and per launch from the same
-# captures (smsp__inst_executed_pipe_fp64.sum x 32 / cells).  On GB300 the
-# FP64 pipe, not HBM, bounds the FP64 kernels.
-MEASURED_FP64_INST_PER_CELL = {"gradients": 236.4, "faces": 232.0, "update": 44.4}
+# captures (smsp__inst_executed_pipe_fp64.sum x 32 / cells).  The gradient and
+# face passes run on the integer pipe (fixed.cuh) and are bound by its issue and
+# by latency; the update is bound by the FP64 pipe (72% busy).
+MEASURED_FP64_INST_PER_CELL = {"gradients": 21.3, "faces": 19.8, "update": 33.2}
 
 
 def measured_traffic(kind: str, n_cells: int, fp32: bool = False):
