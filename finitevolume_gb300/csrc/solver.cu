@@ -664,13 +664,14 @@ bool dataflow_plan(const HostMesh& hm, const int* patch_type, int sms, DataflowP
     std::vector<double> wsum(Wn + 1, 0.0);
     {
         std::vector<char> far(Wn, 0);
-        for (int f = 0; f < F; ++f)
-            if (hm.d_fr[f] < 0 && patch_type[hm.d_fpatch[f]] == FV_BC_CHAR_FARFIELD) far[hm.d_fl[f] / 32] = 1;
+        for (int f = hm.n_int_faces; f < F; ++f)
+            if (patch_type[hm.d_fpatch[f]] == FV_BC_CHAR_FARFIELD) far[hm.d_fl[f] / 32] = 1;
         for (int w = 0; w < Wn; ++w) wsum[w + 1] = wsum[w] + (far[w] ? 1.7 : 1.0);
     }
     p.nb = nb;
     p.cell_off.assign(nb + 1, 0);
-    std::vector<int> owner(N);
+    std::vector<int>& owner = p.owner;
+    owner.resize(N);
     for (int b = 0; b <= nb; ++b) {
         const int w = b == nb ? Wn
                               : (int)(std::lower_bound(wsum.begin(), wsum.end(), wsum[Wn] * b / nb) - wsum.begin());
@@ -687,13 +688,11 @@ bool dataflow_plan(const HostMesh& hm, const int* patch_type, int sms, DataflowP
     for (int b = 0; b < nb; ++b) p.face_off[b + 1] += p.face_off[b];
     {
         std::vector<int> pos(p.face_off.begin(), p.face_off.end() - 1);
-        for (int pass = 0; pass < 2; ++pass)
-            for (int f = 0; f < F; ++f)
-                if ((hm.d_fr[f] < 0) == (pass == 0)) p.faces[pos[owner[hm.d_fl[f]]]++] = f;
+        for (int f = hm.n_int_faces; f < F; ++f) p.faces[pos[owner[hm.d_fl[f]]]++] = f;
+        for (int f = 0; f < hm.n_int_faces; ++f) p.faces[pos[owner[hm.d_fl[f]]]++] = f;
     }
     std::vector<std::vector<int>> dface(nb), dcell(nb);
-    for (int f = 0; f < F; ++f) {
-        if (hm.d_fr[f] < 0) continue;
+    for (int f = 0; f < hm.n_int_faces; ++f) {
         const int a = owner[hm.d_fl[f]], r = owner[hm.d_fr[f]];
         if (a == r) continue;
         dface[a].push_back(r);  // a's face phase reads r's cells
@@ -743,54 +742,63 @@ void Solver::build_dataflow(const HostMesh& hm, int sms) {
     dfp.n_warps = Wn;
     dfp.smem = 0;
     if (own <= kDfMaxSmem) {
-        std::vector<int> block_of(N), mail_of(N, -1), off(nb + 1, 0), xf, fin(nb, 0), slot(hm.d_cf.size(), -1), place(F);
-        std::vector<int2> xc;
-        for (int b = 0; b < nb; ++b)
-            for (int c = p.cell_off[b]; c < p.cell_off[b + 1]; ++c) block_of[c] = b;
-        int n_mail = 0;
-        auto between = [&](int f) { return hm.d_fr[f] >= 0 && block_of[hm.d_fl[f]] != block_of[hm.d_fr[f]]; };
-        for (int f = 0; f < F; ++f)
-            if (between(f))
-                for (int c : {hm.d_fl[f], hm.d_fr[f]})
-                    if (mail_of[c] < 0) mail_of[c] = n_mail++;
+        const std::vector<int>& block_of = p.owner;
+        // faces between blocks, and a mailbox for each of their cells
+        std::vector<unsigned char> between(F, 0);
+        std::vector<int> place(F);
+        const size_t E = hm.d_cf.size();
+        int n_mail = 0, n_between = 0;
+        std::vector<int> mail(N, -1);
+        for (int f = 0; f < hm.n_int_faces; ++f) {
+            const int l = hm.d_fl[f], r = hm.d_fr[f];
+            if (block_of[l] == block_of[r]) continue;
+            between[f] = 1;
+            ++n_between;
+            if (mail[l] < 0) mail[l] = n_mail++;
+            if (mail[r] < 0) mail[r] = n_mail++;
+        }
+        // all lists in one upload, the pairs first for their alignment
+        const size_t nx = (size_t)F + n_between, n_all = 3 * nx + (nb + 1) + nb + N + E;
+        std::unique_ptr<int[]> all(new int[n_all]);
+        int2* xc = reinterpret_cast<int2*>(all.get());
+        int *off = all.get() + 2 * nx, *xf = off + nb + 1, *fin = xf + nx, *mail_of = fin + nb, *slot = mail_of + N;
+        std::memcpy(mail_of, mail.data(), sizeof(int) * N);
+        off[0] = 0;
         size_t smem = 0;
         for (int b = 0; b < nb; ++b) {
             const int c0 = p.cell_off[b], c1 = p.cell_off[b + 1];
+            int at = off[b];
             // the plan's own faces in its order (boundary faces first), then
             // those between blocks, owned or not, as this block's cells list them
             auto add = [&](int f) {
-                place[f] = (int)xf.size() - off[b];
-                xf.push_back(f);
+                place[f] = at - off[b];
+                xf[at] = f;
                 auto code = [&](int c) {
-                    return c < 0 ? INT_MIN : (block_of[c] == b ? c - c0 : -1 - mail_of[c]);
+                    return c < 0 ? INT_MIN : ((unsigned)(c - c0) < (unsigned)(c1 - c0) ? c - c0 : -1 - mail[c]);
                 };
-                xc.push_back(make_int2(code(hm.d_fl[f]), code(hm.d_fr[f])));
+                xc[at++] = make_int2(code(hm.d_fl[f]), code(hm.d_fr[f]));
             };
             for (int j = p.face_off[b]; j < p.face_off[b + 1]; ++j)
-                if (!between(p.faces[j])) add(p.faces[j]);
-            fin[b] = (int)xf.size() - off[b];
-            for (int c = c0; c < c1; ++c)
-                for (int e = hm.d_cf_off[c]; e < hm.d_cf_off[c + 1]; ++e)
-                    if (between(hm.d_cf[e] >> 1)) add(hm.d_cf[e] >> 1);
-            off[b + 1] = (int)xf.size();
-            for (int e = hm.d_cf_off[c0]; e < hm.d_cf_off[c1]; ++e) slot[e] = place[hm.d_cf[e] >> 1];
+                if (!between[p.faces[j]]) add(p.faces[j]);
+            fin[b] = at - off[b];
+            const int e0 = hm.d_cf_off[c0], e1 = hm.d_cf_off[c1];
+            for (int e = e0; e < e1; ++e)
+                if (between[hm.d_cf[e] >> 1]) add(hm.d_cf[e] >> 1);
+            off[b + 1] = at;
+            for (int e = e0; e < e1; ++e) slot[e] = place[hm.d_cf[e] >> 1];
             smem = std::max(smem, 96 * (size_t)(c1 - c0) + 40 * (size_t)(off[b + 1] - off[b]));
         }
         if (smem <= kDfMaxSmem && (opt.strict ? strict::o1df_sm_max_blocks_per_sm(opt.flux, smem)
                                               : fast::o1df_sm_max_blocks_per_sm(opt.flux, smem)) >= 1) {
             dfp.smem = smem;
-            // one upload; the pairs first, for their alignment
-            std::vector<int> all;
-            all.reserve(2 * xc.size() + off.size() + xf.size() + fin.size() + mail_of.size() + slot.size());
-            for (const int2& q : xc) { all.push_back(q.x); all.push_back(q.y); }
-            for (const std::vector<int>* v : {&off, &xf, &fin, &mail_of, &slot}) all.insert(all.end(), v->begin(), v->end());
-            const int* d = dupload(all, owned);
+            int* d = dalloc<int>(n_all, owned);
+            h2d_sync(d, all.get(), sizeof(int) * n_all);
             dfp.xcells = reinterpret_cast<const int2*>(d);
-            dfp.xface_off = d + 2 * xc.size();
-            dfp.xfaces = dfp.xface_off + off.size();
-            dfp.face_in = dfp.xfaces + xf.size();
-            dfp.mail_of = dfp.face_in + fin.size();
-            dfp.slot = dfp.mail_of + mail_of.size();
+            dfp.xface_off = d + (off - all.get());
+            dfp.xfaces = d + (xf - all.get());
+            dfp.face_in = d + (fin - all.get());
+            dfp.mail_of = d + (mail_of - all.get());
+            dfp.slot = d + (slot - all.get());
             dfp.mail = dalloc<double2>(16 * (size_t)std::max(n_mail, 1), owned);
         }
     }

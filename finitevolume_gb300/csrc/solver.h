@@ -46,6 +46,7 @@ struct MGLevel {
 struct DataflowPlan {
     int nb = 0;
     std::vector<int> cell_off, face_off, faces, dep_face_off, dep_face, dep_cell_off, dep_cell;
+    std::vector<int> owner;  // block of each cell
 };
 // Builds the plan over min(sms, cell warps) blocks; patch_type[p] is the
 // FV_BC_* of patch p.  False when a block would wait for more than
