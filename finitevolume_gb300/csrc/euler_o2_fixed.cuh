@@ -297,7 +297,8 @@ __device__ __forceinline__ void grad_lane(const O2Args& a, int c, int k, int e0,
 template <int LIM>
 __global__ void __launch_bounds__(fvgb::kMaxBlock, 2) k_grad_fx(const O2Args a) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int c = t >> 2, k = t & 3;
+    if ((t >> 7) * 32 >= a.m.n_cells) return;
+    const int c = (a.tile_order ? a.tile_order[t >> 7] * 32 : (t >> 7) * 32) + ((t & 127) >> 2), k = t & 3;
     if (c >= a.m.n_cells) return;
     // The geometry is read behind the neighbours' values and between long
     // stretches of arithmetic, with no registers to hold it earlier: the lanes

@@ -280,6 +280,25 @@ void Solver::init(const HostMesh& hm, const fv_bc_t* bcs, int n_bcs, double g, d
             fxa = dalloc<int4>(h2.d_cf.size(), owned);
             fxr = dalloc<int4>(h2.d_cf.size(), owned);
             fxs = dalloc<int>(N, owned);
+            // With polygons: the tiles that hold them (loops over five to nine
+            // faces), first those with boundary faces (a ghost's FP64 chain), before
+            // the others, so that the last wave does not end on the tiles that take
+            // two to three times as long.  Gradient pass, mixed cells: 61k 32 -> 28
+            // us, 242k 82 -> 77, 969k 276 -> 264; on quads or triangles alone the
+            // same order by boundary faces measured 1% slower.
+            std::vector<int> order[3];
+            for (int t = 0; t < (N + 31) / 32; ++t) {
+                bool poly = false, bnd = false;
+                for (int c = 32 * t; c < std::min(N, 32 * t + 32); ++c) {
+                    poly |= hm.d_cf_off[c + 1] - hm.d_cf_off[c] > 4;
+                    for (int e = hm.d_cf_off[c]; e < hm.d_cf_off[c + 1]; ++e) bnd |= (hm.d_cf[e] >> 1) >= hm.n_int_faces;
+                }
+                order[poly ? (bnd ? 0 : 1) : 2].push_back(t);
+            }
+            if (!order[0].empty() || !order[1].empty()) {
+                for (int k : {1, 2}) order[0].insert(order[0].end(), order[k].begin(), order[k].end());
+                tile_order = dupload(order[0], owned);
+            }
             refresh_fixed_geometry();
         }
     }
@@ -576,6 +595,7 @@ O2Args Solver::o2_args() const {
     a.fxa = fxa;
     a.fxr = fxr;
     a.fxs = fxs;
+    a.tile_order = tile_order;
     a.fxc = flux_const();
     a.fsp = fsp;
     return a;

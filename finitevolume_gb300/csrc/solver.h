@@ -119,6 +119,7 @@ struct Solver {
     const float4* fgeom32 = nullptr;
     const St* forcing = nullptr;    // multigrid coarse levels: FAS forcing term
     void* psi_buf = nullptr;        // frozen limiter values [4N], flux precision
+    int* tile_order = nullptr;      // O2Args::tile_order
     St* wf = nullptr;               // FP64 with a limiter: per-entry face states [E] (O2Args::wf)
     int2* fe = nullptr;             //   owner / neighbour entry per face [F]
     int fixed = 0;                  // fixed-point passes (O2Args::fixed) and their geometry

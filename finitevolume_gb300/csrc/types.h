@@ -197,6 +197,7 @@ struct O2Args {
     const int4* fxa;
     const int4* fxr;
     const int* fxs;
+    const int* tile_order;   // order of the gradient pass's 32-cell tiles, the longest first (null: as they are)
     fvfix::FluxConst fxc;
     // Farfield states for those passes: r, u, v, p, c, 1/c, 1/gamma, 0 per
     // patch (batched solves: per instance).
