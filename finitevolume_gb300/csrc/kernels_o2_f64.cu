@@ -14,7 +14,9 @@ void grad(const O2Args& a, int bs, cudaStream_t s) {
     // The adjoint's linearisation (wf null) takes its gradients from the FP64 pass.
     if constexpr (GRAD == 0 && LIM != 0) {
         if (a.fxs && a.wf) {
-            k_grad_fx<LIM><<<(4LL * a.m.n_cells + bs - 1) / bs, bs, 0, s>>>(a);  // four lanes per cell
+            // four lanes per cell; with an order whole tiles, wherever the ragged one stands
+            const long long lanes = a.tile_order ? (a.m.n_cells + 31LL) / 32 * 128 : 4LL * a.m.n_cells;
+            k_grad_fx<LIM><<<(int)((lanes + bs - 1) / bs), bs, 0, s>>>(a);
             return;
         }
     }

@@ -1,4 +1,4 @@
-"""Edges of two work splits.
+"""Edges of three work splits.
 
 - The shared-memory dataflow form on meshes of one to four blocks: one block
   without a mailbox (32 cells), blocks with a ragged last warp (36, 72), against
@@ -7,6 +7,9 @@
 - The batched norms' chunks of 1,024 cells: instances of a multiple of it, a few
   below, a few above, and one small, against the standalone solver's norms
   (1e-12: sums of at most 2,048 squares, 2048 * 2^-53 on either side).
+- The gradient pass's order of tiles on a mesh with polygons, whose last tile is
+  ragged, under launch shapes that are and are not multiples of a tile's 128
+  lanes: every cell is served, so fields are the same bits.
 """
 import numpy as np
 import pytest
@@ -41,6 +44,23 @@ def test_shared_memory_form_on_few_blocks(gpu, size, flux, strict):
         else:
             assert rel_err(a.field(), b.field()) <= 1e-13
             np.testing.assert_allclose(ha, hb, rtol=1e-13, atol=0)
+
+
+def test_tile_order_serves_every_cell_at_any_launch_shape(gpu):
+    poly = meshgen.naca_mixed(32, 16, seed=0)
+    assert poly.n_cells % 32 != 0
+    fs = _fs(0.5, 1.0)
+    bcs = [S.EulerBoundaryCondition(S.EulerBoundaryType.Wall),
+           S.EulerBoundaryCondition(S.EulerBoundaryType.CharacteristicFarfield, S.from_primitive(*fs, GAMMA))]
+    ic = S.EulerInitialCondition(S.EulerICMode.Freestream, rho=fs[0], u=fs[1], v=fs[2], p=fs[3])
+    fields = []
+    for shape in (128, 160, 224, 480, 512):
+        s = S.EulerFVMSolver(S.Mesh(poly), bcs, GAMMA, 1.0, ic, S.NumericalFluxScheme.HLLC, order=2, rk_stages=3,
+                             local_dt=True)
+        s.set_launch(shape, 128, 128)
+        s.run(5)
+        fields.append(s.field())
+    assert all(np.array_equal(f, fields[0]) for f in fields[1:])
 
 
 def test_batched_norms_at_the_chunk_edges(gpu):
