@@ -134,6 +134,14 @@ static __device__ __noinline__ V4<double> ghost_more(const O2Args& a, int f, int
     return ghost_fast(a, f, c, WStore<double>::ld(static_cast<const St*>(a.W), c), q.x, q.y);
 }
 
+// Bitwise or over a quad, by two shuffles: a warp-wide reduction with a mask of
+// its own per quad runs once for each of the warp's eight quads (1.05M cells:
+// eight steps 7.35 -> 7.22 ms).
+__device__ __forceinline__ unsigned quad_or(unsigned quad, unsigned x) {
+    x |= __shfl_xor_sync(quad, x, 1, 4);
+    return x | __shfl_xor_sync(quad, x, 2, 4);
+}
+
 // One variable k of one cell.  The four lanes of a cell meet at the votes:
 // an FP64 cell is one for all its variables, and a face state that is not
 // positive falls back to the cell's.  N: the cell's face count (3 or 4, its
@@ -239,7 +247,7 @@ __device__ __forceinline__ void grad_lane(const O2Args& a, int c, int k, int e0,
         up = max(up, d);
         dn = min(dn, d);
     }
-    bad |= (over >> (27 - (S & 31))) != 0;  // an increment of 2^59 units or more
+    bad |= (over >> (27 - max(S, 0))) != 0;  // an increment of 2^59 units or more
     i64 psi;  // Q60
     if (a.psi_mode == 2) {
         psi = to_fixed<60>(static_cast<const double*>(a.psi_buf)[4 * (size_t)c + k], 1023);
@@ -266,7 +274,7 @@ __device__ __forceinline__ void grad_lane(const O2Args& a, int c, int k, int e0,
             inc[i] = w0 + mul<4>(split(inc[i]), p);
             if (!any_sign && inc[i] <= 0) flags |= 1u << i;
         }
-        flags = __reduce_or_sync(quad, flags);
+        flags = quad_or(quad, flags);
         if (flags >> 31) {
             if (k == 0) grad_cell_f64<LIM>(a, c, fs);
             return;
@@ -274,13 +282,13 @@ __device__ __forceinline__ void grad_lane(const O2Args& a, int c, int k, int e0,
 #pragma unroll
         for (int i = 0; i < N; ++i) out[4 * i] = flags >> i & 1 ? wc : to_double(inc[i], E - 1080);
     } else {
-        if (__reduce_or_sync(quad, bad)) {
+        if (quad_or(quad, bad)) {
             if (k == 0) grad_cell_f64<LIM>(a, c, fs);
             return;
         }
         for (int i = 0; i < n; ++i) {
             const i64 w = w0 + mul<4>(split(increment(e0 + i)), p);
-            const unsigned low = __reduce_or_sync(quad, (unsigned)(!any_sign && w <= 0));
+            const unsigned low = quad_or(quad, (unsigned)(!any_sign && w <= 0));
             out[4 * i] = low ? wc : to_double(w, E - 1080);
         }
     }
