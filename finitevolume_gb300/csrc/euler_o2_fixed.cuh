@@ -260,11 +260,15 @@ __device__ __forceinline__ void grad_lane(const O2Args& a, int c, int k, int e0,
         // double, which limiter freezing stores
         const bool lower = mul<3>(nd, du) < mul<3>(nu, dd);  // both below 16
         const i64 num = lower ? nd : nu, den = lower ? dd : du;
-        psi = num < den ? ratio52(num, den) : (i64)1 << 52;
-        if (a.psi_mode == 1) static_cast<double*>(a.psi_buf)[4 * (size_t)c + k] = to_double(psi, -52);
-        psi <<= 8;
+        psi = (num < den ? ratio52(num, den) : (i64)1 << 52) << 8;
     }
     const Sp p = split(psi);
+    // Captured once the quad has taken the cell: a declined cell's four values
+    // are all lane 0's, from the FP64 pass, and nothing orders another lane's
+    // store before them.
+    auto capture = [&]() {
+        if (a.psi_mode == 1) static_cast<double*>(a.psi_buf)[4 * (size_t)c + k] = to_double(psi, -60);
+    };
     const bool any_sign = k == 1 || k == 2;  // velocities; density and pressure must stay positive
     double* out = reinterpret_cast<double*>(a.wf) + 4 * (size_t)e0 + k;
     if constexpr (N != 0) {
@@ -279,6 +283,7 @@ __device__ __forceinline__ void grad_lane(const O2Args& a, int c, int k, int e0,
             if (k == 0) grad_cell_f64<LIM>(a, c, fs);
             return;
         }
+        capture();
 #pragma unroll
         for (int i = 0; i < N; ++i) out[4 * i] = flags >> i & 1 ? wc : to_double(inc[i], E - 1080);
     } else {
@@ -286,6 +291,7 @@ __device__ __forceinline__ void grad_lane(const O2Args& a, int c, int k, int e0,
             if (k == 0) grad_cell_f64<LIM>(a, c, fs);
             return;
         }
+        capture();
         for (int i = 0; i < n; ++i) {
             const i64 w = w0 + mul<4>(split(increment(e0 + i)), p);
             const unsigned low = quad_or(quad, (unsigned)(!any_sign && w <= 0));
