@@ -240,10 +240,12 @@ void Solver::init(const HostMesh& hm, const fv_bc_t* bcs, int n_bcs, double g, d
         // cubed in that precision).
         std::vector<double> e64(N);
         std::vector<float> e32(N);
+        bool eps2_ok = true;
         for (int c = 0; c < N; ++c) {
             const double kh = opt.venkat_k * h2.d_h[c];
             const float khf = (float)kh;
             e64[c] = kh * kh * kh;
+            eps2_ok = eps2_ok && e64[c] >= 0.0 && std::isfinite(e64[c]);
             e32[c] = khf * khf * khf;
         }
         // The per-entry / per-face reconstruction geometry is stored in the
@@ -276,7 +278,9 @@ void Solver::init(const HostMesh& hm, const fv_bc_t* bcs, int n_bcs, double g, d
         // limiter the least-squares gradients.
         fixed = !cfg.fp32 && cfg.flux != FV_FLUX_EXACT && fixed_gamma() && (cfg.order == 1 || cfg.limiter != 0);
         if (fixed) upload_farfield();
-        if (fixed && cfg.order == 2 && cfg.gradient == 0) {
+        // A negative or infinite eps^2 is the FP64 pass's, for all cells: the
+        // integers of the limiter's quotient have no sign for it.
+        if (fixed && cfg.order == 2 && cfg.gradient == 0 && (cfg.limiter != FV_LIM_VENKAT || eps2_ok)) {
             fxa = dalloc<int4>(h2.d_cf.size(), owned);
             fxr = dalloc<int4>(h2.d_cf.size(), owned);
             fxs = dalloc<int>(N, owned);

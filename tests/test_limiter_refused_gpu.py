@@ -71,3 +71,18 @@ def test_captured_values_of_declined_cells(gpu, limiter, big, tiny_v):
         psi = [np.delete(p, 2, axis=1) for p in psi]
     assert (psi[1] < 0.9).mean() > 0.2
     np.testing.assert_allclose(psi[0], psi[1], rtol=0, atol=1e-10)
+
+
+@pytest.mark.parametrize("k", [-1.0, -0.0, 0.0])
+def test_negative_and_zero_venkat_k(gpu, k):
+    """A negative K makes eps^2 = (K h)^3 negative, which only the FP64 pass forms.  With eps^2 about -1e-4 the
+    quotient's denominator comes near zero at a few cells: 1e-8 leaves it 2^-26 of the squared differences."""
+    poly = meshgen.cartesian(20, 20)
+    U = jumps(poly, 5)
+    psi = []
+    for flux in (S.NumericalFluxScheme.HLLC, S.NumericalFluxScheme.Exact):
+        s = solver(poly, flux, S.Limiter.Venkatakrishnan, venkat_k=k)
+        s.set_field(U)
+        s.freeze_limiter()
+        psi.append(s.limiter_values())
+    np.testing.assert_allclose(psi[0], psi[1], rtol=1e-8, atol=1e-8)
