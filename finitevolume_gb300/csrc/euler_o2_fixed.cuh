@@ -29,9 +29,10 @@ using fvfix::u64;
 // differences of at most d stay below d in the weights' units, an increment
 // below 2^S d.  fxs[c] = S, or -1 where the cell takes the FP64 pass: more
 // than 16 faces, S above 16, or a weight or offset that is not finite or out of
-// range.
+// range; *declined counts those.
 static __global__ void __launch_bounds__(256) k_fix_geom(const fvgb::O2Args a, int4* __restrict__ fxa,
-                                                         int4* __restrict__ fxr, int* __restrict__ fxs) {
+                                                         int4* __restrict__ fxr, int* __restrict__ fxs,
+                                                         int* __restrict__ declined = nullptr) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= a.m.n_cells) return;
     const double2* w = static_cast<const double2*>(a.lsq);
@@ -54,6 +55,7 @@ static __global__ void __launch_bounds__(256) k_fix_geom(const fvgb::O2Args a, i
     bool ok = e1 - e0 <= 16 && S <= 16 && isfinite(sx) && isfinite(sy) && isfinite(rx) && isfinite(ry);
     ok = ok && abs(ex) < 300 && abs(ey) < 300 && abs(px) < 300 && abs(py) < 300;
     fxs[c] = ok ? S : -1;
+    if (!ok && declined) atomicAdd(declined, 1);
     for (int e = e0; e < e1; ++e) {
         const Sp ax = split(ok ? llrint(ldexp(w[e].x, 62 - ex)) : 0), ay = split(ok ? llrint(ldexp(w[e].y, 62 - ey)) : 0);
         const Sp bx = split(ok ? llrint(ldexp(r[e].x, 61 - (S - ex))) : 0);

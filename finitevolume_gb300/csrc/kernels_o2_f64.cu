@@ -64,8 +64,8 @@ void launch_batch_norms(const O2Args& a, int n_inst, const BatchNorms& b, double
     }
 }
 
-void launch_fix_geom(const O2Args& a, int4* fxa, int4* fxr, int* fxs, cudaStream_t s) {
-    ::fast::k_fix_geom<<<(a.m.n_cells + 255) / 256, 256, 0, s>>>(a, fxa, fxr, fxs);
+void launch_fix_geom(const O2Args& a, int4* fxa, int4* fxr, int* fxs, int* declined, cudaStream_t s) {
+    ::fast::k_fix_geom<<<(a.m.n_cells + 255) / 256, 256, 0, s>>>(a, fxa, fxr, fxs, declined);
 }
 
 void launch_prim_f64(const O2Args& a, cudaStream_t s) {

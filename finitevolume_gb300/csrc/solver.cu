@@ -284,6 +284,7 @@ void Solver::init(const HostMesh& hm, const fv_bc_t* bcs, int n_bcs, double g, d
             fxa = dalloc<int4>(h2.d_cf.size(), owned);
             fxr = dalloc<int4>(h2.d_cf.size(), owned);
             fxs = dalloc<int>(N, owned);
+            fx_declined = dalloc<int>(1, owned);
             // With polygons: the tiles that hold them (loops over five to nine
             // faces), first those with boundary faces (a ghost's FP64 chain), before
             // the others, so that the last wave does not end on the tiles that take
@@ -598,7 +599,7 @@ O2Args Solver::o2_args() const {
     a.fixed = fixed;
     a.fxa = fxa;
     a.fxr = fxr;
-    a.fxs = fxs;
+    a.fxs = fx_grad ? fxs : nullptr;
     a.tile_order = tile_order;
     a.fxc = flux_const();
     a.fsp = fsp;
@@ -616,8 +617,22 @@ fvfix::FluxConst Solver::flux_const() const {
 
 void Solver::refresh_fixed_geometry() {
     if (!fxs) return;
-    o2::launch_fix_geom(o2_args(), fxa, fxr, fxs, stream);
+    int declined = 0;
+    FV_CUDA(cudaMemsetAsync(fx_declined, 0, sizeof(int), stream));
+    o2::launch_fix_geom(o2_args(), fxa, fxr, fxs, fx_declined, stream);
     FV_CUDA(cudaGetLastError());
+    FV_CUDA(cudaMemcpyAsync(&declined, fx_declined, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    FV_CUDA(cudaStreamSynchronize(stream));
+    // A declined cell is one lane's work of four in the fixed-point pass, so
+    // beyond an eighth of them all cells take the FP64 pass (262k cells, HLLC, us
+    // an iteration: none declined 238, an eighth 458, three sixteenths 552, all
+    // 1671; the FP64 pass for all 537).
+    const bool use = declined <= N / 8;
+    if (use != fx_grad) {
+        for (auto& kv : graphs) cudaGraphExecDestroy(kv.second);
+        graphs.clear();
+    }
+    fx_grad = use;
 }
 
 void Solver::refresh_primitives() {

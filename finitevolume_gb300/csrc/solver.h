@@ -126,6 +126,8 @@ struct Solver {
     int4* fxa = nullptr;
     int4* fxr = nullptr;
     int* fxs = nullptr;
+    int* fx_declined = nullptr;     // cells without such geometry, and whether they
+    bool fx_grad = false;           // are few enough for the fixed-point gradient pass
     double* fsp = nullptr;          // farfield primitives (O2Args::fsp)
     int psi_mode = 0;               // 0 evaluated, 2 frozen (see O2Args)
 

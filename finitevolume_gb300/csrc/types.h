@@ -247,8 +247,9 @@ void launch_part_f32(const O2Args& a, const O2Config& c, int stage, int part, cu
 // the last face pass; no update
 void launch_residual_f64(const O2Args& a, cudaStream_t s);
 void launch_residual_f32(const O2Args& a, cudaStream_t s);
-// the fixed-point gradient geometry (O2Args::fxa, fxr, fxs) from a.lsq, a.erf
-void launch_fix_geom(const O2Args& a, int4* fxa, int4* fxr, int* fxs, cudaStream_t s);
+// the fixed-point gradient geometry (O2Args::fxa, fxr, fxs) from a.lsq, a.erf;
+// adds the cells that have none to *declined
+void launch_fix_geom(const O2Args& a, int4* fxa, int4* fxr, int* fxs, int* declined, cudaStream_t s);
 void launch_batch_norms(const O2Args& a, int n_inst, const BatchNorms& b, double tol, cudaStream_t s);
 }  // namespace o2
 
