@@ -110,6 +110,7 @@ SIGNATURES = {
     "fv_solver_freeze_limiter": (C.c_int, [_P, C.c_int32]),
     "fv_solver_set_persistent": (C.c_int, [_P, C.c_int32]),
     "fv_solver_persistent": (C.c_int, [_P, _I32, _I32]),
+    "fv_solver_split_launches": (C.c_int, [_P, _I32]),
     "fv_solver_set_wait_limit": (C.c_int, [_P, C.c_int64, C.c_int32]),
     "fv_newton_default": (None, [C.POINTER(NewtonOpts)]),
     "fv_steady_newton": (C.c_int, [_P, C.POINTER(NewtonOpts), _D, _I32, _I32]),

@@ -36,10 +36,10 @@
 // to the two-kernel path too.
 //
 // With local dt a step has no global dependency, and the dataflow forms
-// (k_o1_dataflow_sm; k_o1_dataflow in the strict build, further down) replace
-// the grid barriers by waits on the few blocks that share faces with each
-// block.  Where they do not apply the default build runs the barrier form's
-// phases as launches of their own (k_o1_split_*).
+// (k_o1_dataflow_sm, k_o1_dataflow, further down) replace the grid barriers by
+// waits on the few blocks that share faces with each block.  Beyond the first
+// one's sizes, and with global dt, the default build runs the barrier form's
+// phases as launches of their own (k_o1_split_*) while no wait limit is set.
 //
 // The grid barrier is a counter plus a generation word.  Every wait (grid
 // barrier or neighbour progress) is bounded (PersistCtl::limit, in SM clock
@@ -522,8 +522,9 @@ __global__ void __launch_bounds__(fvgb::kCellBlock, FLUX == FLUX_EXACT ? 2 : 3) 
 // has a handful of neighbours).  The arithmetic per face and per cell is
 // face_phase_face / cell_phase_cell, and the norm partials are formed per
 // 32-cell warp and folded, after the last step, tile by tile in
-// k_cell_o1's order: fields and residual histories are the same bits as
-// the barrier form's.
+// k_cell_o1's order: in the strict build fields and residual histories are the
+// same bits as the barrier form's (the default build's compiler may contract
+// the forms differently: 1e-13).
 //
 // Progress words are published with st.release.gpu after a block barrier
 // (the block's writes of the phase, gathered by bar.sync, are ordered
@@ -636,7 +637,7 @@ __device__ __forceinline__ void df_fold(const O1Args& a, const DfPlan& d, int s,
     __syncthreads();
 }
 
-#ifdef FV_STRICT_ORDER  // (the default build uses the form below or k_o1_split_*)
+// (The default build runs it under a wait limit only: see k_o1_split_*.)
 template <int FLUX>
 __global__ void __launch_bounds__(fvgb::kDfBlock, 1) k_o1_dataflow(const O1Args a, double4_32a* __restrict__ P,
                                                                   PersistCtl* __restrict__ pc, const DfPlan d,
@@ -688,7 +689,6 @@ __global__ void __launch_bounds__(fvgb::kDfBlock, 1) k_o1_dataflow(const O1Args 
     for (int s = b; s < nsteps; s += nb) df_fold(a, d, s, (step0 + s) % a.hist_cap, s == nsteps - 1);
     if (b == 0 && threadIdx.x == 0) a.ctl->step = step0 + nsteps;
 }
-#endif
 
 // The same with the block's own cells and the fluxes of all their faces in
 // shared memory, for blocks that fit (DfPlan::smem).  A face between two
@@ -897,7 +897,6 @@ static int o1df_sm_blocks_per_sm(size_t smem) {
     return nb;
 }
 
-#ifdef FV_STRICT_ORDER
 template <int FLUX>
 static int o1df_blocks_per_sm() {
     int nb = 0;
@@ -905,7 +904,6 @@ static int o1df_blocks_per_sm() {
         return 0;
     return nb;
 }
-#endif
 
 template <int FLUX>
 static cudaError_t launch_o1df(const O1Args& a, double4_32a* P, PersistCtl* pc, const DfPlan& d, int nsteps,
@@ -921,11 +919,7 @@ static cudaError_t launch_o1df(const O1Args& a, double4_32a* P, PersistCtl* pc, 
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     if (d.smem) return cudaLaunchKernelEx(&cfg, k_o1_dataflow_sm<FLUX>, a, pc, d, nsteps);
-#ifdef FV_STRICT_ORDER
     return cudaLaunchKernelEx(&cfg, k_o1_dataflow<FLUX>, a, P, pc, d, nsteps);
-#else
-    return cudaErrorInvalidValue;
-#endif
 }
 
 #ifndef FV_STRICT_ORDER
@@ -1079,7 +1073,6 @@ int o1p_max_blocks_per_sm(int flux, int local) {
         default: return ::FV_KNS::o1p_blocks_per_sm<2, true>();
     }
 }
-#ifdef FV_STRICT_ORDER
 int o1df_max_blocks_per_sm(int flux) {
     switch (flux) {
         case 0: return ::FV_KNS::o1df_blocks_per_sm<0>();
@@ -1087,7 +1080,6 @@ int o1df_max_blocks_per_sm(int flux) {
         default: return ::FV_KNS::o1df_blocks_per_sm<2>();
     }
 }
-#endif
 int o1df_sm_max_blocks_per_sm(int flux, size_t smem) {
     switch (flux) {
         case 0: return ::FV_KNS::o1df_sm_blocks_per_sm<0>(smem);

@@ -757,28 +757,19 @@ bool dataflow_plan(const HostMesh& hm, const int* patch_type, int sms, DataflowP
 }
 
 void Solver::build_dataflow(const HostMesh& hm, int sms) {
-    if (opt.strict && strict::o1df_max_blocks_per_sm(opt.flux) < 1) return;
     DataflowPlan p;
     if (!dataflow_plan(hm, bc.type, sms, p)) return;
-    const int nb = p.nb, Wn = (N + 31) / 32;
+    const int nb = p.nb;
     // The shared-memory form where every block's cells (96 bytes each) and
     // their faces (40) fit: up to about 1,100 cells a block, 170k a mesh.
     // Larger meshes are bound by the work itself: the default build runs the
     // barrier form's phases as launches there (262k cells, Rusanov, 40 steps:
-    // 1.62 ms against 1.97 for the states in L2; 131k 1.04 against 1.06 here),
-    // the strict build keeps the states in L2.
+    // 1.62 ms against 1.97 for the states in L2; 131k 1.04 against 1.06 here) and
+    // keeps the states in L2 only for a wait limit, as the strict build does always.
     size_t own = 0;
     for (int b = 0; b < nb; ++b)
         own = std::max(own, 96 * (size_t)(p.cell_off[b + 1] - p.cell_off[b]) +
                                 40 * (size_t)(p.face_off[b + 1] - p.face_off[b]));
-    if (!opt.strict && own > kDfMaxSmem) return;
-    dfp.cell_off = dupload(p.cell_off, owned);
-    // the per-warp partials of every step of a launch: up to kPersistChunk
-    // steps, fewer on a large mesh (kDfPartialBytes)
-    const size_t per_step = (size_t)Wn * 4 * sizeof(double);
-    dfp.max_steps = (int)std::max<size_t>(8, std::min<size_t>(kPersistChunk, kDfPartialBytes / per_step));
-    dfp.wpart = dalloc<double>((size_t)dfp.max_steps * Wn * 4, owned);
-    dfp.n_warps = Wn;
     dfp.smem = 0;
     if (own <= kDfMaxSmem) {
         const std::vector<int>& block_of = p.owner;
@@ -841,8 +832,26 @@ void Solver::build_dataflow(const HostMesh& hm, int sms) {
             dfp.mail = dalloc<double2>(16 * (size_t)std::max(n_mail, 1), owned);
         }
     }
+    if (!dfp.smem && (opt.strict ? strict::o1df_max_blocks_per_sm(opt.flux) : fast::o1df_max_blocks_per_sm(opt.flux)) < 1)
+        return;
+    if (!dfp.smem && !opt.strict) {
+        std::vector<int>().swap(p.owner);
+        df_late = std::make_unique<DataflowPlan>(std::move(p));
+        return;
+    }
+    upload_dataflow(p);
+}
+
+void Solver::upload_dataflow(const DataflowPlan& p) {
+    const int Wn = (N + 31) / 32;
+    dfp.cell_off = dupload(p.cell_off, owned);
+    // the per-warp partials of every step of a launch: up to kPersistChunk
+    // steps, fewer on a large mesh (kDfPartialBytes)
+    const size_t per_step = (size_t)Wn * 4 * sizeof(double);
+    dfp.max_steps = (int)std::max<size_t>(8, std::min<size_t>(kPersistChunk, kDfPartialBytes / per_step));
+    dfp.wpart = dalloc<double>((size_t)dfp.max_steps * Wn * 4, owned);
+    dfp.n_warps = Wn;
     if (!dfp.smem) {
-        if (!opt.strict) return;
         std::vector<int> df = p.dep_face, dc = p.dep_cell;
         if (df.empty()) df.push_back(0);
         if (dc.empty()) dc.push_back(0);
@@ -852,15 +861,15 @@ void Solver::build_dataflow(const HostMesh& hm, int sms) {
         dfp.dep_face_off = dupload(p.dep_face_off, owned);
         dfp.dep_cell = dupload(dc, owned);
         dfp.dep_cell_off = dupload(p.dep_cell_off, owned);
-        dfp.prog = dalloc<unsigned int>((size_t)nb * kDfProgStride, owned);
+        dfp.prog = dalloc<unsigned int>((size_t)p.nb * kDfProgStride, owned);
     }
-    df_grid = nb;
+    df_grid = p.nb;
     dataflow_ok = true;
 }
 
 int Solver::persistent_form() const {
     if (!persistent) return 0;
-    return dataflow_ok && !barrier_form ? 2 : 1;
+    return dataflow_ok && !barrier_form && (dfp.smem || opt.strict || wait_limit_set) ? 2 : 1;
 }
 
 void Solver::launch_steps(int k, std::vector<int>* classes, std::vector<cudaEvent_t>* events, size_t* ev_pos) {
@@ -913,6 +922,10 @@ void Solver::set_wait_limit(long long cycles, int phantom) {
     h2d_sync(reinterpret_cast<char*>(pctl) + offsetof(PersistCtl, phantom), &phantom, sizeof(int), stream);
     h2d_sync(reinterpret_cast<char*>(pctl) + offsetof(PersistCtl, limit), &cycles, sizeof(long long), stream);
     const bool set = cycles != kDefaultWaitCycles || phantom != 0;
+    if (set && df_late) {
+        upload_dataflow(*df_late);
+        df_late.reset();
+    }
     if (set != wait_limit_set) {
         for (auto& kv : graphs) cudaGraphExecDestroy(kv.second);
         graphs.clear();
@@ -1544,6 +1557,13 @@ int fv_solver_persistent(fv_solver_t s, int32_t* on, int32_t* grid) {
         const int form = s->s.persistent_form();
         if (on) *on = form;
         if (grid) *grid = form == 2 ? s->s.df_grid : s->s.p_grid;
+    });
+}
+
+int fv_solver_split_launches(fv_solver_t s, int32_t* on) {
+    return guarded([&] {
+        if (!s || !on) fvgb::raise(FV_ERR_BAD_ARG, "null solver or result");
+        *on = s->s.split_form();
     });
 }
 

@@ -142,12 +142,16 @@ struct Solver {
     // barriers, one block per SM (DfPlan).  Used unless barrier_form.
     bool dataflow_ok = false;
     bool barrier_form = false;
-    // The default build runs the barrier form's phases as launches of their
-    // own, unless set_persistent asked for that form or a wait limit is set.
+    // Without the shared-memory dataflow form the default build runs the
+    // barrier form's phases as launches of their own, unless set_persistent asked
+    // for that form or a wait limit is set: with one, local time steps run the
+    // dataflow form with the states in L2, whose plan waits in df_late.
     bool wait_limit_set = false;
     bool split_form() const { return persistent && !opt.strict && persistent_form() == 1 && !barrier_form && !wait_limit_set; }
     int df_grid = 0;
     DfPlan dfp{};
+    std::unique_ptr<DataflowPlan> df_late;
+    void upload_dataflow(const DataflowPlan& p);
     static constexpr int kPersistChunk = 256;
     static constexpr long long kDefaultWaitCycles = 2000000000LL;  // ~1 s at 2 GHz
 

@@ -274,6 +274,7 @@ cudaError_t launch_o1_persistent(const O1Args& a, double4_32a* P, PersistCtl* pc
 // Its dataflow form for local dt (grid = the plan's block count, kDfBlock
 // threads per block, at most one block per SM).
 namespace fast {
+int o1df_max_blocks_per_sm(int flux);
 int o1df_sm_max_blocks_per_sm(int flux, size_t smem);
 cudaError_t launch_o1_dataflow(const O1Args& a, double4_32a* P, PersistCtl* pc, const DfPlan& d, int nsteps,
                                int grid, cudaStream_t s);

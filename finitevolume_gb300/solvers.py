@@ -385,10 +385,19 @@ class EulerFVMSolver:
 
     def persistent(self):
         """(form in use, grid size in blocks) of the persistent kernel: form
-        0 two-kernel path, 1 grid-barrier form, 2 dataflow form."""
+        0 two-kernel path, 1 grid-barrier form, 2 dataflow form.  Where
+        split_launches() holds, form 1 is not one launch of that grid."""
         on, grid = C.c_int32(), C.c_int32()
         capi.check(capi.lib().fv_solver_persistent(self._h, C.byref(on), C.byref(grid)))
         return int(on.value), int(grid.value)
+
+    def split_launches(self) -> bool:
+        """Whether the grid-barrier form runs as launches of its phases (the
+        default build with a global time step, or with local ones beyond the
+        shared-memory dataflow form, while no wait limit is set)."""
+        on = C.c_int32()
+        capi.check(capi.lib().fv_solver_split_launches(self._h, C.byref(on)))
+        return bool(on.value)
 
     def set_wait_limit(self, cycles: int, phantom_arrivals: int = 0) -> None:
         """Bound (SM clock cycles) on each wait of the persistent kernel

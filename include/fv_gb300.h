@@ -247,14 +247,17 @@ int fv_solver_set_launch(fv_solver_t s, const int32_t blocks[3]);
  * owns a range of cells, and each phase waits only for the blocks it shares
  * faces with instead of for the whole grid (same results again), on meshes
  * whose cells and fluxes fit in the SMs' shared memory (about 170k cells;
- * strict mode: any).  Elsewhere the default build runs the phases of the
- * grid-barrier form as launches of their own while no wait limit is set;
- * on = 2 keeps the one launch.  fv_solver_persistent reports the form in
- * use (0 two-kernel path, 1 grid-barrier form, 2 dataflow form) and its
- * grid size (either pointer may be NULL).  No reference counterpart (the
- * reference's loops are OpenMP). */
+ * strict mode, or with a wait limit set: any).  Elsewhere the default build
+ * runs the phases of the grid-barrier form as launches of their own while no
+ * wait limit is set; on = 2 keeps the one launch.  fv_solver_persistent
+ * reports the form in use (0 two-kernel path, 1 grid-barrier form, 2 dataflow
+ * form) and the grid size of its cooperative kernel (either pointer may be
+ * NULL); fv_solver_split_launches whether form 1 runs as launches of its
+ * phases, so that this kernel and its grid are not launched.  No reference
+ * counterpart (the reference's loops are OpenMP). */
 int fv_solver_set_persistent(fv_solver_t s, int32_t on);
 int fv_solver_persistent(fv_solver_t s, int32_t* on, int32_t* grid);
+int fv_solver_split_launches(fv_solver_t s, int32_t* on);
 /* Bound on every wait of the persistent kernel (grid barrier, or a
  * neighbour's progress word in the dataflow form), in SM clock cycles
  * (default 2e9, about one second).  A wait that runs out makes the launch
