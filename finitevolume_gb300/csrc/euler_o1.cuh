@@ -66,17 +66,20 @@ __device__ __forceinline__ double warp_sum4(double v0, double v1, double v2, dou
 // The block's smallest cfl * len / lam over its live threads into slot (all
 // threads call it; NaN does not count).  The rates lam / len are compared in
 // FP32 first, within 2^-20 of each other; only the faces within 2^-18 of the
-// block's largest form theirs in FP64 (five instructions, elsewhere none).
+// block's largest form theirs in FP64 (five instructions, elsewhere none), and
+// those whose speed or length is outside [2^-60, 2^61), where a rate could leave
+// FP32's range.
 __device__ __forceinline__ void block_min_step(bool live, double lam, double len, double cfl, unsigned long long* slot) {
     __shared__ unsigned smax[16];
-    unsigned b = live ? __float_as_uint(fvconv::d2f(lam) * fvfix::rcp_f(fvconv::d2f(len))) : 0u;
-    if (b > 0x7f800000u) b = 0u;
+    const unsigned es = (unsigned)__double2hiint(lam) >> 20, el = (unsigned)__double2hiint(len) >> 20;  // signs included
+    const bool in = live && es - 963u < 121u && el - 963u < 121u;
+    const unsigned b = in ? __float_as_uint(fvconv::d2f(lam) * fvfix::rcp_f(fvconv::d2f(len))) : 0u;
     const unsigned wm = __reduce_max_sync(0xffffffffu, b);
     if ((threadIdx.x & 31) == 0) smax[threadIdx.x >> 5] = wm;
     __syncthreads();
     unsigned m = smax[0];
     for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = max(m, smax[w]);
-    if (!live || __uint_as_float(b) < __uint_as_float(m) * (1.0f - 1.0f / 262144.0f)) return;
+    if (!live || (in && __uint_as_float(b) < __uint_as_float(m) * (1.0f - 1.0f / 262144.0f))) return;
     const unsigned long long dt = (unsigned long long)__double_as_longlong((cfl * len) * fvconv::rcp_nr3(lam));
     if (dt <= 0x7ff0000000000000ull) atomicMin(slot, dt);
 }
