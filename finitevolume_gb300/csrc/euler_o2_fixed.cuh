@@ -258,11 +258,11 @@ __device__ __forceinline__ void grad_lane(const O2Args& a, int c, int k, int e0,
         i64 nu, du, nd, dd;
         limiter_side<LIM>(dmax, up, eps2, E, nu, du);
         limiter_side<LIM>(-dmin, -dn, eps2, E, nd, dd);
-        // the smaller quotient, rounded to a multiple of 2^-52: exact as a
-        // double, which limiter freezing stores
+        // the smaller quotient, to 53 bits or 2^-60: exact as a double, which
+        // limiter freezing stores
         const bool lower = mul<3>(nd, du) < mul<3>(nu, dd);  // both below 16
         const i64 num = lower ? nd : nu, den = lower ? dd : du;
-        psi = (num < den ? ratio52(num, den) : (i64)1 << 52) << 8;
+        psi = num < den ? ratio60(num, den) : (i64)1 << 60;
     }
     const Sp p = split(psi);
     // Captured once the quad has taken the cell: a declined cell's four values

@@ -458,18 +458,20 @@ __device__ __forceinline__ bool warp_squares4(const double (&x)[4], double& sum)
     return ok;
 }
 
-// num / den * 2^52, rounded, for 0 < num <= den, den in [2^56, 2^62): three
-// quotient digits of 20, 20 and 12 bits, each from the float quotient of
-// the exact remainder (within 3/4 of a unit).
-__device__ __forceinline__ i64 ratio52(i64 num, i64 den) {
+// num / den * 2^60 for 0 < num <= den, den in [2^56, 2^62): three quotient
+// digits of 20 bits, each from the float quotient of the exact remainder (within
+// 3/4 of a unit), rounded to 53 significant bits: exact as a double.
+__device__ __forceinline__ i64 ratio60(i64 num, i64 den) {
     const float rf = rcp_f((float)(unsigned)((u64)den >> 32));
     const int q1 = __float2int_rn((float)(int)(num >> 32) * rf * 1048576.0f);
     i64 t = (num << 20) - (i64)q1 * den;
     const int q2 = __float2int_rn((float)(int)(t >> 32) * rf * 1048576.0f);
     t = (t << 20) - (i64)q2 * den;
-    const int q3 = __float2int_rn((float)(int)(t >> 32) * rf * 4096.0f);
-    const i64 q = ((i64)q1 << 32) + ((i64)q2 << 12) + q3;
-    return q > ((i64)1 << 52) ? (i64)1 << 52 : q;
+    const int q3 = __float2int_rn((float)(int)(t >> 32) * rf * 1048576.0f);
+    const i64 q = ((i64)q1 << 40) + ((i64)q2 << 20) + q3;
+    const unsigned one = 1u << max(11 - __clz((int)(q >> 32)), 0);  // the last of 53 bits, if above bit 0
+    const i64 r = q + (one >> 1);
+    return min((i64)((u64)r & ~(u64)(one - 1u)), (i64)1 << 60);
 }
 
 }  // namespace fvfix

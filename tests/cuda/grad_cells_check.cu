@@ -5,12 +5,14 @@
 // Cells of 3 to 18 faces with none, one, two or three boundary faces (slip and
 // no-slip walls, outflow, fixed and characteristic farfield), both limiters,
 // evaluated (live) and frozen at one (open: states overshoot, many fall back to
-// the cell's).  A second run has NaN in place of the FP64 weights and offsets,
+// the cell's).  A live run captures the limiter values, too.  A second run has NaN in place of the FP64 weights and offsets,
 // which only cells that the FP64 pass takes read: those without NaN were served.
 // Each line: "<run> faces F boundary B n N served S fallback P wrong Q rms_fixed A
 // rms_fp64 C max_fixed D max_fp64 E", errors relative to the largest value (for
 // velocities: speed or sound speed) and to how much the weights amplify its
-// rounding; wrong: fallbacks that are not the cell's state.
+// rounding; wrong: fallbacks that are not the cell's state.  Live runs then:
+// "<run>_psi faces F boundary B n N small M rms_fixed A rms_fp64 C", the limiter
+// values' errors relative to themselves or 2^-7, and how many are below 2^-4.
 #include <cmath>
 #include <cstdio>
 #include <random>
@@ -141,6 +143,12 @@ template <int LIM> static void check(const char* run, int faces, int bnd, bool o
         a.psi_buf = up(std::vector<double>(4 * n, 1.0));
         a.psi_mode = 2;
     }
+    double *p0 = nullptr, *p1 = nullptr;
+    if (!open) {
+        p0 = up(std::vector<double>(4 * n));
+        p1 = up(std::vector<double>(4 * n));
+        a.psi_mode = 1;
+    }
     int4 *xa, *xr;
     int *xs, *dec;
     cudaMalloc(&xa, sizeof(int4) * E); cudaMalloc(&xr, sizeof(int4) * E); cudaMalloc(&xs, sizeof(int) * n);
@@ -151,13 +159,25 @@ template <int LIM> static void check(const char* run, int faces, int bnd, bool o
     St *fx, *f64, *fn;
     cudaMalloc(&fx, sizeof(St) * E); cudaMalloc(&f64, sizeof(St) * E); cudaMalloc(&fn, sizeof(St) * E);
     a.wf = fx;
+    if (!open) a.psi_buf = p0;
     k_grad_fx<LIM><<<4 * n / 256, 256>>>(a);
     a.wf = f64;
+    if (!open) a.psi_buf = p1;
     k_grad<double, 0, LIM><<<n / 256, 256>>>(a);
     a.wf = fn;
+    if (!open) a.psi_mode = 0;
     a.lsq = a.erf = up(std::vector<double2>(E, make_double2(NAN, NAN)));
     k_grad_fx<LIM><<<4 * n / 256, 256>>>(a);
     auto A = down(fx, E), B = down(f64, E), C = down(fn, E);
+    std::vector<double> P0, P1;
+    if (!open) {
+        P0 = down(p0, 4 * n);
+        P1 = down(p1, 4 * n);
+        cudaFree(p0);
+        cudaFree(p1);
+    }
+    LD q0 = 0, q1 = 0;
+    long small = 0;
     LD s0 = 0, s1 = 0, mx0 = 0, mx1 = 0;
     long served = 0, fallback = 0, wrong = 0, count = 0;
     for (int i = 0; i < n; ++i) {
@@ -191,6 +211,11 @@ template <int LIM> static void check(const char* run, int faces, int bnd, bool o
                 if (ay > 0) psi = fminl(psi, LIM == 1 ? d1 / ay : (d1 * d1 + ep + 2 * d1 * ay) / (d1 * d1 + 2 * ay * ay + d1 * ay + ep));
             }
             if (open) psi = 1;
+            else {
+                const LD s = fmaxl(psi, 1.0L / 128), e0 = (P0[4 * i + k] - psi) / s, e1 = (P1[4 * i + k] - psi) / s;
+                q0 += e0 * e0; q1 += e1 * e1;
+                small += psi < 1.0L / 16;
+            }
             for (int e = off[i]; e < off[i + 1]; ++e) out[4 * (e - off[i]) + k] = wc[k] + psi * (gx * r[e].x + gy * r[e].y);
             sc[k] = big * fmaxl(1, amp);
         }
@@ -217,6 +242,9 @@ template <int LIM> static void check(const char* run, int faces, int bnd, bool o
     }
     printf("%s faces %d boundary %d n %d declined %d served %ld fallback %ld wrong %ld rms_fixed %.4Le rms_fp64 %.4Le max_fixed %.4Le max_fp64 %.4Le\n",
            run, faces, bnd, n, declined, served, fallback, wrong, sqrtl(s0 / (count ? count : 1)), sqrtl(s1 / (count ? count : 1)), mx0, mx1);
+    if (!open)
+        printf("%s_psi faces %d boundary %d n %d small %ld rms_fixed %.4Le rms_fp64 %.4Le\n", run, faces, bnd, 4 * n, small,
+               sqrtl(q0 / (4 * n)), sqrtl(q1 / (4 * n)));
     for (const void* p : {(const void*)a.m.cf_off, (const void*)a.m.fpatch, (const void*)a.m.fgeom, (const void*)a.cnb, a.lsq,
                           (const void*)a.lsq_sum, (const void*)a.eps2, (const void*)a.W, (const void*)fx, (const void*)f64,
                           (const void*)fn, (const void*)xa, (const void*)xr, (const void*)xs})
