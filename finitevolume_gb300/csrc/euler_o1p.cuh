@@ -637,7 +637,8 @@ __device__ __forceinline__ void df_fold(const O1Args& a, const DfPlan& d, int s,
     __syncthreads();
 }
 
-// (The default build runs it under a wait limit only: see k_o1_split_*.)
+// (The default build runs it for the exact Riemann flux, and beyond the next
+// form's sizes under a wait limit: see k_o1_split_*.)
 template <int FLUX>
 __global__ void __launch_bounds__(fvgb::kDfBlock, 1) k_o1_dataflow(const O1Args a, double4_32a* __restrict__ P,
                                                                   PersistCtl* __restrict__ pc, const DfPlan d,
@@ -675,7 +676,8 @@ __global__ void __launch_bounds__(fvgb::kDfBlock, 1) k_o1_dataflow(const O1Args 
         // no block still reads the own cells' step-s states
         if (!df_wait(pc, d.prog, dep_c, nc, 2u * s + 1u)) return;
         double* wp = d.wpart + (size_t)s * d.n_warps * 4;
-        for (int cw = c0 / 32 + warp; cw * 32 < c1; cw += nwarps) {
+        // (a last block without cells starts at N, maybe inside the block before's last warp)
+        for (int cw = (c0 + 31) / 32 + warp; cw * 32 < c1; cw += nwarps) {
             const int c = cw * 32 + lane;
             St R = st_make(0.0, 0.0, 0.0, 0.0);
             if (c < N) cell_phase_cell<true>(a, P, c, g, cfl, 0.0, R);

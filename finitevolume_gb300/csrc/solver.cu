@@ -766,12 +766,17 @@ void Solver::build_dataflow(const HostMesh& hm, int sms) {
     // barrier form's phases as launches there (262k cells, Rusanov, 40 steps:
     // 1.62 ms against 1.97 for the states in L2; 131k 1.04 against 1.06 here) and
     // keeps the states in L2 only for a wait limit, as the strict build does always.
+    // The exact Riemann flux, whose iterations cost far more than an exchange,
+    // loses on the faces that two blocks compute and takes the states in L2 at those
+    // sizes (us a step here and there: 2k quads 126 and 96, 131k 865 and 816, 15k
+    // mixed cells 350 and 210; the launches take 85 to 119% of the latter's time).
+    const bool shared = opt.strict || opt.flux != FV_FLUX_EXACT;
     size_t own = 0;
     for (int b = 0; b < nb; ++b)
         own = std::max(own, 96 * (size_t)(p.cell_off[b + 1] - p.cell_off[b]) +
                                 40 * (size_t)(p.face_off[b + 1] - p.face_off[b]));
     dfp.smem = 0;
-    if (own <= kDfMaxSmem) {
+    if (shared && own <= kDfMaxSmem) {
         const std::vector<int>& block_of = p.owner;
         // faces between blocks, and a mailbox for each of their cells
         std::vector<unsigned char> between(F, 0);
@@ -834,7 +839,8 @@ void Solver::build_dataflow(const HostMesh& hm, int sms) {
     }
     if (!dfp.smem && (opt.strict ? strict::o1df_max_blocks_per_sm(opt.flux) : fast::o1df_max_blocks_per_sm(opt.flux)) < 1)
         return;
-    if (!dfp.smem && !opt.strict) {
+    df_use = opt.strict || own <= kDfMaxSmem;
+    if (!df_use) {
         std::vector<int>().swap(p.owner);
         df_late = std::make_unique<DataflowPlan>(std::move(p));
         return;
@@ -869,7 +875,7 @@ void Solver::upload_dataflow(const DataflowPlan& p) {
 
 int Solver::persistent_form() const {
     if (!persistent) return 0;
-    return dataflow_ok && !barrier_form && (dfp.smem || opt.strict || wait_limit_set) ? 2 : 1;
+    return dataflow_ok && !barrier_form && (df_use || wait_limit_set) ? 2 : 1;
 }
 
 void Solver::launch_steps(int k, std::vector<int>* classes, std::vector<cudaEvent_t>* events, size_t* ev_pos) {

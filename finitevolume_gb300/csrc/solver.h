@@ -142,14 +142,22 @@ struct Solver {
     // barriers, one block per SM (DfPlan).  Used unless barrier_form.
     bool dataflow_ok = false;
     bool barrier_form = false;
-    // Without the shared-memory dataflow form the default build runs the
+    // Beyond the shared-memory dataflow form's sizes the default build runs the
     // barrier form's phases as launches of their own, unless set_persistent asked
     // for that form or a wait limit is set: with one, local time steps run the
     // dataflow form with the states in L2, whose plan waits in df_late.
     bool wait_limit_set = false;
-    bool split_form() const { return persistent && !opt.strict && persistent_form() == 1 && !barrier_form && !wait_limit_set; }
+    // The exact Riemann flux with a global step keeps the one launch on larger
+    // meshes, whose blocks take equal shares of its uneven faces (us a step, launches
+    // and one launch: 8k quads 96 and 158, 15k mixed cells 170 and 170, 32k quads 305
+    // and 265, 61k mixed 679 and 584, 500k quads 3760 and 3702).
+    bool split_form() const {
+        const bool uneven = opt.flux == FV_FLUX_EXACT && opt.dt_mode != FV_DT_LOCAL && N > 12000;
+        return persistent && !opt.strict && persistent_form() == 1 && !barrier_form && !wait_limit_set && !uneven;
+    }
     int df_grid = 0;
     DfPlan dfp{};
+    bool df_use = false;            // also without a wait limit
     std::unique_ptr<DataflowPlan> df_late;
     void upload_dataflow(const DataflowPlan& p);
     static constexpr int kPersistChunk = 256;

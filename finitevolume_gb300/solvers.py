@@ -394,7 +394,8 @@ class EulerFVMSolver:
     def split_launches(self) -> bool:
         """Whether the grid-barrier form runs as launches of its phases (the
         default build with a global time step, or with local ones beyond the
-        shared-memory dataflow form, while no wait limit is set)."""
+        shared-memory dataflow form, while no wait limit is set; not the exact
+        Riemann flux with a global step on more than 12,000 cells)."""
         on = C.c_int32()
         capi.check(capi.lib().fv_solver_split_launches(self._h, C.byref(on)))
         return bool(on.value)

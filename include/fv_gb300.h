@@ -247,9 +247,10 @@ int fv_solver_set_launch(fv_solver_t s, const int32_t blocks[3]);
  * owns a range of cells, and each phase waits only for the blocks it shares
  * faces with instead of for the whole grid (same results again), on meshes
  * whose cells and fluxes fit in the SMs' shared memory (about 170k cells;
- * strict mode, or with a wait limit set: any).  Elsewhere the default build
- * runs the phases of the grid-barrier form as launches of their own while no
- * wait limit is set; on = 2 keeps the one launch.  fv_solver_persistent
+ * strict mode, or with a wait limit set: any).
+ * Elsewhere the default build runs the phases of the grid-barrier form as
+ * launches of their own (but for the exact flux with a global step beyond
+ * 12,000 cells) while no wait limit is set; on = 2 keeps the one launch.  fv_solver_persistent
  * reports the form in use (0 two-kernel path, 1 grid-barrier form, 2 dataflow
  * form) and the grid size of its cooperative kernel (either pointer may be
  * NULL); fv_solver_split_launches whether form 1 runs as launches of its

@@ -65,3 +65,23 @@ def test_requested_forms(gpu):
     t.set_wait_limit(DEFAULT + 1)
     assert t.persistent()[0] == 1 and not t.split_launches()
     t.run(2)
+
+
+@pytest.mark.parametrize("size,local,split", [((64, 33), True, False), ((24, 9), True, False), ((64, 33), False, True), ((160, 75), False, True),
+                                              ((160, 76), False, False), ((160, 76), True, False)])
+def test_exact_flux_forms(gpu, size, local, split):
+    """The exact Riemann flux: the dataflow form in L2 (24 x 9: its last block has no cells, and starts inside another's
+    last warp), and one launch for the global step beyond 12,000 cells; against the grid-barrier form."""
+    M, aoa = 0.5, np.radians(2.0)
+    r, u, v, p = 1.0, M * np.cos(aoa), M * np.sin(aoa), 1.0 / GAMMA
+    bcs = [(0, [0.0] * 4), (3, list(S.from_primitive(r, u, v, p, GAMMA)))]
+    ic = {"mode": "free", "rho": r, "u": u, "v": v, "p": p}
+    poly = meshgen.naca_ogrid(*size)
+    a, b = (gpu_solver(poly, bcs, ic, "exact", cfl=0.5, local_dt=local) for _ in range(2))
+    assert a.persistent()[0] == (2 if local else 1) and a.split_launches() == split
+    b.set_persistent("barrier")
+    assert b.persistent()[0] == 1 and not b.split_launches()
+    for n in (1, 9):
+        ha, hb = a.run(n, history=True), b.run(n, history=True)
+        assert rel_err(a.field(), b.field()) <= 1e-13
+        np.testing.assert_allclose(ha, hb, rtol=1e-13, atol=0)
