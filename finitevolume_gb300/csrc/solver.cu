@@ -839,7 +839,7 @@ void Solver::build_dataflow(const HostMesh& hm, int sms) {
     }
     if (!dfp.smem && (opt.strict ? strict::o1df_max_blocks_per_sm(opt.flux) : fast::o1df_max_blocks_per_sm(opt.flux)) < 1)
         return;
-    df_use = opt.strict || own <= kDfMaxSmem;
+    df_use = opt.strict || dfp.smem || (!shared && own <= kDfMaxSmem);
     if (!df_use) {
         std::vector<int>().swap(p.owner);
         df_late = std::make_unique<DataflowPlan>(std::move(p));

@@ -26,8 +26,10 @@ def _solver(size, local, **kw):
 
 
 @pytest.mark.parametrize("size,local,form,limited", [((64, 32), False, 1, 1), ((64, 32), True, 2, 2),
+                                                     ((512, 330), True, 1, 2),
                                                      ((512, 400), True, 1, 2), ((512, 400), False, 1, 1)])
 def test_forms_with_and_without_a_wait_limit(gpu, size, local, form, limited):
+    """512 x 330: the blocks' own cells and faces fit in shared memory, with their neighbours' faces they do not."""
     a, b = _solver(size, local), _solver(size, local)
     assert a.persistent()[0] == form and a.split_launches() == (form == 1)
     b.set_wait_limit(DEFAULT + 1)
