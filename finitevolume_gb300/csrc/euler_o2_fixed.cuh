@@ -4,12 +4,14 @@
 // ranges of the fixed-point one.
 //
 // Measured on the GB300 (1.05M-cell O-grid, Venkatakrishnan, HLLC, time per
-// launch): gradients and limiter 417 us in FP64 (the FP64 pipe 86% busy), 146
-// here; face fluxes 387 us in FP64 (88% busy), 81 here.  On 2k cells, where a
+// launch): gradients and limiter 417 us in FP64 (the FP64 pipe 86% busy), 143
+// here; face fluxes 387 us in FP64 (88% busy), 80 here.  On 2k cells, where a
 // launch is one wave and the length of a thread's dependent chain counts
 // (FP64 64 clocks an operation, integers 5 to 13), 32 and 21 us became 10
-// and 8.5.  Errors against 128-bit arithmetic are no larger than the FP64
-// forms' (tests/cuda/fixed_check.cu).
+// and 8.5.  Errors against 128-bit arithmetic, relative to the face's or cell's
+// own scale, are no larger than the FP64 forms' (tests/cuda/fixed_check.cu,
+// flux_components_check.cu, grad_cells_check.cu); a component far below that
+// scale keeps fewer bits of its own.
 #pragma once
 
 #include "euler_o2.cuh"
@@ -138,7 +140,7 @@ static __device__ __noinline__ V4<double> ghost_more(const O2Args& a, int f, int
 
 // Bitwise or over a quad, by two shuffles: a warp-wide reduction with a mask of
 // its own per quad runs once for each of the warp's eight quads (1.05M cells:
-// eight steps 7.35 -> 7.22 ms).
+// eight steps 7.35 -> 7.25 ms).
 __device__ __forceinline__ unsigned quad_or(unsigned quad, unsigned x) {
     x |= __shfl_xor_sync(quad, x, 1, 4);
     return x | __shfl_xor_sync(quad, x, 2, 4);

@@ -15,7 +15,10 @@
 // fixed place and keeps all its 53 bits with 4 to 7 bits below them; a
 // smaller operand loses only bits below 2^-58 of the largest.  That is the
 // absolute size of every error here, against 2^-53 of the result for each
-// FP64 operation.  Inputs outside the ranges that rule out overflow (checked
+// FP64 operation: a component far below its block's scale keeps fewer bits of its
+// own (normals within 2^-20 of an axis beside a velocity 2^-20 of the other: the
+// small momentum flux to 3e-7 of itself, 3e-17 of the face's scale; FP64 3e-14 and
+// 5e-17).  Inputs outside the ranges that rule out overflow (checked
 // from the exponents and from the intermediate values) are reported, and the
 // caller evaluates them in FP64: zeros, subnormals, infinities, NaN,
 // non-positive densities and pressures, density ratios above 16, pressure
