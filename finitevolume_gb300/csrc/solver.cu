@@ -230,7 +230,8 @@ void Solver::init(const HostMesh& hm, const fv_bc_t* bcs, int n_bcs, double g, d
         const size_t wsz = cfg.fp32 ? 16 : 32;
         U0 = dalloc<St>(N, owned);
         W = dalloc<char>(wsz * (size_t)N, owned);
-        G = dalloc<char>(2 * wsz * (size_t)N, owned);
+        // limited gradients; FP64 with a limiter leaves face states instead (wf)
+        if (cfg.order == 2 && (cfg.fp32 || cfg.limiter == 0)) G = dalloc<char>(2 * wsz * (size_t)N, owned);
         if (cfg.fp32) ff = reinterpret_cast<St*>(dalloc<char>(16 * (size_t)F, owned));
         cs = dalloc<char>(wsz / 4 * (size_t)N, owned);
         dtv = dalloc<double>(N, owned);

@@ -105,7 +105,7 @@ struct Solver {
     O2Config cfg{};
     St* U0 = nullptr;
     void* W = nullptr;
-    void* G = nullptr;
+    void* G = nullptr;              // null where not used
     void* cs = nullptr;             // sound speed, flux precision
     double* dtv = nullptr;
     const int* cnb = nullptr;
